@@ -178,28 +178,18 @@ def make_sim(F, device: int, mg_fixed: int = 0):
 
 def launches_per_step(sim, cycles_per_step: float) -> float:
     """Kernels launched per step by the captured graph: 5 stencil kernels (the divergence kernel also clears
-    the solve's cycle count), and per V-cycle 10 per level above the shared-memory tail (2 + 2 red-black sweeps of 2 colour launches each,
+    the solve's cycle count), and per V-cycle 10 per level above the coarse kernel (2 + 2 red-black sweeps of 2 colour launches each,
     restriction, prolongation) less one per level below the finest (its first colour-0 sweep runs inside the
-    restriction onto it), the tail kernel, the residual norm and the decision kernel.  The tail starts at the
-    finest level that fits in 200 KB of shared memory (one CTA, or 8 CTAs with distributed levels) and has at
-    most 8192 cells."""
-    n = len(sim.levels)
-    T = n
-    for l in range(n - 1, -1, -1):
-        nx, ny, nz = sim.levels[l]["dims"]
-        cells = nx * ny * nz
-        smem = 0
-        for k in range(l, n):
-            kx, ky, kz = sim.levels[k]["dims"]
-            c = kx * ky * kz
-            dist = k < n - 1 and kz % 16 == 0 and c >= 8 * 512
-            smem += 8 * (c // 8 if dist else c)
-        if cells <= 8192 and smem <= 200 * 1024:
-            T = l
-        else:
+    restriction onto it), the coarse kernel, the residual norm and the decision kernel.  The coarse kernel takes the
+    levels whose half-row x z columns, times their groups of four rows per CTA of a 16-CTA cluster, fit 1024 threads."""
+    T = len(sim.levels)
+    while T > 0:
+        nx, ny, nz = sim.levels[T - 1]["dims"]
+        if (nx + 1) // 2 * nz * ((ny + 63) // 64) > 1024:
             break
-    top = min(T, n - 1)
-    per_cycle = 10 * top - max(top - 1, 0) + (1 if T < n else 0) + 2
+        T -= 1
+    top = min(T, len(sim.levels) - 1)
+    per_cycle = 10 * top - max(top - 1, 0) + (1 if T < len(sim.levels) else 0) + 2
     return 5 + per_cycle * cycles_per_step
 
 

@@ -169,7 +169,8 @@ int fire_sim_set_spots(FireSim* sim, const float* spots, int n);
  * needs (no counterpart in the reference).                                                            */
 int fire_sim_set_mg_omega(FireSim* sim, float omega);
 /* Fault-injection hook for the device-side bounded wait (no counterpart in the reference, which logs
- * WebGPU device loss, src/gpu.js:25-26): the multigrid's single-CTA tail waits for the TMA bulk copies that
+ * WebGPU device loss, src/gpu.js:25-26).  A value other than the default runs the multigrid's coarse end in its
+ * TMA-staged tail kernels (the same bits): the single-CTA one waits for the TMA bulk copies that
  * stage its first level into shared memory for at most `polls` polls (default 4194304, and about a second)
  * before it records a timeout, waits again at the full bound for the copies in flight and returns without
  * running the cycle; fire_sim_sync then reports FIRE_ERR_CUDA ("a device-side wait timed out") and clears

@@ -190,18 +190,23 @@ void record_smooth(FireSim* s, int l, int iters, cudaStream_t st, bool first_don
     launch_smooth(s->levels[l], 1, st);
   }
 }
-// One V(2,2) cycle (src/sim.js:588-599).  Levels [tailFirst, n) run inside one tail kernel.  A restriction
+// Whether the coarse levels run in the register-resident coarse kernel; the TMA-staged tail takes over when nothing fits
+// it, and while its wait limit is lowered (fire_sim_set_tail_wait_limit exercises that kernel's bounded wait).
+bool use_coarse(const FireSim* s) { return s->coarseFirst < (int)s->levels.size() && s->tailWaitPolls == TAIL_WAIT_POLLS; }
+// One V(2,2) cycle (src/sim.js:588-599).  Levels [T, n) run inside one launch.  A restriction
 // onto a level that is smoothed by launches also applies that level's first colour-0 sweep.
 void record_vcycle(FireSim* s, cudaStream_t st) {
   const int n = (int)s->levels.size();
-  const int T = s->tailFirst;
+  const bool co = use_coarse(s);
+  const int T = co ? s->coarseFirst : s->tailFirst;
   const int top = std::min(T, n - 1);
   for (int i = 0; i < top; ++i) {
     record_smooth(s, i, 2, st, i > 0);
     if (i + 1 < top) launch_restrict_smooth(s->levels[i], s->levels[i + 1], st);
     else launch_restrict(s->levels[i], s->levels[i + 1], st);
   }
-  if (T < n) launch_tail(s->levels.data(), T, n, 2, 2, s->coarseIters, s->dCounter + 2, st, false, nullptr, s->tailWaitPolls);
+  if (co) launch_coarse(s->levels.data(), T, n, 2, 2, s->coarseIters, nullptr, 1, s->dCounter + 2, st);
+  else if (T < n) launch_tail(s->levels.data(), T, n, 2, 2, s->coarseIters, s->dCounter + 2, st, false, nullptr, s->tailWaitPolls);
   else record_smooth(s, n - 1, s->coarseIters, st);
   for (int i = top - 1; i >= 0; --i) { launch_prolong(s->levels[i], s->levels[i + 1], st); record_smooth(s, i, 2, st); }
 }
@@ -217,6 +222,11 @@ int record_ev(FireSim* sim, int idx, cudaStream_t st, bool prof) {
 // count (launch_div with the counter), else a clearing kernel is recorded here.
 int record_mg(FireSim* sim, cudaStream_t st, bool counter_cleared) {
   if (sim->mg_max_cycles <= 0) {
+    if (use_coarse(sim) && sim->coarseFirst == 0) {   // the whole hierarchy is on chip: every cycle in one launch
+      if (sim->vcycles > 0)
+        launch_coarse(sim->levels.data(), 0, (int)sim->levels.size(), 2, 2, sim->coarseIters, nullptr, sim->vcycles, sim->dCounter + 2, st);
+      return FIRE_OK;
+    }
     for (int c = 0; c < sim->vcycles; ++c) record_vcycle(sim, st);
     return FIRE_OK;
   }
@@ -421,6 +431,7 @@ int fire_sim_create(const FireConfig* cfg, const float* logs, int n_logs, FireSi
     sim->coarseIters = (int)std::max(8.0, std::min(64.0, std::ceil(std::log(0.05) / std::log(mu * mu))));
     const int n = (int)sim->levels.size();
     sim->tailFirst = tail_first(sim->levels.data(), n);
+    sim->coarseFirst = coarse_first(sim->levels.data(), n);
   }
 
   // device arena
@@ -482,7 +493,7 @@ int fire_sim_create(const FireConfig* cfg, const float* logs, int n_logs, FireSi
       cudaEventCreateWithFlags(&sim->forkEv, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&sim->joinEv, cudaEventDisableTiming) != cudaSuccess)
     return fail(FIRE_ERR_CUDA);
-  if (mg_configure(TAIL_SMEM_BUDGET) != cudaSuccess) return fail(set_err(sim, FIRE_ERR_CUDA, "tail kernel smem opt-in failed"));
+  if (mg_configure(TAIL_SMEM_BUDGET) != cudaSuccess || coarse_configure() != cudaSuccess) return fail(set_err(sim, FIRE_ERR_CUDA, "tail kernel smem opt-in failed"));
   if (step_configure() != cudaSuccess) return fail(set_err(sim, FIRE_ERR_CUDA, "forces kernel smem opt-in failed"));
 
   // zero state (reset semantics), bake the tables (src/noise.js), upload logs
@@ -949,7 +960,9 @@ int fire_sim_run_mg(FireSim* sim, int op, int level, int arg, void* stream) {
       break;
     case 4:   // the shared-memory V-cycle from `level` down, if it fits
       if (!tail_fits(sim->levels.data(), level, n)) return FIRE_ERR_BAD_ARG;
-      launch_tail(sim->levels.data(), level, n, 2, 2, sim->coarseIters, sim->dCounter + 2, st, false, nullptr, sim->tailWaitPolls);
+      if (sim->tailWaitPolls == TAIL_WAIT_POLLS && coarse_fits(sim->levels.data(), level, n))
+        launch_coarse(sim->levels.data(), level, n, 2, 2, sim->coarseIters, nullptr, 1, sim->dCounter + 2, st);
+      else launch_tail(sim->levels.data(), level, n, 2, 2, sim->coarseIters, sim->dCounter + 2, st, false, nullptr, sim->tailWaitPolls);
       break;
     default: return FIRE_ERR_BAD_ARG;
   }
@@ -1104,7 +1117,10 @@ struct FireEnsemble {
   cudaEvent_t ringEv[4] = {};
   bool ringUsed[4] = {};
   int ringPos = 0;
-  void* dTail[2] = {nullptr, nullptr};      // tail descriptors by form (single CTA, cluster)
+  void* dCoarse[COARSE_KINDS] = {};         // coarse-kernel descriptors by kind
+  int coarseCount[COARSE_KINDS] = {};
+  size_t coarseSmem[COARSE_KINDS] = {};
+  void* dTail[2] = {nullptr, nullptr};      // tail descriptors by form (single CTA, cluster), for members the coarse kernel does not fit
   int tailCount[2] = {0, 0};
   size_t tailSmem[2] = {0, 0};
   int* dErr = nullptr;
@@ -1142,6 +1158,11 @@ int ens_err(FireEnsemble* e, int code, const char* msg) {
   return code;
 }
 
+// Levels a member smooths by batched launches; the rest run in its coarse end.
+int ens_top(const FireSim* s) {
+  const int n = (int)s->levels.size();
+  return std::min(s->coarseFirst < n ? s->coarseFirst : s->tailFirst, n - 1);
+}
 // Records one ensemble step (src/sim.js:633-644 for every member): adv1, adv2, curl + forces, div,
 // `vcycles` V(2,2) cycles, project.
 // Launch descriptions of one ensemble step: the members' stage pointers, one BatchMap per tile candidate,
@@ -1164,7 +1185,7 @@ void ens_context(FireEnsemble* e, EnsCtx& c) {
     c.SB.s[i] = StepInst{e->dBlocks + (size_t)i * BLOCK_FLOATS, s->f, s->d, s->levels[0].b, s->levels[0].p};
     for (int v = 0; v < CELL_TILES; ++v) map_add(c.cell[v], i, step_grid(s->d, v));
     for (int v = 0; v < FORCES_TILES; ++v) map_add(c.forces[v], i, forces_grid(s->d, v));
-    c.depth = std::max(c.depth, std::min(s->tailFirst, (int)s->levels.size() - 1));
+    c.depth = std::max(c.depth, ens_top(s));
   }
   // per level: the members that have it outside their tail, and every member's level l and l + 1
   c.smoothMap.assign(c.depth, map_empty());
@@ -1173,7 +1194,7 @@ void ens_context(FireEnsemble* e, EnsCtx& c) {
   for (int l = 0; l <= c.depth; ++l) std::memset(&c.LB[l], 0, sizeof(LevelBatch));
   for (int i = 0; i < n; ++i) {
     FireSim* s = e->sims[i];
-    const int top = std::min(s->tailFirst, (int)s->levels.size() - 1);
+    const int top = ens_top(s);
     for (int l = 0; l <= c.depth && l < (int)s->levels.size(); ++l) c.LB[l].l[i] = s->levels[l];
     for (int l = 0; l < top; ++l) {
       map_add(c.smoothMap[l], i, smooth_grid(s->levels[l]));
@@ -1197,6 +1218,8 @@ void ens_mg(FireEnsemble* e, const EnsCtx& c, cudaStream_t st) {
       for (int k = 0; k < 2; ++k) { launch_smooth_batch(c.smoothMap[l], c.LB[l], 0, st); launch_smooth_batch(c.smoothMap[l], c.LB[l], 1, st); }
       launch_restrict_batch(c.coarseMap[l], c.LB[l], c.LB[l + 1], st);
     }
+    for (int kind = 0; kind < COARSE_KINDS; ++kind)
+      launch_coarse_batch(kind, e->dCoarse[kind], e->coarseCount[kind], e->coarseSmem[kind], 2, 2, st);
     for (int kind = 0; kind < 2; ++kind)
       launch_tail_batch(kind, e->dTail[kind], e->tailCount[kind], e->tailSmem[kind], 2, 2, e->dErr, st);
     for (int l = c.depth - 1; l >= 0; --l) {
@@ -1280,6 +1303,7 @@ int fire_ensemble_destroy(FireEnsemble* e) {
   for (int k = 0; k < ENS_RING; ++k) if (e->ringEv[k]) cudaEventDestroy(e->ringEv[k]);
   if (e->hRing) cudaFreeHost(e->hRing);
   if (e->dBlocks) cudaFree(e->dBlocks);
+  for (void* p : e->dCoarse) if (p) cudaFree(p);
   for (int k = 0; k < 2; ++k) if (e->dTail[k]) cudaFree(e->dTail[k]);
   if (e->dErr) cudaFree(e->dErr);
   for (FireSim* s : e->sims) fire_sim_destroy(s);
@@ -1318,17 +1342,35 @@ int fire_ensemble_create(const FireConfig* cfgs, int n, FireEnsemble** out) {
   }
   for (int k = 0; k < ENS_RING; ++k)
     if (cudaEventCreateWithFlags(&e->ringEv[k], cudaEventDisableTiming) != cudaSuccess) { fire_ensemble_destroy(e); return FIRE_ERR_CUDA; }
-  // tail descriptors, grouped by form
-  std::vector<unsigned char> desc[2];
+  // descriptors of the members' coarse ends, grouped by form
+  std::vector<unsigned char> desc[2], cdesc[COARSE_KINDS];
   for (int i = 0; i < n; ++i) {
     FireSim* s = e->sims[i];
     const int L = (int)s->levels.size();
+    if (s->coarseFirst < L) {
+      std::vector<unsigned char> d(coarse_desc_size());
+      size_t smem = 0;
+      const int kind = coarse_desc_fill(s->levels.data(), s->coarseFirst, L, s->coarseIters, e->dErr, d.data(), &smem);
+      if (kind < 0) { fire_ensemble_destroy(e); return FIRE_ERR_CUDA; }
+      cdesc[kind].insert(cdesc[kind].end(), d.begin(), d.end());
+      e->coarseCount[kind] += 1;
+      e->coarseSmem[kind] = std::max(e->coarseSmem[kind], smem);
+      continue;
+    }
     const int kind = tail_kind(s->levels.data(), s->tailFirst, L);
     const size_t sz = tail_desc_size(kind);
     desc[kind].resize(desc[kind].size() + sz);
     tail_desc_fill(s->levels.data(), s->tailFirst, L, s->coarseIters, desc[kind].data() + desc[kind].size() - sz);
     e->tailCount[kind] += 1;
     e->tailSmem[kind] = std::max(e->tailSmem[kind], tail_smem_bytes(s->levels.data(), s->tailFirst, L));
+  }
+  for (int k = 0; k < COARSE_KINDS; ++k) {
+    if (!e->coarseCount[k]) continue;
+    if (cudaMalloc(&e->dCoarse[k], cdesc[k].size()) != cudaSuccess ||
+        cudaMemcpy(e->dCoarse[k], cdesc[k].data(), cdesc[k].size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+      fire_ensemble_destroy(e);
+      return FIRE_ERR_CUDA;
+    }
   }
   for (int k = 0; k < 2; ++k) {
     if (!e->tailCount[k]) continue;

@@ -164,6 +164,21 @@ size_t tail_smem_bytes(const MGLevel* levels, int first, int n, bool coarse64 = 
 constexpr int TAIL_WAIT_POLLS = 1 << 22;
 cudaError_t launch_tail(const MGLevel* levels, int first, int n, int pre, int post, int coarse, int* err, cudaStream_t st,
                         bool coarse64 = false, const double* cinv = nullptr, int wait_polls = TAIL_WAIT_POLLS);
+// The coarse end of the cycle with register-resident cells (fire_coarse.cu): levels [first, n) in one launch of one CTA
+// or one cluster.  coarse_first: the finest `first` it takes (n if none); direct: the coarsest level is solved with
+// a dense FP64 inverse (cinv).  `cycles` > 1 (first == 0 only) repeats the whole V-cycle inside the launch.
+// Bit-identical to the launch-per-phase kernels (omega 1).  `err` receives 1 if a bounded wait for a neighbouring CTA's rows ran out.
+int coarse_first(const MGLevel* levels, int n, bool direct = false);
+bool coarse_fits(const MGLevel* levels, int first, int n, bool direct = false);
+cudaError_t launch_coarse(const MGLevel* levels, int first, int n, int pre, int post, int coarse, const double* cinv, int cycles,
+                          int* err, cudaStream_t st);
+cudaError_t coarse_configure();
+// Batched over simulations: the host fills coarse_desc_size() bytes each and groups them by the returned kind
+// (COARSE_KINDS of them; -1: does not fit); a launch takes `count` descriptors of one kind and their largest smem.
+constexpr int COARSE_KINDS = 4;
+size_t coarse_desc_size();
+int coarse_desc_fill(const MGLevel* levels, int first, int n, int coarse, int* err, void* out, size_t* smem);
+cudaError_t launch_coarse_batch(int kind, const void* dev_descs, int count, size_t smem, int pre, int post, cudaStream_t st);
 // Opts the tail kernels into `max_tail_smem` bytes of dynamic shared memory on the current device.
 cudaError_t mg_configure(size_t max_tail_smem);
 // Batched forms: one launch per level operation over the simulations of a BatchMap.

@@ -44,7 +44,7 @@ int setup_device(int dev, unsigned char** base) {
   if (!s.ready) {
     void* ptr = nullptr;
     if (cudaGetSymbolAddress(&ptr, g_noalloc_scratch) != cudaSuccess || ptr == nullptr) return FIRE_ERR_CUDA;
-    if (mg_configure(TAIL_SMEM_BUDGET) != cudaSuccess) return FIRE_ERR_CUDA;
+    if (mg_configure(TAIL_SMEM_BUDGET) != cudaSuccess || coarse_configure() != cudaSuccess) return FIRE_ERR_CUDA;
     s.base = static_cast<unsigned char*>(ptr);
     s.ready = true;
   }
@@ -99,7 +99,8 @@ extern "C" int fire_poisson_vcycles_noalloc(float* p, const float* b, int nx, in
   const double PI = 3.14159265358979323846;
   const double mu = (std::cos(PI / C.nx) + std::cos(PI / (2.0 * C.ny)) + std::cos(PI / C.nz)) / 3.0;
   const int coarse = (int)std::max(8.0, std::min(64.0, std::ceil(std::log(0.05) / std::log(mu * mu))));
-  const int T = tail_first(levels.data(), n);
+  const int co = coarse_first(levels.data(), n);
+  const int T = co < n ? co : tail_first(levels.data(), n);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int top = std::min(T, n - 1);
   // every launch's own status is checked, so an error left by the caller's earlier work is neither blamed on
@@ -114,7 +115,8 @@ extern "C" int fire_poisson_vcycles_noalloc(float* p, const float* b, int nx, in
       ok = ok && launch_restrict(levels[i], levels[i + 1], st) == cudaSuccess;
     }
     if (!ok) break;
-    if (T < n) ok = launch_tail(levels.data(), T, n, 2, 2, coarse, err, st) == cudaSuccess;
+    if (co < n) ok = launch_coarse(levels.data(), T, n, 2, 2, coarse, nullptr, 1, err, st) == cudaSuccess;
+    else if (T < n) ok = launch_tail(levels.data(), T, n, 2, 2, coarse, err, st) == cudaSuccess;
     else sweeps(levels[n - 1], coarse);
     for (int i = top - 1; i >= 0 && ok; --i) {
       ok = launch_prolong(levels[i], levels[i + 1], st) == cudaSuccess;

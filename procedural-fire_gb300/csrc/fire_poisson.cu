@@ -690,6 +690,7 @@ struct FirePoisson {
   std::vector<PLevel> levels;
   std::vector<MGLevel> mg;      // float view (levels >= tailFirst are FP32; all levels in the FP32 form)
   int tailFirst = 0;
+  bool coarse = false;          // levels [tailFirst, n) run in the register-resident coarse kernel, else in the tail kernel
   int coarseIters = 8;
   void* arena = nullptr;
   float4* partials = nullptr;
@@ -849,7 +850,9 @@ void ir_vcycle(FirePoisson* ps, bool zero_first, cudaStream_t st) {
     }
     prestrict(L[i], L[i + 1], st);
   }
-  if (T < n) {
+  if (ps->coarse) {
+    launch_coarse(ps->mg.data(), T, n, 2, 2, 0, ps->cinv, 1, ps->err, st);
+  } else if (T < n) {
     launch_tail(ps->mg.data(), T, n, 2, 2, COARSE64_SWEEPS, ps->err, st, true, ps->cinv);
   } else {
     for (int k = 0; k < ps->coarseIters; ++k) {
@@ -869,7 +872,8 @@ void fp32_vcycle(FirePoisson* ps, cudaStream_t st) {
     for (int k = 0; k < 2; ++k) { launch_smooth(ps->mg[i], 0, st); launch_smooth(ps->mg[i], 1, st); }
     launch_restrict(ps->mg[i], ps->mg[i + 1], st);
   }
-  if (T < n) launch_tail(ps->mg.data(), T, n, 2, 2, ps->coarseIters, ps->err, st);
+  if (ps->coarse) launch_coarse(ps->mg.data(), T, n, 2, 2, ps->coarseIters, nullptr, 1, ps->err, st);
+  else if (T < n) launch_tail(ps->mg.data(), T, n, 2, 2, ps->coarseIters, ps->err, st);
   else for (int k = 0; k < ps->coarseIters; ++k) { launch_smooth(ps->mg[n - 1], 0, st); launch_smooth(ps->mg[n - 1], 1, st); }
   for (int i = top - 1; i >= 0; --i) {
     launch_prolong(ps->mg[i], ps->mg[i + 1], st);
@@ -1061,7 +1065,12 @@ int fire_poisson_create(const int res[3], float h, int precision, int device, Fi
   std::vector<double> cinv;
   const MGLevel& C = ps->mg.back();
   const int ccells = C.nx * C.ny * C.nz;
-  const bool direct = ps->ir && ps->tailFirst < n && ccells <= COARSE_DIRECT_MAX && coarse_inverse(C, cinv);
+  // the coarse kernel takes the FP32 cycle, and the refinement's where the coarsest level gets its dense inverse
+  const bool small = ccells <= COARSE_DIRECT_MAX;
+  const int cf = !ps->ir || small ? coarse_first(ps->mg.data(), n, ps->ir) : n;
+  const bool direct = ps->ir && std::min(ps->tailFirst, cf) < n && small && coarse_inverse(C, cinv);
+  ps->coarse = cf < n && direct == ps->ir;
+  if (ps->coarse) ps->tailFirst = cf;
   // arena: level arrays (level 0 of the FP32 form is the caller's x and b), partials, state
   size_t off = 0;
   std::vector<size_t> pOff(n), bOff(n);
@@ -1107,7 +1116,7 @@ int fire_poisson_create(const int res[3], float h, int precision, int device, Fi
   ps->src = (float*)(A + srcOff);
   if (ps->ir) ps->xlo = (float*)(A + loOff);
   if (direct) ps->cinv = (double*)(A + cinvOff);
-  if (cudaMemset(ps->arena, 0, off) != cudaSuccess || mg_configure(TAIL_SMEM_BUDGET) != cudaSuccess ||
+  if (cudaMemset(ps->arena, 0, off) != cudaSuccess || mg_configure(TAIL_SMEM_BUDGET) != cudaSuccess || coarse_configure() != cudaSuccess ||
       cudaStreamCreateWithFlags(&ps->capStream, cudaStreamNonBlocking) != cudaSuccess ||
       (direct && cudaMemcpy(ps->cinv, cinv.data(), sizeof(double) * cinv.size(), cudaMemcpyHostToDevice) != cudaSuccess)) {
     fire_poisson_destroy(ps);
@@ -1186,6 +1195,7 @@ int fire_poisson_set_study(FirePoisson* ps, int coarse_sweeps) {
   for (MGLevel& L : ps->mg) L.study = 1;
   ps->coarseIters = coarse_sweeps;
   ps->tailFirst = tail_first(ps->mg.data(), (int)ps->mg.size(), false);   // single-CTA tails in this variant
+  ps->coarse = false;
   if (ps->exec) { cudaGraphExecDestroy(ps->exec); ps->exec = nullptr; }
   return FIRE_OK;
 }

@@ -22,6 +22,7 @@ SOURCES = {
     "fire_tables.cu": ["-fmad=false"],
     "fire_step.cu": [],
     "fire_mg.cu": [],
+    "fire_coarse.cu": [],
     "fire_stats.cu": [],
     "fire_api.cu": [],
     "fire_noalloc.cu": [],
