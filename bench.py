@@ -178,9 +178,8 @@ def make_sim(F, device: int, mg_fixed: int = 0):
 
 def launches_per_step(sim, cycles_per_step: float) -> float:
     """Kernels launched per step by the captured graph: 5 stencil kernels (the divergence kernel also clears
-    the solve's cycle count), and per V-cycle 10 per level above the coarse kernel (2 + 2 red-black sweeps of 2 colour launches each,
-    restriction, prolongation) less one per level below the finest (its first colour-0 sweep runs inside the
-    restriction onto it), the coarse kernel, the residual norm and the decision kernel.  The coarse kernel takes the
+    the solve's cycle count), and per V-cycle 4 per level above the coarse kernel (two sweeps in one launch before and after,
+    restriction, prolongation), the coarse kernel, the residual norm and the decision kernel.  The coarse kernel takes the
     levels whose half-row x z columns, times their groups of four rows per CTA of a 16-CTA cluster, fit 1024 threads."""
     T = len(sim.levels)
     while T > 0:
@@ -189,7 +188,7 @@ def launches_per_step(sim, cycles_per_step: float) -> float:
             break
         T -= 1
     top = min(T, len(sim.levels) - 1)
-    per_cycle = 10 * top - max(top - 1, 0) + (1 if T < len(sim.levels) else 0) + 2
+    per_cycle = 4 * top + (1 if T < len(sim.levels) else 0) + 2
     return 5 + per_cycle * cycles_per_step
 
 

@@ -182,33 +182,27 @@ int upload_block(FireSim* sim, float dt, cudaStream_t st, bool with_logs, const 
   return FIRE_OK;
 }
 
-// `iters` red-black sweeps of level l (src/sim.js:576-586): colour 0 then colour 1, one launch each; with
-// first_done the first colour-0 sweep has already been applied (by the fused restriction).
-void record_smooth(FireSim* s, int l, int iters, cudaStream_t st, bool first_done = false) {
+// `iters` red-black sweeps of level l (src/sim.js:576-586): colour 0 then colour 1, one launch each.
+void record_smooth(FireSim* s, int l, int iters, cudaStream_t st) {
   for (int k = 0; k < iters; ++k) {
-    if (k > 0 || !first_done) launch_smooth(s->levels[l], 0, st);
+    launch_smooth(s->levels[l], 0, st);
     launch_smooth(s->levels[l], 1, st);
   }
 }
 // Whether the coarse levels run in the register-resident coarse kernel; the TMA-staged tail takes over when nothing fits
 // it, and while its wait limit is lowered (fire_sim_set_tail_wait_limit exercises that kernel's bounded wait).
 bool use_coarse(const FireSim* s) { return s->coarseFirst < (int)s->levels.size() && s->tailWaitPolls == TAIL_WAIT_POLLS; }
-// One V(2,2) cycle (src/sim.js:588-599).  Levels [T, n) run inside one launch.  A restriction
-// onto a level that is smoothed by launches also applies that level's first colour-0 sweep.
+// One V(2,2) cycle (src/sim.js:588-599).  Levels [T, n) run inside one launch.
 void record_vcycle(FireSim* s, cudaStream_t st) {
   const int n = (int)s->levels.size();
   const bool co = use_coarse(s);
   const int T = co ? s->coarseFirst : s->tailFirst;
   const int top = std::min(T, n - 1);
-  for (int i = 0; i < top; ++i) {
-    record_smooth(s, i, 2, st, i > 0);
-    if (i + 1 < top) launch_restrict_smooth(s->levels[i], s->levels[i + 1], st);
-    else launch_restrict(s->levels[i], s->levels[i + 1], st);
-  }
+  launch_down(s->levels.data(), top, st);
   if (co) launch_coarse(s->levels.data(), T, n, 2, 2, s->coarseIters, nullptr, 1, s->dCounter + 2, st);
   else if (T < n) launch_tail(s->levels.data(), T, n, 2, 2, s->coarseIters, s->dCounter + 2, st, false, nullptr, s->tailWaitPolls);
   else record_smooth(s, n - 1, s->coarseIters, st);
-  for (int i = top - 1; i >= 0; --i) { launch_prolong(s->levels[i], s->levels[i + 1], st); record_smooth(s, i, 2, st); }
+  launch_up(s->levels.data(), top, st);
 }
 
 int record_ev(FireSim* sim, int idx, cudaStream_t st, bool prof) {
@@ -432,6 +426,8 @@ int fire_sim_create(const FireConfig* cfg, const float* logs, int n_logs, FireSi
     const int n = (int)sim->levels.size();
     sim->tailFirst = tail_first(sim->levels.data(), n);
     sim->coarseFirst = coarse_first(sim->levels.data(), n);
+    // every level but the coarsest may be smoothed by launches (all of them with the TMA-staged tail)
+    for (int l = 0; l < std::min(std::max(sim->coarseFirst, sim->tailFirst), n - 1); ++l) sim->levels[l].sweep = plan_sweep(sim->levels[l]);
   }
 
   // device arena
@@ -439,11 +435,12 @@ int fire_sim_create(const FireConfig* cfg, const float* logs, int n_logs, FireSi
   size_t off = 0;
   std::vector<size_t> fieldOff(11);
   for (int i = 0; i < 11; ++i) { fieldOff[i] = off; off = align_up(off + cells * sizeof(float4)); }
-  std::vector<size_t> pOff(sim->levels.size()), bOff(sim->levels.size());
+  std::vector<size_t> pOff(sim->levels.size()), bOff(sim->levels.size()), p2Off(sim->levels.size());
   for (size_t l = 0; l < sim->levels.size(); ++l) {
     size_t c = (size_t)sim->levels[l].nx * sim->levels[l].ny * sim->levels[l].nz;
     pOff[l] = off; off = align_up(off + c * sizeof(float));
     bOff[l] = off; off = align_up(off + c * sizeof(float));
+    if (sim->levels[l].sweep.px > 0) { p2Off[l] = off; off = align_up(off + c * sizeof(float)); }
   }
   const size_t tabBytes = (size_t)TABLE_N * TABLE_N * TABLE_N * sizeof(uint2);
   size_t solidOff = off; off = align_up(off + cells);
@@ -466,6 +463,7 @@ int fire_sim_create(const FireConfig* cfg, const float* logs, int n_logs, FireSi
   for (size_t l = 0; l < sim->levels.size(); ++l) {
     sim->levels[l].p = (float*)(A + pOff[l]);
     sim->levels[l].b = (float*)(A + bOff[l]);
+    if (sim->levels[l].sweep.px > 0) sim->levels[l].p2 = (float*)(A + p2Off[l]);
   }
   sim->noise = (uint2*)(A + noiseOff);
   sim->curl = (uint2*)(A + curlOff);
@@ -493,7 +491,7 @@ int fire_sim_create(const FireConfig* cfg, const float* logs, int n_logs, FireSi
       cudaEventCreateWithFlags(&sim->forkEv, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&sim->joinEv, cudaEventDisableTiming) != cudaSuccess)
     return fail(FIRE_ERR_CUDA);
-  if (mg_configure(TAIL_SMEM_BUDGET) != cudaSuccess || coarse_configure() != cudaSuccess) return fail(set_err(sim, FIRE_ERR_CUDA, "tail kernel smem opt-in failed"));
+  if (mg_configure(TAIL_SMEM_BUDGET) != cudaSuccess || coarse_configure() != cudaSuccess || sweep_configure() != cudaSuccess) return fail(set_err(sim, FIRE_ERR_CUDA, "tail kernel smem opt-in failed"));
   if (step_configure() != cudaSuccess) return fail(set_err(sim, FIRE_ERR_CUDA, "forces kernel smem opt-in failed"));
 
   // zero state (reset semantics), bake the tables (src/noise.js), upload logs

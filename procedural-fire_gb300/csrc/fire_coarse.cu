@@ -18,7 +18,7 @@
 //   * the levels below are gathered on CTA 0 and synchronised by a named barrier over just the warps that own cells; the
 //     coarse rows a CTA's prolongation reads are copied back once.
 // The arithmetic of every update, residual and prolongation is that of the launch-per-phase kernels of
-// fire_mg.cu, in the same order, written with explicit FMAs, so the cycle with omega 1 is bit-identical to theirs:
+// fire_mg.cu, in the same order, written with explicit FMAs, so the cycle is bit-identical to theirs:
 // __fdividef(a, d) equals a * rcp.approx(d) bit for bit for the diagonals 3..9 (checked over 2^30 values of a
 // for each), and a zero added for a missing neighbour does not change a sum that starts at +0.
 //
@@ -441,8 +441,9 @@ __device__ __forceinline__ void sweep_colour(Own<K>& o, const Slab& L, int c, bo
       sum = __fadd_rn(sum, n.zp[k]);
       sum = __fadd_rn(sum, nbr_ym(o, n, c, k));
       sum = __fadd_rn(sum, nbr_yp(o, n, c, k));
-      const float v = __fmul_rn(__fmaf_rn(-L.h2, o.b[c][k], sum), o.rd[c][k]);
-      o.p[c][k] = kRelax ? __fmaf_rn(L.omega, __fsub_rn(v, o.p[c][k]), o.p[c][k]) : v;
+      const float t = __fmaf_rn(-L.h2, o.b[c][k], sum);
+      // relaxed: the change t rd - p takes one rounding, as the single launches' contracted form does
+      o.p[c][k] = kRelax ? __fmaf_rn(L.omega, __fmaf_rn(t, o.rd[c][k], -o.p[c][k]), o.p[c][k]) : __fmul_rn(t, o.rd[c][k]);
     }
   }
   own_write<K, kSplit>(o, L, c, ex);

@@ -53,6 +53,12 @@ struct Fields {
 };
 struct Dims { int nx, ny, nz; };
 
+// How the two-sweep kernel (fire_sweep.cu) cuts a level into tiles; px == 0: the level is swept by colour launches.
+struct SweepPlan {
+  int px, ty;            // pairs of columns and thread rows of a block
+  int ntx, nty, ntz;     // tiles
+  int cx, cy, cz;        // cells of a tile that are written (the last ones of an axis may be fewer)
+};
 struct MGLevel {
   int nx, ny, nz;
   float h;
@@ -64,6 +70,8 @@ struct MGLevel {
   // prolongAdd): ghost values from the cell's old value, p <- mix(p, (sum_nb - h^2 b) / 6, omega), and
   // clamp-to-edge trilinear prolongation without sign flips.  Only the standalone solver's FP32 form sets it.
   int study = 0;
+  float* p2 = nullptr;  // where the two-sweep kernel writes, when it is used
+  SweepPlan sweep{};
 };
 
 // ---- batched launches over many independent simulations ----
@@ -139,9 +147,20 @@ void launch_forces_batch(const BatchMap& m, const StepBatch& I, const uint2* noi
 void launch_div_batch(const BatchMap& m, const StepBatch& I, int tile, cudaStream_t st);
 void launch_project_batch(const BatchMap& m, const StepBatch& I, int tile, cudaStream_t st);
 
+// ---- kernel launchers (fire_sweep.cu) ----
+// Two red-black sweeps from p (zero: from zero) into out; bit-identical to the four colour launches.
+SweepPlan plan_sweep(const MGLevel& L, int sms = 152);
+cudaError_t launch_sweep2(const MGLevel& L, const float* p, float* out, bool zero, cudaStream_t st);
+cudaError_t sweep_configure();
+
 // ---- kernel launchers (fire_mg.cu) ----
 cudaError_t launch_smooth(const MGLevel& L, int color, cudaStream_t st);
-cudaError_t launch_restrict(const MGLevel& F, const MGLevel& C, cudaStream_t st);
+// clear: the coarse pressure is set to zero (the two-sweep kernel does not read it).
+cudaError_t launch_restrict(const MGLevel& F, const MGLevel& C, cudaStream_t st, bool clear = true);
+// The levels a cycle smooths by launches, and back: two sweeps and the restriction of each onto the next, prolongation and two
+// sweeps.  Levels [0, top); level `top` receives its right-hand side and a pressure of zero.
+cudaError_t launch_down(const MGLevel* levels, int top, cudaStream_t st);
+cudaError_t launch_up(const MGLevel* levels, int top, cudaStream_t st);
 // Restriction fused with the coarse level's first colour-0 sweep (bit-identical to launch_restrict followed
 // by launch_smooth(C, 0)); not for study levels.
 cudaError_t launch_restrict_smooth(const MGLevel& F, const MGLevel& C, cudaStream_t st);
@@ -167,7 +186,7 @@ cudaError_t launch_tail(const MGLevel* levels, int first, int n, int pre, int po
 // The coarse end of the cycle with register-resident cells (fire_coarse.cu): levels [first, n) in one launch of one CTA
 // or one cluster.  coarse_first: the finest `first` it takes (n if none); direct: the coarsest level is solved with
 // a dense FP64 inverse (cinv).  `cycles` > 1 (first == 0 only) repeats the whole V-cycle inside the launch.
-// Bit-identical to the launch-per-phase kernels (omega 1).  `err` receives 1 if a bounded wait for a neighbouring CTA's rows ran out.
+// Bit-identical to the launch-per-phase kernels.  `err` receives 1 if a bounded wait for a neighbouring CTA's rows ran out.
 int coarse_first(const MGLevel* levels, int n, bool direct = false);
 bool coarse_fits(const MGLevel* levels, int first, int n, bool direct = false);
 cudaError_t launch_coarse(const MGLevel* levels, int first, int n, int pre, int post, int coarse, const double* cinv, int cycles,

@@ -132,7 +132,7 @@ __device__ __forceinline__ void restrict_body(const float* __restrict__ p, const
   const float ih2 = 1.0f / (h * h);
   const int t = cx + cnx * (cy + cny * cz);
   bc[t] = restrict_cell(p, b, cx, cy, cz, nx, ny, nz, ih2);
-  pc[t] = 0.0f;
+  if (pc) pc[t] = 0.0f;
 }
 // Restriction fused with the coarse level's first colour-0 sweep.  The coarse pressure starts at zero, so that
 // sweep's update of a colour-0 cell reads only the cell's own right-hand side: it is formed here from the value
@@ -1086,8 +1086,9 @@ cudaError_t launch_smooth(const MGLevel& L, int color, cudaStream_t st) {
                       L.omega);
   return launch_pdl(L.study ? k_smooth_study : k_smooth, g, kBlock, 0, st, L.p, (const float*)L.b, L.nx, L.ny, L.nz, L.h, color, L.omega);
 }
-cudaError_t launch_restrict(const MGLevel& F, const MGLevel& C, cudaStream_t st) {
-  return launch_pdl(k_restrict, grid3(C.nx, C.ny, C.nz), kBlock, 0, st, (const float*)F.p, (const float*)F.b, F.nx, F.ny, F.nz, F.h, C.b, C.p);
+cudaError_t launch_restrict(const MGLevel& F, const MGLevel& C, cudaStream_t st, bool clear) {
+  return launch_pdl(k_restrict, grid3(C.nx, C.ny, C.nz), kBlock, 0, st, (const float*)F.p, (const float*)F.b, F.nx, F.ny, F.nz, F.h, C.b,
+                    clear ? C.p : (float*)nullptr);
 }
 cudaError_t launch_restrict_smooth(const MGLevel& F, const MGLevel& C, cudaStream_t st) {
   if (C.study) return cudaErrorInvalidValue;   // the studies' smoother has its own update; not fused

@@ -23,6 +23,7 @@ SOURCES = {
     "fire_step.cu": [],
     "fire_mg.cu": [],
     "fire_coarse.cu": [],
+    "fire_sweep.cu": [],
     "fire_stats.cu": [],
     "fire_api.cu": [],
     "fire_noalloc.cu": [],

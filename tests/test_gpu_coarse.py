@@ -1,8 +1,7 @@
 """The register-resident coarse end of the V-cycle against the same cycle built from single multigrid operations.
 
 On these grids the V-cycle stage is one launch of the coarse kernel; the same cycle from `sweeps`, `restrict` and
-`prolong` launches performs the same operations in the same order, so with omega 1 the pressures agree bit for
-bit.  The grids sit at the kernel's edges: one CTA with one row per thread (8x16x8, 2x2x2) and with four (10x15x10: a
+`prolong` launches performs the same operations in the same order, so with omega 1 the pressures agree bit for bit.  The grids sit at the kernel's edges: one CTA with one row per thread (8x16x8, 2x2x2) and with four (10x15x10: a
 partial last group of rows), levels split over the cluster (16x32x16; 32x64x32: two of them; 12x24x12: fewer
 rows than CTAs; 64x16x16: half the CTAs), odd sizes (25x49x25, 33x47x29: a single level of 64 sweeps, a row that ends at an
 even x), the larger CTA sizes (40x60x40; 44x90x20), and many row groups on few columns (6x200x6).
