@@ -161,9 +161,6 @@ cudaError_t launch_restrict(const MGLevel& F, const MGLevel& C, cudaStream_t st,
 // sweeps.  Levels [0, top); level `top` receives its right-hand side and a pressure of zero.
 cudaError_t launch_down(const MGLevel* levels, int top, cudaStream_t st);
 cudaError_t launch_up(const MGLevel* levels, int top, cudaStream_t st);
-// Restriction fused with the coarse level's first colour-0 sweep (bit-identical to launch_restrict followed
-// by launch_smooth(C, 0)); not for study levels.
-cudaError_t launch_restrict_smooth(const MGLevel& F, const MGLevel& C, cudaStream_t st);
 cudaError_t launch_prolong(const MGLevel& F, const MGLevel& C, cudaStream_t st);
 // One launch runs the V-cycle over levels [first, n) out of shared memory: a single CTA when every level
 // fits in its shared memory, or a thread-block cluster whose CTAs each hold a z-slab of the finer tail

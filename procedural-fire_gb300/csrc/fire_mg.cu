@@ -19,6 +19,7 @@
 
 #include "fire_device.cuh"
 #include "fire_launch.cuh"
+#include "fire_level.cuh"
 
 namespace fire {
 
@@ -122,50 +123,6 @@ __device__ __forceinline__ float restrict_cell(const float* p, const float* b, i
   }
   return acc * 0.125f;
 }
-__device__ __forceinline__ void restrict_body(const float* __restrict__ p, const float* __restrict__ b, int nx, int ny, int nz, float h,
-                                              float* __restrict__ bc, float* __restrict__ pc, uint3 blk) {
-  pdl_wait();
-  pdl_trigger();
-  const int cnx = nx / 2, cny = ny / 2, cnz = nz / 2;
-  const int cx = blk.x * GX + threadIdx.x, cy = blk.y * GY + threadIdx.y, cz = blk.z * GZ + threadIdx.z;
-  if (cx >= cnx || cy >= cny || cz >= cnz) return;
-  const float ih2 = 1.0f / (h * h);
-  const int t = cx + cnx * (cy + cny * cz);
-  bc[t] = restrict_cell(p, b, cx, cy, cz, nx, ny, nz, ih2);
-  if (pc) pc[t] = 0.0f;
-}
-// Restriction fused with the coarse level's first colour-0 sweep.  The coarse pressure starts at zero, so that
-// sweep's update of a colour-0 cell reads only the cell's own right-hand side: it is formed here from the value
-// just restricted with the smoother's arithmetic (rb_update over zero neighbours: the same diagonal, the same
-// explicit FMA and quotient, the same relaxation from an old value of zero), so the result is bit-identical
-// to restricting and then sweeping.  Colour-1 cells keep zero.
-template <bool kRelax>
-__device__ __forceinline__ void restrict_smooth_body(const float* __restrict__ p, const float* __restrict__ b, int nx, int ny, int nz,
-                                                     float h, float* __restrict__ bc, float* __restrict__ pc, float hc, float omega,
-                                                     uint3 blk) {
-  pdl_wait();
-  pdl_trigger();
-  const int cnx = nx / 2, cny = ny / 2, cnz = nz / 2;
-  const int cx = blk.x * GX + threadIdx.x, cy = blk.y * GY + threadIdx.y, cz = blk.z * GZ + threadIdx.z;
-  if (cx >= cnx || cy >= cny || cz >= cnz) return;
-  const int t = cx + cnx * (cy + cny * cz);
-  const float r = restrict_cell(p, b, cx, cy, cz, nx, ny, nz, 1.0f / (h * h));
-  bc[t] = r;
-  float v = 0.0f;
-  if (((cx + cy + cz) & 1) == 0) {
-    float diag = 6.0f;   // rb_update's ghost rules: open sides and top add 1, the floor subtracts 1
-    if (cx == 0) diag += 1.0f;
-    if (cx == cnx - 1) diag += 1.0f;
-    if (cz == 0) diag += 1.0f;
-    if (cz == cnz - 1) diag += 1.0f;
-    if (cy == 0) diag -= 1.0f;
-    if (cy == cny - 1) diag += 1.0f;
-    v = __fdividef(__fmaf_rn(-(hc * hc), r, 0.0f), diag);
-    if (kRelax) v = fmaf(omega, v - 0.0f, 0.0f);
-  }
-  pc[t] = v;
-}
-
 // ---------------- prolongation with mirror ghosts (src/sim.js:468-495) ----------------
 template <bool kClamp = false>
 __device__ __forceinline__ float prolong_cell(const float* pc, int x, int y, int z, int ncx, int ncy, int ncz) {
@@ -190,52 +147,6 @@ __device__ __forceinline__ float prolong_cell(const float* pc, int x, int y, int
   }
   return acc;
 }
-// One thread per coarse cell: the 3x3x3 coarse neighbourhood (with the mirror signs of prolong_cell) is
-// loaded once and the 8 fine children are formed from it.  For fine index c = 2 cc + d the trilinear base is
-// g0 = cc - 1 + d with fraction 0.75 (d = 0) or 0.25 (d = 1), so child d reads coarse offsets d-1 and d;
-// each child's sum runs in prolong_cell's order, so the result is identical.
-template <bool kClamp = false>
-__device__ __forceinline__ void prolong_body(float* __restrict__ p, const float* __restrict__ pc, int nx, int ny, int nz, uint3 blk) {
-  pdl_wait();
-  pdl_trigger();
-  const int ncx = nx / 2, ncy = ny / 2, ncz = nz / 2;
-  const int cx = blk.x * GX + threadIdx.x, cy = blk.y * GY + threadIdx.y, cz = blk.z * GZ + threadIdx.z;
-  if (cx >= ncx || cy >= ncy || cz >= ncz) return;
-  float v[3][3][3];   // [dz][dy][dx] for offsets -1..1
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int bb = 0; bb < 3; ++bb)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const int qx = cx + c - 1, qy = cy + bb - 1, qz = cz + a - 1;
-        float val = __ldg(pc + min(max(qx, 0), ncx - 1) + ncx * (min(max(qy, 0), ncy - 1) + ncy * min(max(qz, 0), ncz - 1)));
-        if (!kClamp) {
-          if (qx < 0 || qx >= ncx) val = -val;
-          if (qz < 0 || qz >= ncz) val = -val;
-          if (qy >= ncy) val = -val;
-        }
-        v[a][bb][c] = val;
-      }
-#pragma unroll
-  for (int dz = 0; dz < 2; ++dz)
-#pragma unroll
-    for (int dy = 0; dy < 2; ++dy)
-#pragma unroll
-      for (int dx = 0; dx < 2; ++dx) {
-        const float fx = dx ? 0.25f : 0.75f, fy = dy ? 0.25f : 0.75f, fz = dz ? 0.25f : 0.75f;
-        float acc = 0.0f;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int ox = q & 1, oy = (q >> 1) & 1, oz = (q >> 2) & 1;
-          const float wx = ox ? fx : 1.0f - fx, wy = oy ? fy : 1.0f - fy, wz = oz ? fz : 1.0f - fz;
-          acc += v[dz + oz][dy + oy][dx + ox] * wx * wy * wz;
-        }
-        const int t = (2 * cx + dx) + nx * ((2 * cy + dy) + ny * (2 * cz + dz));
-        p[t] = p[t] + acc;
-      }
-}
-
 // Per-level kernels of one simulation, and their batched forms over many simulations (one grid; each CTA
 // finds its simulation's level from the BatchMap and runs the same body).
 __global__ void __launch_bounds__(GX * GY * GZ) k_smooth(float* __restrict__ p, const float* __restrict__ b, int nx, int ny, int nz, float h,
@@ -248,26 +159,19 @@ __global__ void __launch_bounds__(GX * GY * GZ) k_smooth1(float* __restrict__ p,
   if (omega == 1.0f) smooth_body_t<false, false, 1>(p, b, nx, ny, nz, h, color, blockIdx, omega);
   else smooth_body_t<true, false, 1>(p, b, nx, ny, nz, h, color, blockIdx, omega);
 }
-__global__ void __launch_bounds__(GX * GY * GZ) k_restrict(const float* __restrict__ p, const float* __restrict__ b, int nx, int ny, int nz,
+template <int kDepth, bool kPair>
+__global__ void __launch_bounds__(LX * LY * LZ) k_restrict(const float* __restrict__ p, const float* __restrict__ b, int nx, int ny, int nz,
                                                            float h, float* __restrict__ bc, float* __restrict__ pc) {
-  restrict_body(p, b, nx, ny, nz, h, bc, pc, blockIdx);
+  restrict_march<kDepth, kPair>(p, b, nx, ny, nz, h, bc, pc, blockIdx);
 }
-template <bool kRelax>
-__global__ void __launch_bounds__(GX * GY * GZ) k_restrict_smooth(const float* __restrict__ p, const float* __restrict__ b, int nx, int ny,
-                                                                  int nz, float h, float* __restrict__ bc, float* __restrict__ pc, float hc,
-                                                                  float omega) {
-  restrict_smooth_body<kRelax>(p, b, nx, ny, nz, h, bc, pc, hc, omega, blockIdx);
+template <int kDepth, bool kPair, bool kClamp>
+__global__ void __launch_bounds__(LX * LY * LZ) k_prolong(float* __restrict__ p, const float* __restrict__ pc, int nx, int ny, int nz) {
+  prolong_march<kDepth, kPair, kClamp>(p, pc, nx, ny, nz, blockIdx);
 }
-__global__ void __launch_bounds__(GX * GY * GZ) k_prolong(float* __restrict__ p, const float* __restrict__ pc, int nx, int ny, int nz) {
-  prolong_body(p, pc, nx, ny, nz, blockIdx);
-}
-// The convergence studies' smoother and prolongation (MGLevel::study).
+// The convergence studies' smoother (MGLevel::study).
 __global__ void __launch_bounds__(GX * GY * GZ) k_smooth_study(float* __restrict__ p, const float* __restrict__ b, int nx, int ny, int nz,
                                                                float h, int color, float omega) {
   smooth_body_t<false, true>(p, b, nx, ny, nz, h, color, blockIdx, omega);
-}
-__global__ void __launch_bounds__(GX * GY * GZ) k_prolong_clamp(float* __restrict__ p, const float* __restrict__ pc, int nx, int ny, int nz) {
-  prolong_body<true>(p, pc, nx, ny, nz, blockIdx);
 }
 __global__ void __launch_bounds__(GX * GY * GZ) k_smooth_b(const __grid_constant__ BatchMap m, const __grid_constant__ LevelBatch L, int color) {
   uint3 blk; int i;
@@ -275,17 +179,17 @@ __global__ void __launch_bounds__(GX * GY * GZ) k_smooth_b(const __grid_constant
   const MGLevel& v = L.l[i];
   smooth_body(v.p, v.b, v.nx, v.ny, v.nz, v.h, color, blk, v.omega);
 }
-__global__ void __launch_bounds__(GX * GY * GZ) k_restrict_b(const __grid_constant__ BatchMap m, const __grid_constant__ LevelBatch F,
+__global__ void __launch_bounds__(LX * LY * LZ) k_restrict_b(const __grid_constant__ BatchMap m, const __grid_constant__ LevelBatch F,
                                                              const __grid_constant__ LevelBatch C) {
   uint3 blk; int i;
   batch_locate(m, blk, i);
-  restrict_body(F.l[i].p, F.l[i].b, F.l[i].nx, F.l[i].ny, F.l[i].nz, F.l[i].h, C.l[i].b, C.l[i].p, blk);
+  restrict_march<TRANSFER_DEPTH, true>((const float*)F.l[i].p, (const float*)F.l[i].b, F.l[i].nx, F.l[i].ny, F.l[i].nz, F.l[i].h, C.l[i].b, C.l[i].p, blk);
 }
-__global__ void __launch_bounds__(GX * GY * GZ) k_prolong_b(const __grid_constant__ BatchMap m, const __grid_constant__ LevelBatch F,
+__global__ void __launch_bounds__(LX * LY * LZ) k_prolong_b(const __grid_constant__ BatchMap m, const __grid_constant__ LevelBatch F,
                                                             const __grid_constant__ LevelBatch C) {
   uint3 blk; int i;
   batch_locate(m, blk, i);
-  prolong_body(F.l[i].p, C.l[i].p, F.l[i].nx, F.l[i].ny, F.l[i].nz, blk);
+  prolong_march<TRANSFER_DEPTH, true, false>(F.l[i].p, (const float*)C.l[i].p, F.l[i].nx, F.l[i].ny, F.l[i].nz, blk);
 }
 
 // ---------------- single-CTA tail V-cycle out of shared memory ----------------
@@ -1072,6 +976,7 @@ __global__ void __launch_bounds__(RB) k_sum_decide(const float4* __restrict__ pa
 }
 
 // ---------------- launchers ----------------
+static_assert(LX == GX && LY == GY && LZ == GZ, "one CTA shape");
 static dim3 grid3(int x, int y, int z) { return dim3((x + GX - 1) / GX, (y + GY - 1) / GY, (z + GZ - 1) / GZ); }
 static const dim3 kBlock(GX, GY, GZ);
 
@@ -1086,17 +991,23 @@ cudaError_t launch_smooth(const MGLevel& L, int color, cudaStream_t st) {
                       L.omega);
   return launch_pdl(L.study ? k_smooth_study : k_smooth, g, kBlock, 0, st, L.p, (const float*)L.b, L.nx, L.ny, L.nz, L.h, color, L.omega);
 }
+// A caller's level-0 arrays may be aligned to 4 bytes only: pairs are then moved as two loads.
+static bool pair_aligned(const void* p, const void* b) { return ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(b)) & 7u) == 0; }
+static bool transfer_deep(const MGLevel& C) { return (long)C.nx * C.ny * C.nz >= TRANSFER_DEEP_CELLS; }
 cudaError_t launch_restrict(const MGLevel& F, const MGLevel& C, cudaStream_t st, bool clear) {
-  return launch_pdl(k_restrict, grid3(C.nx, C.ny, C.nz), kBlock, 0, st, (const float*)F.p, (const float*)F.b, F.nx, F.ny, F.nz, F.h, C.b,
-                    clear ? C.p : (float*)nullptr);
-}
-cudaError_t launch_restrict_smooth(const MGLevel& F, const MGLevel& C, cudaStream_t st) {
-  if (C.study) return cudaErrorInvalidValue;   // the studies' smoother has its own update; not fused
-  return launch_pdl(C.omega == 1.0f ? k_restrict_smooth<false> : k_restrict_smooth<true>, grid3(C.nx, C.ny, C.nz), kBlock, 0, st,
-                    (const float*)F.p, (const float*)F.b, F.nx, F.ny, F.nz, F.h, C.b, C.p, C.h, C.omega);
+  const bool deep = transfer_deep(C), pairs = pair_aligned(F.p, F.b);
+  return launch_pdl(!pairs ? k_restrict<1, false> : deep ? k_restrict<TRANSFER_DEPTH, true> : k_restrict<1, true>,
+                    transfer_grid(C.nx, C.ny, C.nz, pairs && deep ? TRANSFER_DEPTH : 1), kBlock, 0, st, (const float*)F.p, (const float*)F.b, F.nx,
+                    F.ny, F.nz, F.h, C.b, clear ? C.p : (float*)nullptr);
 }
 cudaError_t launch_prolong(const MGLevel& F, const MGLevel& C, cudaStream_t st) {
-  return launch_pdl(F.study ? k_prolong_clamp : k_prolong, grid3(C.nx, C.ny, C.nz), kBlock, 0, st, F.p, (const float*)C.p, F.nx, F.ny, F.nz);
+  const bool deep = transfer_deep(C), pairs = pair_aligned(F.p, nullptr);
+  auto go = [&](auto kernel, int depth) {
+    return launch_pdl(kernel, transfer_grid(C.nx, C.ny, C.nz, depth), kBlock, 0, st, F.p, (const float*)C.p, F.nx, F.ny, F.nz);
+  };
+  if (F.study) return pairs ? go(k_prolong<1, true, true>, 1) : go(k_prolong<1, false, true>, 1);
+  if (!pairs) return go(k_prolong<1, false, false>, 1);
+  return deep ? go(k_prolong<TRANSFER_DEPTH, true, false>, TRANSFER_DEPTH) : go(k_prolong<1, true, false>, 1);
 }
 // Number of leading levels of [first, n) that the cluster tail distributes: each has z-planes for an even
 // number per CTA, at least CTAIL_MIN_CELLS cells per CTA, and a coarser level below it.
@@ -1215,7 +1126,7 @@ cudaError_t mg_configure(size_t max_tail_smem) {
   return cudaSuccess;
 }
 dim3 smooth_grid(const MGLevel& L) { return grid3((L.nx + 1) >> 1, L.ny, (L.nz + SMZ - 1) / SMZ); }
-dim3 coarse_grid(const MGLevel& C) { return grid3(C.nx, C.ny, C.nz); }
+dim3 coarse_grid(const MGLevel& C) { return transfer_grid(C.nx, C.ny, C.nz, TRANSFER_DEPTH); }
 void launch_smooth_batch(const BatchMap& m, const LevelBatch& L, int color, cudaStream_t st) {
   launch_pdl(k_smooth_b, dim3(m.prefix[m.n]), kBlock, 0, st, m, L, color);
 }

@@ -22,6 +22,7 @@
 #include <algorithm>
 #include "fire_device.cuh"
 #include "fire_launch.cuh"
+#include "fire_level.cuh"
 
 namespace fire {
 namespace {
@@ -32,13 +33,6 @@ constexpr int SW_THREADS = 512;   // 128 registers a thread
 constexpr int SW_AHEAD = 4;       // planes of p and b in flight: a step takes about 0.3 us, a load from L2 0.4 and more
 constexpr int SW_RING = 7;        // entries a thread's ring is long: six planes, and one more so that 32 lanes hit all banks
 
-// Two neighbouring cells of a row in storage T: copied to shared memory as they are, widened to FP32 when read from there.
-template <typename T> struct Cells2;
-template <> struct Cells2<float> {
-  using V = float2;
-  static __device__ __forceinline__ float2 get(V v) { return v; }
-  static __device__ __forceinline__ V put(float2 v) { return v; }
-};
 // Asynchronous copy of one pair; zeros where it lies outside the domain.
 template <typename V>
 __device__ __forceinline__ void copy_pair(V* dst, const void* src, bool in) {
@@ -298,12 +292,9 @@ cudaError_t launch_sweep2(const MGLevel& L, const float* p, float* out, bool zer
   return launch_sweep2_t<float>(p, L.b, out, L.sweep, L.nx, L.ny, L.nz, L.h, L.omega, zero, st);
 }
 
-static cudaError_t sweeps_by_launches(const MGLevel& L, bool first_done, cudaStream_t st) {
+static cudaError_t sweeps_by_launches(const MGLevel& L, cudaStream_t st) {
   cudaError_t e = cudaSuccess;
-  for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
-    if (k > 0 || !first_done) e = launch_smooth(L, 0, st);
-    if (e == cudaSuccess) e = launch_smooth(L, 1, st);
-  }
+  for (int k = 0; k < 4 && e == cudaSuccess; ++k) e = launch_smooth(L, k & 1, st);
   return e;
 }
 static MGLevel on_p2(MGLevel L) {
@@ -312,16 +303,12 @@ static MGLevel on_p2(MGLevel L) {
 }
 cudaError_t launch_down(const MGLevel* levels, int top, cudaStream_t st) {
   cudaError_t e = cudaSuccess;
-  bool first_done = false;   // the restriction onto this level has already applied its first colour-0 sweep
   for (int i = 0; i < top && e == cudaSuccess; ++i) {
     const MGLevel& L = levels[i];
     const bool two = L.sweep.px > 0;
-    e = two ? launch_sweep2(L, L.p, L.p2, i > 0, st) : sweeps_by_launches(L, first_done, st);
-    if (e != cudaSuccess) break;
-    const MGLevel F = two ? on_p2(L) : L;
-    const MGLevel& C = levels[i + 1];
-    first_done = i + 1 < top && C.sweep.px == 0;
-    e = first_done ? launch_restrict_smooth(F, C, st) : launch_restrict(F, C, st, i + 1 == top);
+    e = two ? launch_sweep2(L, L.p, L.p2, i > 0, st) : sweeps_by_launches(L, st);
+    // a level that starts with the two-sweep kernel does not read its pressure
+    if (e == cudaSuccess) e = launch_restrict(two ? on_p2(L) : L, levels[i + 1], st, i + 1 == top || levels[i + 1].sweep.px == 0);
   }
   return e;
 }
@@ -331,7 +318,7 @@ cudaError_t launch_up(const MGLevel* levels, int top, cudaStream_t st) {
     const MGLevel& L = levels[i];
     const bool two = L.sweep.px > 0;
     e = launch_prolong(two ? on_p2(L) : L, levels[i + 1], st);
-    if (e == cudaSuccess) e = two ? launch_sweep2(L, L.p2, L.p, false, st) : sweeps_by_launches(L, false, st);
+    if (e == cudaSuccess) e = two ? launch_sweep2(L, L.p2, L.p, false, st) : sweeps_by_launches(L, st);
   }
   return e;
 }
