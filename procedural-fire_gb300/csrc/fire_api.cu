@@ -201,7 +201,7 @@ void record_vcycle(FireSim* s, cudaStream_t st) {
   launch_down(s->levels.data(), top, st);
   if (co) launch_coarse(s->levels.data(), T, n, 2, 2, s->coarseIters, nullptr, 1, s->dCounter + 2, st);
   else if (T < n) launch_tail(s->levels.data(), T, n, 2, 2, s->coarseIters, s->dCounter + 2, st, false, nullptr, s->tailWaitPolls);
-  else record_smooth(s, n - 1, s->coarseIters, st);
+  else launch_sweeps(s->levels[n - 1], s->coarseIters, st);
   launch_up(s->levels.data(), top, st);
 }
 
@@ -426,8 +426,8 @@ int fire_sim_create(const FireConfig* cfg, const float* logs, int n_logs, FireSi
     const int n = (int)sim->levels.size();
     sim->tailFirst = tail_first(sim->levels.data(), n);
     sim->coarseFirst = coarse_first(sim->levels.data(), n);
-    // every level but the coarsest may be smoothed by launches (all of them with the TMA-staged tail)
-    for (int l = 0; l < std::min(std::max(sim->coarseFirst, sim->tailFirst), n - 1); ++l) sim->levels[l].sweep = plan_sweep(sim->levels[l]);
+    // every level outside the coarse kernel or the TMA-staged tail, whichever is in use, is smoothed by launches
+    for (int l = 0; l < std::max(sim->coarseFirst, sim->tailFirst); ++l) sim->levels[l].sweep = plan_sweep(sim->levels[l]);
   }
 
   // device arena

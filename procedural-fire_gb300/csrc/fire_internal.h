@@ -151,6 +151,12 @@ void launch_project_batch(const BatchMap& m, const StepBatch& I, int tile, cudaS
 // Two red-black sweeps from p (zero: from zero) into out; bit-identical to the four colour launches.
 SweepPlan plan_sweep(const MGLevel& L, int sms = 152);
 cudaError_t launch_sweep2(const MGLevel& L, const float* p, float* out, bool zero, cudaStream_t st);
+// The same on a level's arrays in storage T (float, __half, __nv_bfloat16; omega 1 for the last two).
+template <typename T>
+cudaError_t launch_sweep2_t(const T* p, const T* b, T* out, const SweepPlan& P, int nx, int ny, int nz, float h, float omega, bool zero,
+                            cudaStream_t st);
+// `iters` sweeps in place, two-sweep launches as far as the level has a plan.
+cudaError_t launch_sweeps(const MGLevel& L, int iters, cudaStream_t st);
 cudaError_t sweep_configure();
 
 // ---- kernel launchers (fire_mg.cu) ----

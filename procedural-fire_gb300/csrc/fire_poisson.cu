@@ -15,6 +15,11 @@
 // where each test is one small kernel that sums the residual partials in a fixed order (double-float),
 // updates the scales and sets the conditional node's value.  The FP32 form runs the step's own V-cycle on
 // (x, b) with the same pre-pass and test.
+// The cycles run the step's kernels on the storage types: two sweeps per pass (fire_sweep.cu; each value is rounded to the
+// storage type where a colour launch would have stored it), marched transfers (fire_level.cuh), the coarse kernel.  All
+// levels are in the plain layout: with one pass per two sweeps a red-black split saves no bytes, and plain pairs serve every
+// kernel.  Measured (GB300, whole solves, colour launches on a split level 0 -> this): 256x512x256 with FP32 storage 7.20 ->
+// 4.98 ms, 128x256x128 with half 1.38 -> 1.06 ms; FP32 form at 64x128x64 296 -> 283 us.
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
 #include <cmath>
@@ -27,10 +32,15 @@
 #include "fire_internal.h"
 #include "fire_device.cuh"
 #include "fire_launch.cuh"
+#include "fire_level.cuh"
 #include "fire_nvtx.h"
 
 namespace fire {
 namespace {
+
+// Loads widen to FP32, stores round to nearest.
+template <typename T> __device__ __forceinline__ float ld(const T* p) { return Cells2<T>::one(*p); }
+template <typename T> __device__ __forceinline__ void st(T* p, float v) { *p = Cells2<T>::back(v); }
 
 constexpr int GX = 32, GY = 4, GZ = 2, NT = GX * GY * GZ;
 constexpr int SMZ = 2;   // cells of one colour per smoother thread (as the step's smoother)
@@ -38,37 +48,7 @@ constexpr int RZ = 8;    // z-planes per residual thread
 constexpr int SUMSQ_CTAS = 1024;
 constexpr int COARSE64_SWEEPS = 64;
 
-// ---- storage types: loads widen to FP32, stores round to nearest ----
-template <typename T> struct Sto;
-template <> struct Sto<float> {
-  static __device__ __forceinline__ float ld(const float* p) { return *p; }
-  static __device__ __forceinline__ void st(float* p, float v) { *p = v; }
-};
-template <> struct Sto<__half> {
-  static __device__ __forceinline__ float ld(const __half* p) { return __half2float(*p); }
-  static __device__ __forceinline__ void st(__half* p, float v) { *p = __float2half_rn(v); }
-};
-template <> struct Sto<__nv_bfloat16> {
-  static __device__ __forceinline__ float ld(const __nv_bfloat16* p) { return __bfloat162float(*p); }
-  static __device__ __forceinline__ void st(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
-};
-
-// A level's array in one of two layouts.  Plain: x fastest, then y, then z.  Red-black split (even nx): the
-// cells of colour (x + y + z) & 1 == c are stored contiguously in half c (nx/2 * ny * nz elements each) at
-// (x >> 1) + (nx/2) * (y + ny * z), so a colour sweep reads one half, writes the other with unit stride and
-// touches each byte once (the interleaved layout moves whole cache lines of both colours every sweep).
-template <typename T>
-struct LV {
-  T* a;
-  int nx, ny, nz, split;
-  __device__ __forceinline__ T* at(int x, int y, int z) const {
-    if (!split) return a + (x + nx * (y + ny * z));
-    const int hx = nx >> 1;
-    return a + (((x + y + z) & 1) ? hx * ny * nz : 0) + (x >> 1) + hx * (y + ny * z);
-  }
-};
-
-// Red-black sweep of one colour (mgSmooth, src/sim.js:417-437) on T storage in the plain layout.  zero_nbrs:
+// Red-black sweep of one colour (mgSmooth, src/sim.js:417-437) on T storage, for levels the two-sweep kernel does not take.  zero_nbrs:
 // the level's current values are taken as zero (the first half-sweep of a correction solve from e = 0: the
 // colour being updated never reads its own old value, so the other colour's stale contents are not read).
 template <typename T>
@@ -90,312 +70,31 @@ __global__ void __launch_bounds__(NT) k_psmooth(T* __restrict__ p, const T* __re
       const int c = x + y * sy + z * sz;
       float sum = 0.0f, diag = 6.0f;
       const bool rd = !zero_nbrs;
-      if (x > 0) { if (rd) sum += Sto<T>::ld(p + c - 1); } else diag += 1.0f;
-      if (x < nx - 1) { if (rd) sum += Sto<T>::ld(p + c + 1); } else diag += 1.0f;
-      if (z > 0) { if (rd) sum += Sto<T>::ld(p + c - sz); } else diag += 1.0f;
-      if (z < nz - 1) { if (rd) sum += Sto<T>::ld(p + c + sz); } else diag += 1.0f;
-      if (y > 0) { if (rd) sum += Sto<T>::ld(p + c - sy); } else diag -= 1.0f;
-      if (y < ny - 1) { if (rd) sum += Sto<T>::ld(p + c + sy); } else diag += 1.0f;
-      v[k] = __fdividef(sum - h2 * Sto<T>::ld(b + c), diag);
+      if (x > 0) { if (rd) sum += ld(p + c - 1); } else diag += 1.0f;
+      if (x < nx - 1) { if (rd) sum += ld(p + c + 1); } else diag += 1.0f;
+      if (z > 0) { if (rd) sum += ld(p + c - sz); } else diag += 1.0f;
+      if (z < nz - 1) { if (rd) sum += ld(p + c + sz); } else diag += 1.0f;
+      if (y > 0) { if (rd) sum += ld(p + c - sy); } else diag -= 1.0f;
+      if (y < ny - 1) { if (rd) sum += ld(p + c + sy); } else diag += 1.0f;
+      v[k] = __fdividef(sum - h2 * ld(b + c), diag);
     }
   }
 #pragma unroll
   for (int k = 0; k < SMZ; ++k) {
     const int z = zb + k;
     const int x = gx * 2 + ((y + z + color) & 1);
-    if (z < nz && x < nx) Sto<T>::st(p + x + sy * y + sz * z, v[k]);
+    if (z < nz && x < nx) st(p + x + sy * y + sz * z, v[k]);
   }
 }
-// The same sweep on the red-black split layout: a thread updates the colour cell at half-index gx of SMZ
-// rows; its x neighbours are the other colour's entries gx - 1 + s and gx + s (s = the cell's x parity),
-// its y and z neighbours the other colour's entry gx of the adjacent rows.
-template <typename T, bool kZero>
-__global__ void __launch_bounds__(NT) k_psmooth_rb(T* __restrict__ p, const T* __restrict__ b, int nx, int ny, int nz, float h, int color) {
-  pdl_wait();
-  pdl_trigger();
-  const int hx = nx >> 1, half = hx * ny * nz, ry = hx, rz = hx * ny;
-  const int gx = blockIdx.x * GX + threadIdx.x, y = blockIdx.y * GY + threadIdx.y;
-  const int zb = (blockIdx.z * GZ + threadIdx.z) * SMZ;
-  if (gx >= hx || y >= ny) return;
-  T* __restrict__ pc = p + color * half;
-  const T* __restrict__ po = p + (1 - color) * half;
-  const T* __restrict__ bc = b + color * half;
-  const float h2 = h * h;
-  float v[SMZ];
-#pragma unroll
-  for (int k = 0; k < SMZ; ++k) {
-    const int z = zb + k;
-    if (z < nz) {
-      const int s = (y + z + color) & 1;
-      const int r = gx + ry * y + rz * z;
-      float sum = 0.0f, diag = 6.0f;
-      if (gx > 0 || s) { if (!kZero) sum += Sto<T>::ld(po + r - 1 + s); } else diag += 1.0f;
-      if (gx < hx - 1 || !s) { if (!kZero) sum += Sto<T>::ld(po + r + s); } else diag += 1.0f;
-      if (z > 0) { if (!kZero) sum += Sto<T>::ld(po + r - rz); } else diag += 1.0f;
-      if (z < nz - 1) { if (!kZero) sum += Sto<T>::ld(po + r + rz); } else diag += 1.0f;
-      if (y > 0) { if (!kZero) sum += Sto<T>::ld(po + r - ry); } else diag -= 1.0f;
-      if (y < ny - 1) { if (!kZero) sum += Sto<T>::ld(po + r + ry); } else diag += 1.0f;
-      v[k] = __fdividef(sum - h2 * Sto<T>::ld(bc + r), diag);
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < SMZ; ++k) {
-    const int z = zb + k;
-    if (z < nz) Sto<T>::st(pc + gx + ry * y + rz * z, v[k]);
-  }
+// The transfers between levels of any two storage types (fire_level.cuh).
+template <int kDepth, typename TF, typename TC>
+__global__ void __launch_bounds__(NT) k_prestrict(const TF* __restrict__ p, const TF* __restrict__ b, int nx, int ny, int nz, float h,
+                                                  TC* __restrict__ bc, TC* __restrict__ pc) {
+  restrict_march<kDepth, true>(p, b, nx, ny, nz, h, bc, pc, blockIdx);
 }
-
-// Two adjacent entries (2 g, 2 g + 1) as one 4- or 8-byte load / store.
-template <typename T> struct Pair;
-template <> struct Pair<float> {
-  static __device__ __forceinline__ float2 ld(const float* p) { return *reinterpret_cast<const float2*>(p); }
-  static __device__ __forceinline__ void st(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
-};
-template <> struct Pair<__half> {
-  static __device__ __forceinline__ float2 ld(const __half* p) { return __half22float2(*reinterpret_cast<const __half2*>(p)); }
-  static __device__ __forceinline__ void st(__half* p, float a, float b) { *reinterpret_cast<__half2*>(p) = __floats2half2_rn(a, b); }
-};
-template <> struct Pair<__nv_bfloat16> {
-  static __device__ __forceinline__ float2 ld(const __nv_bfloat16* p) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)); }
-  static __device__ __forceinline__ void st(__nv_bfloat16* p, float a, float b) {
-    *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(a, b);
-  }
-};
-// k_psmooth_rb with a pair of same-colour cells (half-indices 2 g, 2 g + 1 of one row) per thread and SMZ
-// rows: b, the y and z neighbours and the result move as pairs; the three x neighbours of the pair are one
-// pair plus one scalar of the other colour (which side depends on the row's x parity s).  Needs nx % 4 == 0
-// so every colour half and row starts at an even entry.  Same arithmetic and order as k_psmooth_rb.
-template <typename T, bool kZero>
-__global__ void __launch_bounds__(NT) k_psmooth_rb2(T* __restrict__ p, const T* __restrict__ b, int nx, int ny, int nz, float h, int color) {
-  pdl_wait();
-  pdl_trigger();
-  const int hx = nx >> 1, half = hx * ny * nz, ry = hx, rz = hx * ny;
-  const int g = blockIdx.x * GX + threadIdx.x, y = blockIdx.y * GY + threadIdx.y;
-  const int zb = (blockIdx.z * GZ + threadIdx.z) * SMZ;
-  const int gx = 2 * g;
-  if (gx >= hx || y >= ny) return;
-  T* __restrict__ pc = p + color * half;
-  const T* __restrict__ po = p + (1 - color) * half;
-  const T* __restrict__ bc = b + color * half;
-  const float h2 = h * h;
-  float v0[SMZ], v1[SMZ];
-#pragma unroll
-  for (int k = 0; k < SMZ; ++k) {
-    const int z = zb + k;
-    if (z < nz) {
-      const int s = (y + z + color) & 1;
-      const int r = gx + ry * y + rz * z;
-      float2 o = make_float2(0.0f, 0.0f), ym = o, yp = o, zm = o, zp = o;
-      float side = 0.0f;
-      // x neighbours: s = 0 -> entries 2g-1 (cell 0's x-), 2g, 2g+1; s = 1 -> 2g, 2g+1, 2g+2 (cell 1's x+)
-      const bool cell0_xm = gx > 0 || s, cell1_xp = gx + 1 < hx - 1 || !s;
-      if (!kZero) {
-        o = Pair<T>::ld(po + r);
-        if (!s && cell0_xm) side = Sto<T>::ld(po + r - 1);
-        if (s && cell1_xp) side = Sto<T>::ld(po + r + 2);
-        if (z > 0) zm = Pair<T>::ld(po + r - rz);
-        if (z < nz - 1) zp = Pair<T>::ld(po + r + rz);
-        if (y > 0) ym = Pair<T>::ld(po + r - ry);
-        if (y < ny - 1) yp = Pair<T>::ld(po + r + ry);
-      }
-      const float2 bv = Pair<T>::ld(bc + r);
-      // cell 0 (half-index 2g): x- = s ? o.x : side, x+ = s ? o.y : o.x
-      {
-        float sum = 0.0f, diag = 6.0f;
-        if (cell0_xm) { if (!kZero) sum += s ? o.x : side; } else diag += 1.0f;
-        if (!kZero) sum += s ? o.y : o.x;   // x+ of cell 0 always exists (cell 1 follows it)
-        if (z > 0) { if (!kZero) sum += zm.x; } else diag += 1.0f;
-        if (z < nz - 1) { if (!kZero) sum += zp.x; } else diag += 1.0f;
-        if (y > 0) { if (!kZero) sum += ym.x; } else diag -= 1.0f;
-        if (y < ny - 1) { if (!kZero) sum += yp.x; } else diag += 1.0f;
-        v0[k] = __fdividef(sum - h2 * bv.x, diag);
-      }
-      // cell 1 (half-index 2g+1): x- = s ? o.y : o.x, x+ = s ? side : o.y
-      {
-        float sum = 0.0f, diag = 6.0f;
-        if (!kZero) sum += s ? o.y : o.x;   // x- of cell 1 always exists
-        if (cell1_xp) { if (!kZero) sum += s ? side : o.y; } else diag += 1.0f;
-        if (z > 0) { if (!kZero) sum += zm.y; } else diag += 1.0f;
-        if (z < nz - 1) { if (!kZero) sum += zp.y; } else diag += 1.0f;
-        if (y > 0) { if (!kZero) sum += ym.y; } else diag -= 1.0f;
-        if (y < ny - 1) { if (!kZero) sum += yp.y; } else diag += 1.0f;
-        v1[k] = __fdividef(sum - h2 * bv.y, diag);
-      }
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < SMZ; ++k) {
-    const int z = zb + k;
-    if (z < nz) Pair<T>::st(pc + gx + ry * y + rz * z, v0[k], v1[k]);
-  }
-}
-
-template <typename T>
-__device__ __forceinline__ float pgv(const LV<T>& L, int x, int y, int z, float me) {
-  if (x < 0 || z < 0 || x >= L.nx || z >= L.nz || y >= L.ny) return -me;
-  if (y < 0) return me;
-  return Sto<T>::ld(L.at(x, y, z));
-}
-// Fused residual + 8-child restriction (src/sim.js:439-466); coarse p set to 0.  Either level in either layout.
-template <typename TF, typename TC>
-__global__ void __launch_bounds__(NT) k_prestrict(const TF* __restrict__ p, const TF* __restrict__ b, int fsplit, int nx, int ny, int nz,
-                                                  float h, TC* __restrict__ bc, TC* __restrict__ pc, int csplit) {
-  pdl_wait();
-  pdl_trigger();
-  const int cnx = nx / 2, cny = ny / 2, cnz = nz / 2;
-  const int cx = blockIdx.x * GX + threadIdx.x, cy = blockIdx.y * GY + threadIdx.y, cz = blockIdx.z * GZ + threadIdx.z;
-  if (cx >= cnx || cy >= cny || cz >= cnz) return;
-  const LV<TF> P{const_cast<TF*>(p), nx, ny, nz, fsplit}, B{const_cast<TF*>(b), nx, ny, nz, fsplit};
-  const float ih2 = 1.0f / (h * h);
-  float acc = 0.0f;
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int x = 2 * cx + (q & 1), y = 2 * cy + ((q >> 1) & 1), z = 2 * cz + ((q >> 2) & 1);
-    const float me = Sto<TF>::ld(P.at(x, y, z));
-    const float lap = (pgv(P, x - 1, y, z, me) + pgv(P, x + 1, y, z, me) + pgv(P, x, y - 1, z, me) + pgv(P, x, y + 1, z, me) +
-                       pgv(P, x, y, z - 1, me) + pgv(P, x, y, z + 1, me) - 6.0f * me) * ih2;
-    acc += Sto<TF>::ld(B.at(x, y, z)) - lap;
-  }
-  const LV<TC> PC{pc, cnx, cny, cnz, csplit}, BC{bc, cnx, cny, cnz, csplit};
-  Sto<TC>::st(BC.at(cx, cy, cz), acc * 0.125f);
-  Sto<TC>::st(PC.at(cx, cy, cz), 0.0f);
-}
-// Trilinear prolongation with mirror ghosts (src/sim.js:468-495), coarse-cell centric as the step's k_prolong.
-template <typename TF, typename TC>
-__global__ void __launch_bounds__(NT) k_pprolong(TF* __restrict__ p, int fsplit, const TC* __restrict__ pc, int csplit, int nx, int ny, int nz) {
-  pdl_wait();
-  pdl_trigger();
-  const int ncx = nx / 2, ncy = ny / 2, ncz = nz / 2;
-  const int cx = blockIdx.x * GX + threadIdx.x, cy = blockIdx.y * GY + threadIdx.y, cz = blockIdx.z * GZ + threadIdx.z;
-  if (cx >= ncx || cy >= ncy || cz >= ncz) return;
-  const LV<TC> C{const_cast<TC*>(pc), ncx, ncy, ncz, csplit};
-  const LV<TF> F{p, nx, ny, nz, fsplit};
-  float v[3][3][3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int bb = 0; bb < 3; ++bb)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const int qx = cx + c - 1, qy = cy + bb - 1, qz = cz + a - 1;
-        float val = Sto<TC>::ld(C.at(min(max(qx, 0), ncx - 1), min(max(qy, 0), ncy - 1), min(max(qz, 0), ncz - 1)));
-        if (qx < 0 || qx >= ncx) val = -val;
-        if (qz < 0 || qz >= ncz) val = -val;
-        if (qy >= ncy) val = -val;
-        v[a][bb][c] = val;
-      }
-#pragma unroll
-  for (int dz = 0; dz < 2; ++dz)
-#pragma unroll
-    for (int dy = 0; dy < 2; ++dy)
-#pragma unroll
-      for (int dx = 0; dx < 2; ++dx) {
-        const float fx = dx ? 0.25f : 0.75f, fy = dy ? 0.25f : 0.75f, fz = dz ? 0.25f : 0.75f;
-        float acc = 0.0f;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int ox = q & 1, oy = (q >> 1) & 1, oz = (q >> 2) & 1;
-          const float wx = ox ? fx : 1.0f - fx, wy = oy ? fy : 1.0f - fy, wz = oz ? fz : 1.0f - fz;
-          acc += v[dz + oz][dy + oy][dx + ox] * wx * wy * wz;
-        }
-        TF* pf = F.at(2 * cx + dx, 2 * cy + dy, 2 * cz + dz);
-        Sto<TF>::st(pf, Sto<TF>::ld(pf) + acc);
-      }
-}
-
-// Value of cell (x, y, z) of a red-black split level (half = nx/2 * ny * nz, hx = nx/2).
-template <typename T>
-__device__ __forceinline__ float ld_rb(const T* p, int half, int hx, int ny, int x, int y, int z) {
-  return Sto<T>::ld(p + (((x + y + z) & 1) ? half : 0) + (x >> 1) + hx * (y + ny * z));
-}
-// Fused residual + 8-child restriction (src/sim.js:439-466) from a red-black split fine level into a plain
-// coarse level.  The 32 distinct fine values the 8 children and their faces need (a 4x4x4 block without
-// its edges and corners) are loaded once into v[z][y][x] (offsets -1..2 around the children); the
-// arithmetic and its order are k_prestrict's, so the results are identical.
-template <typename TF, typename TC>
-__global__ void __launch_bounds__(NT) k_prestrict_rb(const TF* __restrict__ p, const TF* __restrict__ b, int nx, int ny, int nz, float h,
-                                                     TC* __restrict__ bc, TC* __restrict__ pc) {
-  pdl_wait();
-  pdl_trigger();
-  const int cnx = nx / 2, cny = ny / 2, cnz = nz / 2;
-  const int cx = blockIdx.x * GX + threadIdx.x, cy = blockIdx.y * GY + threadIdx.y, cz = blockIdx.z * GZ + threadIdx.z;
-  if (cx >= cnx || cy >= cny || cz >= cnz) return;
-  const int hx = nx >> 1, half = hx * ny * nz;
-  const int x0 = 2 * cx - 1, y0 = 2 * cy - 1, z0 = 2 * cz - 1;
-  float v[4][4][4];
-#pragma unroll
-  for (int iz = 0; iz < 4; ++iz)
-#pragma unroll
-    for (int iy = 0; iy < 4; ++iy)
-#pragma unroll
-      for (int ix = 0; ix < 4; ++ix) {
-        const bool cz_ = iz == 1 || iz == 2, cy_ = iy == 1 || iy == 2, cx_ = ix == 1 || ix == 2;
-        const int inner = (cz_ ? 1 : 0) + (cy_ ? 1 : 0) + (cx_ ? 1 : 0);
-        v[iz][iy][ix] = 0.0f;
-        if (inner >= 2) {   // children (inner == 3) and their face neighbours (inner == 2)
-          const int x = x0 + ix, y = y0 + iy, z = z0 + iz;
-          if (x >= 0 && x < nx && y >= 0 && y < ny && z >= 0 && z < nz) v[iz][iy][ix] = ld_rb(p, half, hx, ny, x, y, z);
-        }
-      }
-  const float ih2 = 1.0f / (h * h);
-  float acc = 0.0f;
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int dx = q & 1, dy = (q >> 1) & 1, dz = (q >> 2) & 1;
-    const int ix = 1 + dx, iy = 1 + dy, iz = 1 + dz;
-    const int x = 2 * cx + dx, y = 2 * cy + dy, z = 2 * cz + dz;
-    const float me = v[iz][iy][ix];
-    const float gxm = x > 0 ? v[iz][iy][ix - 1] : -me, gxp = x < nx - 1 ? v[iz][iy][ix + 1] : -me;
-    const float gym = y > 0 ? v[iz][iy - 1][ix] : me, gyp = y < ny - 1 ? v[iz][iy + 1][ix] : -me;
-    const float gzm = z > 0 ? v[iz - 1][iy][ix] : -me, gzp = z < nz - 1 ? v[iz + 1][iy][ix] : -me;
-    const float lap = (gxm + gxp + gym + gyp + gzm + gzp - 6.0f * me) * ih2;
-    acc += ld_rb(b, half, hx, ny, x, y, z) - lap;
-  }
-  const int t = cx + cnx * (cy + cny * cz);
-  Sto<TC>::st(bc + t, acc * 0.125f);
-  Sto<TC>::st(pc + t, 0.0f);
-}
-// k_pprolong from a plain coarse level into a red-black split fine level: child (2cx+dx, 2cy+dy, 2cz+dz)
-// is entry cx of colour half (dx + dy + dz) & 1 in its row.
-template <typename TF, typename TC>
-__global__ void __launch_bounds__(NT) k_pprolong_rb(TF* __restrict__ p, const TC* __restrict__ pc, int nx, int ny, int nz) {
-  pdl_wait();
-  pdl_trigger();
-  const int ncx = nx / 2, ncy = ny / 2, ncz = nz / 2;
-  const int cx = blockIdx.x * GX + threadIdx.x, cy = blockIdx.y * GY + threadIdx.y, cz = blockIdx.z * GZ + threadIdx.z;
-  if (cx >= ncx || cy >= ncy || cz >= ncz) return;
-  const int hx = nx >> 1, half = hx * ny * nz;
-  float v[3][3][3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int bb = 0; bb < 3; ++bb)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const int qx = cx + c - 1, qy = cy + bb - 1, qz = cz + a - 1;
-        float val = Sto<TC>::ld(pc + min(max(qx, 0), ncx - 1) + ncx * (min(max(qy, 0), ncy - 1) + ncy * min(max(qz, 0), ncz - 1)));
-        if (qx < 0 || qx >= ncx) val = -val;
-        if (qz < 0 || qz >= ncz) val = -val;
-        if (qy >= ncy) val = -val;
-        v[a][bb][c] = val;
-      }
-#pragma unroll
-  for (int dz = 0; dz < 2; ++dz)
-#pragma unroll
-    for (int dy = 0; dy < 2; ++dy)
-#pragma unroll
-      for (int dx = 0; dx < 2; ++dx) {
-        const float fx = dx ? 0.25f : 0.75f, fy = dy ? 0.25f : 0.75f, fz = dz ? 0.25f : 0.75f;
-        float acc = 0.0f;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int ox = q & 1, oy = (q >> 1) & 1, oz = (q >> 2) & 1;
-          const float wx = ox ? fx : 1.0f - fx, wy = oy ? fy : 1.0f - fy, wz = oz ? fz : 1.0f - fz;
-          acc += v[dz + oz][dy + oy][dx + ox] * wx * wy * wz;
-        }
-        TF* pf = p + (((dx + dy + dz) & 1) ? half : 0) + cx + hx * ((2 * cy + dy) + ny * (2 * cz + dz));
-        Sto<TF>::st(pf, Sto<TF>::ld(pf) + acc);
-      }
+template <int kDepth, typename TF, typename TC>
+__global__ void __launch_bounds__(NT) k_pprolong(TF* __restrict__ p, const TC* __restrict__ pc, int nx, int ny, int nz) {
+  prolong_march<kDepth, true, false>(p, pc, nx, ny, nz, blockIdx);
 }
 
 // Solver state on the device.
@@ -452,7 +151,7 @@ __device__ __forceinline__ float lap_diff(float me, float xm, float xp, float ym
 // into rT (if given).  Partials: (||r||^2, ||b||^2).
 template <typename TR>
 __global__ void __launch_bounds__(NT) k_pres(const float* __restrict__ xh, const float* __restrict__ xl, const float* __restrict__ b,
-                                             TR* __restrict__ rT, int rsplit, const PState* __restrict__ ps, int nx, int ny, int nz, float ih2,
+                                             TR* __restrict__ rT, const PState* __restrict__ ps, int nx, int ny, int nz, float ih2,
                                              float4* __restrict__ partials) {
   pdl_wait();
   pdl_trigger();
@@ -483,7 +182,7 @@ __global__ void __launch_bounds__(NT) k_pres(const float* __restrict__ xh, const
         }
         const float bv = __ldg(b + t);
         const float r = (bv - d * ih2) - dl * ih2;
-        if (rT) Sto<TR>::st(LV<TR>{rT, nx, ny, nz, rsplit}.at(x, y, z), r * s);
+        if (rT) st(rT + t, r * s);
         rr += r * r;
         bb += bv * bv;
         prev = cur; cur = next;
@@ -496,12 +195,11 @@ __global__ void __launch_bounds__(NT) k_pres(const float* __restrict__ xh, const
 }
 
 // k_pres for even nx with one thread per x pair (2 gx, 2 gx + 1) and RZ planes: every load of xh, xl and b
-// is a float2 (plus one scalar on each side for the x neighbours), and the two residuals land at entry gx
-// of the two colour halves when rT is red-black split.
+// is a float2 (plus one scalar on each side for the x neighbours), and the two residuals are stored as a pair.
 // kFull: nz is a multiple of the planes a CTA covers, so no plane test is needed inside the march.
 template <typename TR, bool kFull>
 __global__ void __launch_bounds__(NT) k_pres2(const float* __restrict__ xh, const float* __restrict__ xl, const float* __restrict__ b,
-                                              TR* __restrict__ rT, int rsplit, const PState* __restrict__ ps, int nx, int ny, int nz, float ih2,
+                                              TR* __restrict__ rT, const PState* __restrict__ ps, int nx, int ny, int nz, float ih2,
                                               float4* __restrict__ partials) {
   pdl_wait();
   pdl_trigger();
@@ -511,7 +209,7 @@ __global__ void __launch_bounds__(NT) k_pres2(const float* __restrict__ xh, cons
   float rr = 0.0f, bb = 0.0f;
   if (gx < hx && y < ny && z0 < nz) {
     const float s = rT ? ps->sc[1] : 1.0f;
-    const int sy = nx, sz = nx * ny, halfn = hx * ny * nz;
+    const int sy = nx, sz = nx * ny;
     const bool hxm = gx > 0, hxp = gx < hx - 1, hym = y > 0, hyp = y < ny - 1;
     const float2 zero2 = make_float2(0.0f, 0.0f);
     auto ld2 = [](const float* q) { return __ldg(reinterpret_cast<const float2*>(q)); };
@@ -540,16 +238,7 @@ __global__ void __launch_bounds__(NT) k_pres2(const float* __restrict__ xh, cons
         }
         const float2 bv = ld2(b + t);
         const float r0 = (bv.x - d0 * ih2) - dl0 * ih2, r1 = (bv.y - d1 * ih2) - dl1 * ih2;
-        if (rT) {
-          if (rsplit) {
-            const int c0 = (y + z) & 1, idx = gx + hx * (y + ny * z);
-            Sto<TR>::st(rT + c0 * halfn + idx, r0 * s);
-            Sto<TR>::st(rT + (1 - c0) * halfn + idx, r1 * s);
-          } else {
-            Sto<TR>::st(rT + t, r0 * s);
-            Sto<TR>::st(rT + t + 1, r1 * s);
-          }
-        }
+        if (rT) st2<true>(rT + t, make_float2(r0 * s, r1 * s));
         rr += r0 * r0;
         rr += r1 * r1;
         bb += bv.x * bv.x;
@@ -573,10 +262,9 @@ __device__ __forceinline__ void pair_add(float& hi, float& lo, float d) {
   hi = __fadd_rn(s, l2);
   lo = __fsub_rn(l2, __fsub_rn(hi, s));
 }
-// One thread per x pair (2 gx, 2 gx + 1) of a row: the pair is one float2 of xh and xl, and in the split
-// layout its two e values sit at the same half-index of the two colour halves.
+// One thread per x pair (2 gx, 2 gx + 1) of a row: the pair is one float2 of xh and xl and one pair of e.
 template <typename TE>
-__global__ void __launch_bounds__(NT) k_pupdate(float* __restrict__ xh, float* __restrict__ xl, const TE* __restrict__ e, int esplit,
+__global__ void __launch_bounds__(NT) k_pupdate(float* __restrict__ xh, float* __restrict__ xl, const TE* __restrict__ e,
                                                 const PState* __restrict__ ps, int nx, int ny, int nz) {
   pdl_wait();
   pdl_trigger();
@@ -584,18 +272,18 @@ __global__ void __launch_bounds__(NT) k_pupdate(float* __restrict__ xh, float* _
   const int x = 2 * gx;
   if (x >= nx || y >= ny || z >= nz) return;
   const float u = ps->sc[0];
-  const LV<TE> E{const_cast<TE*>(e), nx, ny, nz, esplit};
   const int t = x + nx * (y + ny * z);
-  if (x + 1 < nx && (nx & 1) == 0) {
+  if ((nx & 1) == 0) {
     float2 hv = *reinterpret_cast<const float2*>(xh + t);
     float2 lv = *reinterpret_cast<const float2*>(xl + t);
-    pair_add(hv.x, lv.x, __fmul_rn(Sto<TE>::ld(E.at(x, y, z)), u));
-    pair_add(hv.y, lv.y, __fmul_rn(Sto<TE>::ld(E.at(x + 1, y, z)), u));
+    const float2 ev = ld2<true>(e + t);
+    pair_add(hv.x, lv.x, __fmul_rn(ev.x, u));
+    pair_add(hv.y, lv.y, __fmul_rn(ev.y, u));
     *reinterpret_cast<float2*>(xh + t) = hv;
     *reinterpret_cast<float2*>(xl + t) = lv;
   } else {
-    pair_add(xh[t], xl[t], __fmul_rn(Sto<TE>::ld(E.at(x, y, z)), u));
-    if (x + 1 < nx) pair_add(xh[t + 1], xl[t + 1], __fmul_rn(Sto<TE>::ld(E.at(x + 1, y, z)), u));
+    pair_add(xh[t], xl[t], __fmul_rn(ld(e + t), u));
+    if (x + 1 < nx) pair_add(xh[t + 1], xl[t + 1], __fmul_rn(ld(e + t + 1), u));
   }
 }
 
@@ -670,14 +358,15 @@ using namespace fire;
 
 // Storage type of a level's arrays.
 enum { STO_F32 = 0, STO_F16 = 1, STO_BF16 = 2 };
-// One level of the solver: storage type, layout (red-black split or plain) and device arrays.
+// One level of the refinement: storage type and device arrays; p2 and sweep as in MGLevel.
 struct PLevel {
   int nx, ny, nz;
   float h;
   int sto;
-  int split;
   void* p;
   void* b;
+  void* p2;
+  SweepPlan sweep;
 };
 
 struct FirePoisson {
@@ -718,73 +407,59 @@ size_t align_up(size_t v) { return (v + 255) / 256 * 256; }
 size_t elem_bytes(int sto) { return sto == STO_F32 ? 4 : 2; }
 int storage_of(int prec) { return prec == FIRE_POISSON_FP16 ? STO_F16 : prec == FIRE_POISSON_BF16 ? STO_BF16 : STO_F32; }
 
-template <typename T>
-void psmooth_t(const PLevel& L, int color, int zero, cudaStream_t st) {
-  if (L.split && L.nx % 4 == 0) {
-    const dim3 g = grid3(L.nx >> 2, L.ny, (L.nz + SMZ - 1) / SMZ);
-    if (zero) launch_pdl(k_psmooth_rb2<T, true>, g, kBlock, 0, st, (T*)L.p, (const T*)L.b, L.nx, L.ny, L.nz, L.h, color);
-    else launch_pdl(k_psmooth_rb2<T, false>, g, kBlock, 0, st, (T*)L.p, (const T*)L.b, L.nx, L.ny, L.nz, L.h, color);
-  } else if (L.split) {
-    const dim3 g = grid3(L.nx >> 1, L.ny, (L.nz + SMZ - 1) / SMZ);
-    if (zero) launch_pdl(k_psmooth_rb<T, true>, g, kBlock, 0, st, (T*)L.p, (const T*)L.b, L.nx, L.ny, L.nz, L.h, color);
-    else launch_pdl(k_psmooth_rb<T, false>, g, kBlock, 0, st, (T*)L.p, (const T*)L.b, L.nx, L.ny, L.nz, L.h, color);
-  } else {
-    const dim3 g = grid3((L.nx + 1) >> 1, L.ny, (L.nz + SMZ - 1) / SMZ);
-    launch_pdl(k_psmooth<T>, g, kBlock, 0, st, (T*)L.p, (const T*)L.b, L.nx, L.ny, L.nz, L.h, color, zero);
-  }
+// f(T{}) with the level's storage type.
+template <typename F>
+void with_type(int sto, F&& f) {
+  if (sto == STO_F16) f(__half());
+  else if (sto == STO_BF16) f(__nv_bfloat16());
+  else f(float());
 }
 void psmooth(const PLevel& L, int color, int zero, cudaStream_t st) {
-  switch (L.sto) {
-    case STO_F16: psmooth_t<__half>(L, color, zero, st); break;
-    case STO_BF16: psmooth_t<__nv_bfloat16>(L, color, zero, st); break;
-    default: psmooth_t<float>(L, color, zero, st);
+  with_type(L.sto, [&](auto t) {
+    using T = decltype(t);
+    launch_pdl(k_psmooth<T>, grid3((L.nx + 1) >> 1, L.ny, (L.nz + SMZ - 1) / SMZ), kBlock, 0, st, (T*)L.p, (const T*)L.b, L.nx, L.ny, L.nz,
+               L.h, color, zero);
+  });
+}
+void psweep2(const PLevel& L, const void* p, void* out, bool zero, cudaStream_t st) {
+  with_type(L.sto, [&](auto t) {
+    using T = decltype(t);
+    launch_sweep2_t((const T*)p, (const T*)L.b, (T*)out, L.sweep, L.nx, L.ny, L.nz, L.h, 1.0f, zero, st);
+  });
+}
+// `iters` sweeps in place; pairs of two-sweep launches where the level has a plan (the second of a pair writes p again).
+void psweeps(const PLevel& L, int iters, bool zero, cudaStream_t st) {
+  int done = 0;
+  for (; L.sweep.px > 0 && done + 4 <= iters; done += 4) {
+    psweep2(L, L.p, L.p2, zero && done == 0, st);
+    psweep2(L, L.p2, L.p, false, st);
+  }
+  for (; done < iters; ++done) {
+    psmooth(L, 0, zero && done == 0, st);
+    psmooth(L, 1, 0, st);
   }
 }
-template <typename TF, typename TC>
-void prestrict_tt(const PLevel& F, const PLevel& C, cudaStream_t st) {
-  if (F.split && !C.split)
-    launch_pdl(k_prestrict_rb<TF, TC>, grid3(C.nx, C.ny, C.nz), kBlock, 0, st, (const TF*)F.p, (const TF*)F.b, F.nx, F.ny, F.nz, F.h,
-               (TC*)C.b, (TC*)C.p);
-  else
-    launch_pdl(k_prestrict<TF, TC>, grid3(C.nx, C.ny, C.nz), kBlock, 0, st, (const TF*)F.p, (const TF*)F.b, F.split, F.nx, F.ny, F.nz,
-               F.h, (TC*)C.b, (TC*)C.p, C.split);
+bool deep(const PLevel& C) { return (long)C.nx * C.ny * C.nz >= TRANSFER_DEEP_CELLS; }
+void prestrict(const PLevel& F, const void* p, const PLevel& C, bool clear, cudaStream_t st) {
+  with_type(F.sto, [&](auto f) {
+    with_type(C.sto, [&](auto c) {
+      using TF = decltype(f);
+      using TC = decltype(c);
+      launch_pdl(deep(C) ? k_prestrict<TRANSFER_DEPTH, TF, TC> : k_prestrict<1, TF, TC>,
+                 transfer_grid(C.nx, C.ny, C.nz, deep(C) ? TRANSFER_DEPTH : 1), kBlock, 0, st, (const TF*)p, (const TF*)F.b, F.nx, F.ny, F.nz,
+                 F.h, (TC*)C.b, clear ? (TC*)C.p : (TC*)nullptr);
+    });
+  });
 }
-template <typename TF>
-void prestrict_to(const PLevel& F, const PLevel& C, cudaStream_t st) {
-  switch (C.sto) {
-    case STO_F16: prestrict_tt<TF, __half>(F, C, st); break;
-    case STO_BF16: prestrict_tt<TF, __nv_bfloat16>(F, C, st); break;
-    default: prestrict_tt<TF, float>(F, C, st);
-  }
-}
-void prestrict(const PLevel& F, const PLevel& C, cudaStream_t st) {
-  switch (F.sto) {
-    case STO_F16: prestrict_to<__half>(F, C, st); break;
-    case STO_BF16: prestrict_to<__nv_bfloat16>(F, C, st); break;
-    default: prestrict_to<float>(F, C, st);
-  }
-}
-template <typename TF, typename TC>
-void pprolong_tt(const PLevel& F, const PLevel& C, cudaStream_t st) {
-  if (F.split && !C.split)
-    launch_pdl(k_pprolong_rb<TF, TC>, grid3(C.nx, C.ny, C.nz), kBlock, 0, st, (TF*)F.p, (const TC*)C.p, F.nx, F.ny, F.nz);
-  else
-    launch_pdl(k_pprolong<TF, TC>, grid3(C.nx, C.ny, C.nz), kBlock, 0, st, (TF*)F.p, F.split, (const TC*)C.p, C.split, F.nx, F.ny, F.nz);
-}
-template <typename TF>
-void pprolong_from(const PLevel& F, const PLevel& C, cudaStream_t st) {
-  switch (C.sto) {
-    case STO_F16: pprolong_tt<TF, __half>(F, C, st); break;
-    case STO_BF16: pprolong_tt<TF, __nv_bfloat16>(F, C, st); break;
-    default: pprolong_tt<TF, float>(F, C, st);
-  }
-}
-void pprolong(const PLevel& F, const PLevel& C, cudaStream_t st) {
-  switch (F.sto) {
-    case STO_F16: pprolong_from<__half>(F, C, st); break;
-    case STO_BF16: pprolong_from<__nv_bfloat16>(F, C, st); break;
-    default: pprolong_from<float>(F, C, st);
-  }
+void pprolong(const PLevel& F, void* p, const PLevel& C, cudaStream_t st) {
+  with_type(F.sto, [&](auto f) {
+    with_type(C.sto, [&](auto c) {
+      using TF = decltype(f);
+      using TC = decltype(c);
+      launch_pdl(deep(C) ? k_pprolong<TRANSFER_DEPTH, TF, TC> : k_pprolong<1, TF, TC>,
+                 transfer_grid(C.nx, C.ny, C.nz, deep(C) ? TRANSFER_DEPTH : 1), kBlock, 0, st, (TF*)p, (const TC*)C.p, F.nx, F.ny, F.nz);
+    });
+  });
 }
 
 // The residual kernel's grid: x pairs for even nx (k_pres2), single cells otherwise (k_pres).
@@ -794,39 +469,22 @@ dim3 pres_grid(const PLevel& L) {
 }
 
 // r = b - A (xh + xl); written scaled into level 0's RHS when `write` (refinement forms); partials for the test.
-template <typename TR>
-void pres_t(FirePoisson* ps, const PState* state, const float* b, const float* xh, const float* xl, TR* rT, int rsplit, cudaStream_t st) {
-  const PLevel& L = ps->levels[0];
-  if (L.nx % 2 == 0 && L.nz % (GZ * RZ) == 0)
-    launch_pdl(k_pres2<TR, true>, pres_grid(L), kBlock, 0, st, xh, xl, b, rT, rsplit, state, L.nx, L.ny, L.nz, 1.0f / (L.h * L.h),
-               ps->partials);
-  else if (L.nx % 2 == 0)
-    launch_pdl(k_pres2<TR, false>, pres_grid(L), kBlock, 0, st, xh, xl, b, rT, rsplit, state, L.nx, L.ny, L.nz, 1.0f / (L.h * L.h),
-               ps->partials);
-  else
-    launch_pdl(k_pres<TR>, pres_grid(L), kBlock, 0, st, xh, xl, b, rT, rsplit, state, L.nx, L.ny, L.nz, 1.0f / (L.h * L.h), ps->partials);
-}
 void pres(FirePoisson* ps, const PState* state, const float* b, const float* xh, const float* xl, bool write, cudaStream_t st) {
   const PLevel& L = ps->levels[0];
-  if (!write) { pres_t<float>(ps, state, b, xh, xl, nullptr, 0, st); return; }
-  switch (L.sto) {
-    case STO_F16: pres_t<__half>(ps, state, b, xh, xl, (__half*)L.b, L.split, st); break;
-    case STO_BF16: pres_t<__nv_bfloat16>(ps, state, b, xh, xl, (__nv_bfloat16*)L.b, L.split, st); break;
-    default: pres_t<float>(ps, state, b, xh, xl, (float*)L.b, L.split, st);
-  }
-}
-template <typename TE>
-void pupdate_t(FirePoisson* ps, float* xh, float* xl, cudaStream_t st) {
-  const PLevel& L = ps->levels[0];
-  launch_pdl(k_pupdate<TE>, grid3((L.nx + 1) >> 1, L.ny, L.nz), kBlock, 0, st, xh, xl, (const TE*)L.p, L.split, (const PState*)ps->state,
-             L.nx, L.ny, L.nz);
+  with_type(write ? L.sto : STO_F32, [&](auto t) {
+    using TR = decltype(t);
+    auto kernel = L.nx % 2 ? k_pres<TR> : L.nz % (GZ * RZ) ? k_pres2<TR, false> : k_pres2<TR, true>;
+    launch_pdl(kernel, pres_grid(L), kBlock, 0, st, xh, xl, b, write ? (TR*)L.b : (TR*)nullptr, state, L.nx, L.ny, L.nz, 1.0f / (L.h * L.h),
+               ps->partials);
+  });
 }
 void pupdate(FirePoisson* ps, float* xh, float* xl, cudaStream_t st) {
-  switch (ps->levels[0].sto) {
-    case STO_F16: pupdate_t<__half>(ps, xh, xl, st); break;
-    case STO_BF16: pupdate_t<__nv_bfloat16>(ps, xh, xl, st); break;
-    default: pupdate_t<float>(ps, xh, xl, st);
-  }
+  const PLevel& L = ps->levels[0];
+  with_type(L.sto, [&](auto t) {
+    using TE = decltype(t);
+    launch_pdl(k_pupdate<TE>, grid3((L.nx + 1) >> 1, L.ny, L.nz), kBlock, 0, st, xh, xl, (const TE*)L.p, (const PState*)ps->state, L.nx, L.ny,
+               L.nz);
+  });
 }
 void ptest(FirePoisson* ps, PState* state, int mode, int first, int count, double tol, int max_iters, cudaGraphConditionalHandle h,
            int set_cond, cudaStream_t st) {
@@ -844,41 +502,34 @@ void ir_vcycle(FirePoisson* ps, bool zero_first, cudaStream_t st) {
   const int n = (int)ps->levels.size(), T = ps->tailFirst, top = std::min(T, n - 1);
   std::vector<PLevel>& L = ps->levels;
   for (int i = 0; i < top; ++i) {
-    for (int k = 0; k < 2; ++k) {
-      psmooth(L[i], 0, (i == 0 && zero_first && k == 0) ? 1 : 0, st);
-      psmooth(L[i], 1, 0, st);
-    }
-    prestrict(L[i], L[i + 1], st);
+    const bool two = L[i].sweep.px > 0;
+    if (two) psweep2(L[i], L[i].p, L[i].p2, i > 0 || zero_first, st);
+    else psweeps(L[i], 2, i > 0 || zero_first, st);
+    // a level that is smoothed here next starts from zero without reading its pressure
+    prestrict(L[i], two ? L[i].p2 : L[i].p, L[i + 1], i + 1 == top, st);
   }
   if (ps->coarse) {
     launch_coarse(ps->mg.data(), T, n, 2, 2, 0, ps->cinv, 1, ps->err, st);
   } else if (T < n) {
     launch_tail(ps->mg.data(), T, n, 2, 2, COARSE64_SWEEPS, ps->err, st, true, ps->cinv);
   } else {
-    for (int k = 0; k < ps->coarseIters; ++k) {
-      psmooth(L[n - 1], 0, (n == 1 && zero_first && k == 0) ? 1 : 0, st);
-      psmooth(L[n - 1], 1, 0, st);
-    }
+    psweeps(L[n - 1], ps->coarseIters, n == 1 && zero_first, st);
   }
   for (int i = top - 1; i >= 0; --i) {
-    pprolong(L[i], L[i + 1], st);
-    for (int k = 0; k < 2; ++k) { psmooth(L[i], 0, 0, st); psmooth(L[i], 1, 0, st); }
+    const bool two = L[i].sweep.px > 0;
+    pprolong(L[i], two ? L[i].p2 : L[i].p, L[i + 1], st);
+    if (two) psweep2(L[i], L[i].p2, L[i].p, false, st);
+    else psweeps(L[i], 2, false, st);
   }
 }
 // The step's V(2,2) cycle (src/sim.js:588-599) on (x, b).
 void fp32_vcycle(FirePoisson* ps, cudaStream_t st) {
   const int n = (int)ps->mg.size(), T = ps->tailFirst, top = std::min(T, n - 1);
-  for (int i = 0; i < top; ++i) {
-    for (int k = 0; k < 2; ++k) { launch_smooth(ps->mg[i], 0, st); launch_smooth(ps->mg[i], 1, st); }
-    launch_restrict(ps->mg[i], ps->mg[i + 1], st);
-  }
+  launch_down(ps->mg.data(), top, st);
   if (ps->coarse) launch_coarse(ps->mg.data(), T, n, 2, 2, ps->coarseIters, nullptr, 1, ps->err, st);
   else if (T < n) launch_tail(ps->mg.data(), T, n, 2, 2, ps->coarseIters, ps->err, st);
-  else for (int k = 0; k < ps->coarseIters; ++k) { launch_smooth(ps->mg[n - 1], 0, st); launch_smooth(ps->mg[n - 1], 1, st); }
-  for (int i = top - 1; i >= 0; --i) {
-    launch_prolong(ps->mg[i], ps->mg[i + 1], st);
-    for (int k = 0; k < 2; ++k) { launch_smooth(ps->mg[i], 0, st); launch_smooth(ps->mg[i], 1, st); }
-  }
+  else launch_sweeps(ps->mg[n - 1], ps->coarseIters, st);
+  launch_up(ps->mg.data(), top, st);
 }
 
 // Dense inverse of the coarsest operator A (A p = (sum of ghost-ruled neighbours - diag p) / h^2, as the
@@ -1073,7 +724,7 @@ int fire_poisson_create(const int res[3], float h, int precision, int device, Fi
   if (ps->coarse) ps->tailFirst = cf;
   // arena: level arrays (level 0 of the FP32 form is the caller's x and b), partials, state
   size_t off = 0;
-  std::vector<size_t> pOff(n), bOff(n);
+  std::vector<size_t> pOff(n), bOff(n), p2Off(n);
   ps->levels.resize(n);
   const int sto = storage_of(precision);
   for (int l = 0; l < n; ++l) {
@@ -1081,9 +732,10 @@ int fire_poisson_create(const int res[3], float h, int precision, int device, Fi
     PLevel& L = ps->levels[l];
     L.nx = M.nx; L.ny = M.ny; L.nz = M.nz; L.h = M.h;
     L.sto = (ps->ir && l < ps->tailFirst) ? sto : STO_F32;
-    // level 0 (the only level whose arrays outgrow L2) in the red-black split layout; the rest plain
-    L.split = (ps->ir && l == 0 && l < ps->tailFirst && M.nx % 2 == 0) ? 1 : 0;
+    // every level that launches smooth: all above the coarse end, and the coarsest itself where none takes it
+    if (l < ps->tailFirst) L.sweep = ps->mg[l].sweep = plan_sweep(ps->mg[l]);
     const size_t bytes = align_up((size_t)M.nx * M.ny * M.nz * elem_bytes(L.sto));
+    if (L.sweep.px > 0) { p2Off[l] = off; off += bytes; }
     if (l == 0 && !ps->ir) { pOff[l] = bOff[l] = (size_t)-1; continue; }
     pOff[l] = off; off += bytes;
     bOff[l] = off; off += bytes;
@@ -1103,6 +755,10 @@ int fire_poisson_create(const int res[3], float h, int precision, int device, Fi
   if (cudaMalloc(&ps->arena, off) != cudaSuccess) { delete ps; return FIRE_ERR_OOM; }
   char* A = (char*)ps->arena;
   for (int l = 0; l < n; ++l) {
+    if (ps->levels[l].sweep.px > 0) {
+      ps->levels[l].p2 = A + p2Off[l];
+      ps->mg[l].p2 = (float*)(A + p2Off[l]);   // used by the FP32 form
+    }
     if (pOff[l] == (size_t)-1) continue;
     ps->levels[l].p = A + pOff[l];
     ps->levels[l].b = A + bOff[l];
@@ -1117,6 +773,7 @@ int fire_poisson_create(const int res[3], float h, int precision, int device, Fi
   if (ps->ir) ps->xlo = (float*)(A + loOff);
   if (direct) ps->cinv = (double*)(A + cinvOff);
   if (cudaMemset(ps->arena, 0, off) != cudaSuccess || mg_configure(TAIL_SMEM_BUDGET) != cudaSuccess || coarse_configure() != cudaSuccess ||
+      sweep_configure() != cudaSuccess ||
       cudaStreamCreateWithFlags(&ps->capStream, cudaStreamNonBlocking) != cudaSuccess ||
       (direct && cudaMemcpy(ps->cinv, cinv.data(), sizeof(double) * cinv.size(), cudaMemcpyHostToDevice) != cudaSuccess)) {
     fire_poisson_destroy(ps);
@@ -1192,7 +849,7 @@ int fire_poisson_set_study(FirePoisson* ps, int coarse_sweeps) {
   if (!ps || ps->ir || coarse_sweeps < 1 || coarse_sweeps > 4096) return FIRE_ERR_BAD_ARG;
   DeviceGuard dg(ps->device);
   if (cudaDeviceSynchronize() != cudaSuccess) return FIRE_ERR_CUDA;
-  for (MGLevel& L : ps->mg) L.study = 1;
+  for (MGLevel& L : ps->mg) { L.study = 1; L.sweep = SweepPlan{}; }   // the study's sweeps are colour launches
   ps->coarseIters = coarse_sweeps;
   ps->tailFirst = tail_first(ps->mg.data(), (int)ps->mg.size(), false);   // single-CTA tails in this variant
   ps->coarse = false;

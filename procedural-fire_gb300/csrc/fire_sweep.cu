@@ -63,7 +63,7 @@ __device__ __forceinline__ float update(const Sweeper& w, float old, float own, 
   return kRelax ? __fmaf_rn(w.omega, __fmaf_rn(t, rd, -old), old) : __fmul_rn(t, rd);
 }
 // Step k = I (mod 6) of the march.  kEdge: some of the planes k-4 .. k-1 lie outside the domain or touch its bottom or top.
-template <bool kRelax, int I, bool kEdge>
+template <typename T, bool kRelax, int I, bool kEdge>
 __device__ __forceinline__ void step(const Sweeper& w, Col (&c)[SW_ROWS][2], int k) {
   constexpr int a0 = (I & 1) ? 0 : 1;   // working column of row 0: (x + y + k - 1) even, y even; row 1's is the other
   float4 far[SW_ROWS];
@@ -87,8 +87,9 @@ __device__ __forceinline__ void step(const Sweeper& w, Col (&c)[SW_ROWS][2], int
       const float yp = r + 1 < SW_ROWS ? c[r + 1 < SW_ROWS ? r + 1 : r][a].v[slot(I, j)] : hi[j - 1];
       float rd = w.rd[r][a];
       if (kEdge && (z == 0 || z == w.nz - 1)) rd = w.rdz[r][a];
-      const float v = update<kRelax>(w, m.v[slot(I, j)], c[r][1 - a].v[slot(I, j)], f[j - 1], m.v[slot(I, j + 1)], m.v[slot(I, j - 1)], ym, yp,
+      float v = update<kRelax>(w, m.v[slot(I, j)], c[r][1 - a].v[slot(I, j)], f[j - 1], m.v[slot(I, j + 1)], m.v[slot(I, j - 1)], ym, yp,
                                      m.b[slot(I, j)], rd);
+      v = Cells2<T>::one(Cells2<T>::back(v));   // what a colour launch would have stored
       if (!kEdge || (unsigned)z < (unsigned)w.nz) m.v[slot(I, j)] = v;
     }
   }
@@ -119,7 +120,8 @@ __device__ __forceinline__ void sweep2_body(const T* __restrict__ p, const T* __
   w.S = sw_smem + w.pitch * (SW_ROWS * ty + 1) + px + 1;
   for (int i = tid; i < 2 * w.par; i += blockDim.x) sw_smem[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   const int x = t.lx + 2 * px, y = t.ly + SW_ROWS * ty;
-  w.live = work && x < nx && y < ny;   // nx and ny are even: pairs and both rows
+  w.live = work && x < nx && y < ny;   // nx is even; of an odd ny the last thread row has one row in the domain
+  const bool both = y + 1 < ny;
   const bool core = w.live && x >= t.x0 && x < t.x1 && y >= t.y0 && y < t.y1;
   Col c[SW_ROWS][2];
 #pragma unroll
@@ -129,6 +131,7 @@ __device__ __forceinline__ void sweep2_body(const T* __restrict__ p, const T* __
       const float d = 6.0f + (x + q == 0 ? 1.0f : 0.0f) + (x + q == nx - 1 ? 1.0f : 0.0f) + (y + r == ny - 1 ? 1.0f : 0.0f) - (y + r == 0 ? 1.0f : 0.0f);
       asm("rcp.approx.f32 %0, %1;" : "=f"(w.rd[r][q]) : "f"(d));
       asm("rcp.approx.f32 %0, %1;" : "=f"(w.rdz[r][q]) : "f"(d + 1.0f));
+      if (r == 1 && !both) w.rd[r][q] = w.rdz[r][q] = 0.0f;   // a row outside stays zero
 #pragma unroll
       for (int j = 0; j < 6; ++j) c[r][q].v[j] = c[r][q].b[j] = 0.0f;
     }
@@ -140,7 +143,7 @@ __device__ __forceinline__ void sweep2_body(const T* __restrict__ p, const T* __
   V* ring[2 * SW_ROWS];
 #pragma unroll
   for (int q = 0; q < 2 * SW_ROWS; ++q) ring[q] = reinterpret_cast<V*>(sw_smem + 2 * w.par) + (q * blockDim.x + tid) * SW_RING;
-  const int first = w.live ? x + nx * (y + ny * k) : 0, row = w.live ? nx : 0;
+  const int first = w.live ? x + nx * (y + ny * k) : 0, row = w.live && both ? nx : 0;
   const T *pq = p + first, *bq = b + first;   // the plane to ask for next
   T* oq = out + first;                        // plane k - 4, once it is inside the chunk
   const int ahead = w.live ? plane : 0;
@@ -150,8 +153,9 @@ __device__ __forceinline__ void sweep2_body(const T* __restrict__ p, const T* __
     const bool in = w.live && q < nz && q <= kend;
 #pragma unroll
     for (int r = 0; r < SW_ROWS; ++r) {
-      if (!kZero) copy_pair(ring[r] + entry, pq + r * row, in);
-      copy_pair(ring[SW_ROWS + r] + entry, bq + r * row, in);
+      const bool here = in && (r == 0 || both);
+      if (!kZero) copy_pair(ring[r] + entry, pq + r * row, here);
+      copy_pair(ring[SW_ROWS + r] + entry, bq + r * row, here);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
     if (q + 1 < nz) { pq += ahead; bq += ahead; }
@@ -174,7 +178,7 @@ __device__ __forceinline__ void sweep2_body(const T* __restrict__ p, const T* __
         c[r][0].v[slot(I, 0)] = c[r][1].v[slot(I, 0)] = 0.0f;
       }
     }
-    step<kRelax, I, kEdge>(w, c, k);
+    step<T, kRelax, I, kEdge>(w, c, k);
 #pragma unroll
     for (int r = 0; r < SW_ROWS; ++r) {   // b of plane k: used from the next step on; its slot held plane k - 6's
       const float2 v = Cells2<T>::get(ring[SW_ROWS + r][I]);
@@ -186,7 +190,7 @@ __device__ __forceinline__ void sweep2_body(const T* __restrict__ p, const T* __
       if (core && k - SW_HALO >= t.z0)
 #pragma unroll
         for (int r = 0; r < SW_ROWS; ++r)
-          *reinterpret_cast<V*>(oq + r * nx) = Cells2<T>::put(make_float2(c[r][0].v[slot(I, 4)], c[r][1].v[slot(I, 4)]));
+          if (r == 0 || both) *reinterpret_cast<V*>(oq + r * nx) = Cells2<T>::put(make_float2(c[r][0].v[slot(I, 4)], c[r][1].v[slot(I, 4)]));
       oq += plane;
     }
     ++k;
@@ -245,7 +249,7 @@ constexpr double SW_STEP = 300.0, SW_WARP = 30.0, SW_START = 1500.0;
 SweepPlan plan_sweep(const MGLevel& L, int sms) {
   const int nx = L.nx, ny = L.ny, nz = L.nz;
   SweepPlan best{};
-  if (L.study || nx % 2 || ny % 2 || nx < 8 || ny < 4 || nz < 4) return best;   // odd rows: the coarsest level's colour launches
+  if (L.study || nx % 2 || nx < 8 || ny < 4 || nz < 4) return best;   // odd rows have no aligned pairs: colour launches
   double cost = 1e30;
   auto even = [](int v) { return (v + 1) & ~1; };
   for (int ntx = 1; ntx <= 16; ++ntx) {
@@ -286,15 +290,30 @@ cudaError_t launch_sweep2_t(const T* p, const T* b, T* out, const SweepPlan& P, 
   const size_t smem = sweep_smem(P);
   auto go = [&](auto kernel) { return launch_pdl(kernel, grid, block, smem, st, p, b, out, nx, ny, nz, h, omega, P); };
   if (omega == 1.0f) return zero ? go(k_sweep2<T, true, false>) : go(k_sweep2<T, false, false>);
-  return zero ? go(k_sweep2<T, true, true>) : go(k_sweep2<T, false, true>);
+  if constexpr (sizeof(T) != sizeof(float)) return cudaErrorInvalidValue;   // the refinement's sweeps are Gauss-Seidel
+  else return zero ? go(k_sweep2<T, true, true>) : go(k_sweep2<T, false, true>);
 }
 cudaError_t launch_sweep2(const MGLevel& L, const float* p, float* out, bool zero, cudaStream_t st) {
   return launch_sweep2_t<float>(p, L.b, out, L.sweep, L.nx, L.ny, L.nz, L.h, L.omega, zero, st);
 }
 
-static cudaError_t sweeps_by_launches(const MGLevel& L, cudaStream_t st) {
+template cudaError_t launch_sweep2_t<float>(const float*, const float*, float*, const SweepPlan&, int, int, int, float, float, bool, cudaStream_t);
+template cudaError_t launch_sweep2_t<__half>(const __half*, const __half*, __half*, const SweepPlan&, int, int, int, float, float, bool,
+                                             cudaStream_t);
+template cudaError_t launch_sweep2_t<__nv_bfloat16>(const __nv_bfloat16*, const __nv_bfloat16*, __nv_bfloat16*, const SweepPlan&, int, int, int,
+                                                    float, float, bool, cudaStream_t);
+
+cudaError_t launch_sweeps(const MGLevel& L, int iters, cudaStream_t st) {
   cudaError_t e = cudaSuccess;
-  for (int k = 0; k < 4 && e == cudaSuccess; ++k) e = launch_smooth(L, k & 1, st);
+  int done = 0;
+  for (; L.sweep.px > 0 && done + 4 <= iters && e == cudaSuccess; done += 4) {   // p -> p2 -> p
+    e = launch_sweep2(L, L.p, L.p2, false, st);
+    if (e == cudaSuccess) e = launch_sweep2(L, L.p2, L.p, false, st);
+  }
+  for (; done < iters && e == cudaSuccess; ++done) {
+    e = launch_smooth(L, 0, st);
+    if (e == cudaSuccess) e = launch_smooth(L, 1, st);
+  }
   return e;
 }
 static MGLevel on_p2(MGLevel L) {
@@ -306,7 +325,7 @@ cudaError_t launch_down(const MGLevel* levels, int top, cudaStream_t st) {
   for (int i = 0; i < top && e == cudaSuccess; ++i) {
     const MGLevel& L = levels[i];
     const bool two = L.sweep.px > 0;
-    e = two ? launch_sweep2(L, L.p, L.p2, i > 0, st) : sweeps_by_launches(L, st);
+    e = two ? launch_sweep2(L, L.p, L.p2, i > 0, st) : launch_sweeps(L, 2, st);
     // a level that starts with the two-sweep kernel does not read its pressure
     if (e == cudaSuccess) e = launch_restrict(two ? on_p2(L) : L, levels[i + 1], st, i + 1 == top || levels[i + 1].sweep.px == 0);
   }
@@ -318,7 +337,7 @@ cudaError_t launch_up(const MGLevel* levels, int top, cudaStream_t st) {
     const MGLevel& L = levels[i];
     const bool two = L.sweep.px > 0;
     e = launch_prolong(two ? on_p2(L) : L, levels[i + 1], st);
-    if (e == cudaSuccess) e = two ? launch_sweep2(L, L.p2, L.p, false, st) : sweeps_by_launches(L, st);
+    if (e == cudaSuccess) e = two ? launch_sweep2(L, L.p2, L.p, false, st) : launch_sweeps(L, 2, st);
   }
   return e;
 }
@@ -331,6 +350,10 @@ cudaError_t sweep_configure() {
   opt_in(k_sweep2<float, true, false>);
   opt_in(k_sweep2<float, false, true>);
   opt_in(k_sweep2<float, true, true>);
+  opt_in(k_sweep2<__half, false, false>);
+  opt_in(k_sweep2<__half, true, false>);
+  opt_in(k_sweep2<__nv_bfloat16, false, false>);
+  opt_in(k_sweep2<__nv_bfloat16, true, false>);
   return e;
 }
 

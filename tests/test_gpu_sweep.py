@@ -34,3 +34,37 @@ def test_cycle_matches_colour_launches(res, omega):
         assert FC.rel_l2(pa, pb) <= 1e-5
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("res", [(120, 101, 90), (150, 100, 77)])
+def test_single_large_level_matches_colour_launches(res):
+    """A grid without coarser levels and too large for the on-chip kernel: all its sweeps are two-sweep launches, in place by
+    pairs, with the odd remainder by colour; an odd row count leaves a thread row with one row in the domain."""
+    a, b = C._sim(res, 1.0), C._sim(res, 1.0)
+    a.run_stage("vcycle", 0.01)
+    b.run_mg("sweeps", 0, a.info().coarse_iters)
+    a.sync()
+    np.testing.assert_array_equal(a.level(0, "p"), b.level(0, "p"))
+    a.close()
+    b.close()
+
+
+@pytest.mark.parametrize("precision", ["fp16", "bf16", "ir32"])
+@pytest.mark.parametrize("res", [(46, 92, 44), (50, 98, 50), (96, 110, 70), (120, 101, 90)])
+def test_refinement_forms_reach_the_tolerance(precision, res):
+    """The same kernel on levels in half, bfloat16 and float: the residual that the solver reports and the one computed afresh
+    from the returned pair agree (both are sums of squares in double-float of FP32 residuals of the same pair: 1e-5), and
+    lie at the tolerance asked for on a hierarchy, below the start on a single level (whose sweeps only smooth)."""
+    torch = pytest.importorskip("torch")
+    import fire_sim as F
+    ps = F.Poisson(res, 0.01, precision)
+    n = (res[2], res[1], res[0])
+    b, x, lo = (torch.zeros(n, device="cuda") for _ in range(3))
+    ps.make_rhs(b, seed=5)
+    single = bool(res[1] % 2)
+    ps.solve(b, x, x_lo=lo, tol=1e-6, max_iters=4 if single else 40)
+    out = ps.result()
+    rel = ps.residual(b, x, x_lo=lo)
+    assert abs(rel - out["rel_residual"]) <= 1e-5 * out["rel_residual"] + 1e-12
+    assert out["rel_residual"] <= (0.9 * out["rel_residual_initial"] if single else 1e-6)
+    ps.close()
