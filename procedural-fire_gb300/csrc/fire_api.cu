@@ -1102,8 +1102,8 @@ int fire_sim_set_step_stats(FireSim* sim, int enable) {
 // ==================================================================================================
 // Ensemble: many independent simulations of uneven sizes advanced together.  Every stage of a step is
 // one launch over all members (a BatchMap concatenates their block grids), the multigrid levels outside
-// each member's shared-memory tail are batched level by level, and the tails of all members run in one
-// launch per tail form; the whole step is one CUDA graph.  Members are ordinary FireSim handles (created
+// each member's on-chip coarse end are batched level by level, and the coarse ends of all members run in one
+// launch per form; the whole step is one CUDA graph.  Members are ordinary FireSim handles (created
 // and owned by the ensemble) so their parameters, spots, events, fields and diagnostics use the FireSim
 // API; their parameter blocks are staged into one contiguous device array and copied with one copy.
 constexpr int ENS_STAGES = 5;   // adv1, adv2, forces, div, project
@@ -1169,7 +1169,7 @@ struct EnsCtx {
   StepBatch SB;
   BatchMap cell[CELL_TILES], forces[FORCES_TILES];
   int depth = 0;
-  std::vector<BatchMap> smoothMap, coarseMap;
+  std::vector<BatchMap> sweepMap, smoothMap, coarseMap;   // two-sweep tiles; colour launches (levels without a plan); transfers
   std::vector<LevelBatch> LB;
 };
 void ens_context(FireEnsemble* e, EnsCtx& c) {
@@ -1178,14 +1178,17 @@ void ens_context(FireEnsemble* e, EnsCtx& c) {
   for (auto& m : c.cell) m = map_empty();
   for (auto& m : c.forces) m = map_empty();
   c.depth = 0;
+  double cells = 0.0;
   for (int i = 0; i < n; ++i) {
     FireSim* s = e->sims[i];
     c.SB.s[i] = StepInst{e->dBlocks + (size_t)i * BLOCK_FLOATS, s->f, s->d, s->levels[0].b, s->levels[0].p};
     for (int v = 0; v < CELL_TILES; ++v) map_add(c.cell[v], i, step_grid(s->d, v));
     for (int v = 0; v < FORCES_TILES; ++v) map_add(c.forces[v], i, forces_grid(s->d, v));
     c.depth = std::max(c.depth, ens_top(s));
+    cells += (double)s->d.nx * s->d.ny * s->d.nz;
   }
   // per level: the members that have it outside their tail, and every member's level l and l + 1
+  c.sweepMap.assign(c.depth, map_empty());
   c.smoothMap.assign(c.depth, map_empty());
   c.coarseMap.assign(c.depth, map_empty());
   c.LB.assign(c.depth + 1, LevelBatch{});
@@ -1193,9 +1196,18 @@ void ens_context(FireEnsemble* e, EnsCtx& c) {
   for (int i = 0; i < n; ++i) {
     FireSim* s = e->sims[i];
     const int top = ens_top(s);
-    for (int l = 0; l <= c.depth && l < (int)s->levels.size(); ++l) c.LB[l].l[i] = s->levels[l];
+    for (int l = 0; l <= c.depth && l < (int)s->levels.size(); ++l) {
+      MGLevel& L = c.LB[l].l[i] = s->levels[l];
+      L.sweep = SweepPlan{};
+      if (l < top && L.p2) {   // cut for the member's share of the SMs, as all members' tiles run at once
+        const double share = (double)s->d.nx * s->d.ny * s->d.nz / cells;
+        L.sweep = plan_sweep(L, std::max(1, (int)(152 * share)), SW_BATCH_THREADS);
+      }
+    }
     for (int l = 0; l < top; ++l) {
-      map_add(c.smoothMap[l], i, smooth_grid(s->levels[l]));
+      const SweepPlan& P = c.LB[l].l[i].sweep;
+      if (P.px) map_add(c.sweepMap[l], i, dim3(P.ntx * P.nty * P.ntz));
+      else map_add(c.smoothMap[l], i, smooth_grid(s->levels[l]));
       map_add(c.coarseMap[l], i, coarse_grid(s->levels[l + 1]));
     }
   }
@@ -1209,11 +1221,16 @@ void ens_stage(FireEnsemble* e, const EnsCtx& c, int stage, int tile, cudaStream
     default: launch_project_batch(c.cell[tile], c.SB, tile, st); break;
   }
 }
+// Two sweeps of level l of every member that smooths it by launches.
+void ens_sweeps(const EnsCtx& c, int l, bool down, cudaStream_t st) {
+  if (c.sweepMap[l].n) launch_sweep2_batch(c.sweepMap[l], c.LB[l], down, down && l > 0, st);
+  for (int k = 0; k < 4 && c.smoothMap[l].n; ++k) launch_smooth_batch(c.smoothMap[l], c.LB[l], k & 1, st);
+}
 void ens_mg(FireEnsemble* e, const EnsCtx& c, cudaStream_t st) {
   const int V = e->sims[0]->vcycles;
   for (int cy = 0; cy < V; ++cy) {
     for (int l = 0; l < c.depth; ++l) {
-      for (int k = 0; k < 2; ++k) { launch_smooth_batch(c.smoothMap[l], c.LB[l], 0, st); launch_smooth_batch(c.smoothMap[l], c.LB[l], 1, st); }
+      ens_sweeps(c, l, true, st);
       launch_restrict_batch(c.coarseMap[l], c.LB[l], c.LB[l + 1], st);
     }
     for (int kind = 0; kind < COARSE_KINDS; ++kind)
@@ -1222,7 +1239,7 @@ void ens_mg(FireEnsemble* e, const EnsCtx& c, cudaStream_t st) {
       launch_tail_batch(kind, e->dTail[kind], e->tailCount[kind], e->tailSmem[kind], 2, 2, e->dErr, st);
     for (int l = c.depth - 1; l >= 0; --l) {
       launch_prolong_batch(c.coarseMap[l], c.LB[l], c.LB[l + 1], st);
-      for (int k = 0; k < 2; ++k) { launch_smooth_batch(c.smoothMap[l], c.LB[l], 0, st); launch_smooth_batch(c.smoothMap[l], c.LB[l], 1, st); }
+      ens_sweeps(c, l, false, st);
     }
   }
 }

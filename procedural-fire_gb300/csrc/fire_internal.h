@@ -149,7 +149,8 @@ void launch_project_batch(const BatchMap& m, const StepBatch& I, int tile, cudaS
 
 // ---- kernel launchers (fire_sweep.cu) ----
 // Two red-black sweeps from p (zero: from zero) into out; bit-identical to the four colour launches.
-SweepPlan plan_sweep(const MGLevel& L, int sms = 152);
+// sms: the SMs the level may count on; block: threads of a CTA (0: as many as the tile has).
+SweepPlan plan_sweep(const MGLevel& L, int sms = 152, int block = 0);
 cudaError_t launch_sweep2(const MGLevel& L, const float* p, float* out, bool zero, cudaStream_t st);
 // The same on a level's arrays in storage T (float, __half, __nv_bfloat16; omega 1 for the last two).
 template <typename T>
@@ -157,6 +158,10 @@ cudaError_t launch_sweep2_t(const T* p, const T* b, T* out, const SweepPlan& P, 
                             cudaStream_t st);
 // `iters` sweeps in place, two-sweep launches as far as the level has a plan.
 cudaError_t launch_sweeps(const MGLevel& L, int iters, cudaStream_t st);
+// The same level of each simulation of a batch (plans for SW_BATCH_THREADS, one block per tile): p (zero: from zero) -> p2 down
+// the cycle, p2 -> p up.
+constexpr int SW_BATCH_THREADS = 512;
+cudaError_t launch_sweep2_batch(const BatchMap& m, const LevelBatch& L, bool down, bool zero, cudaStream_t st);
 cudaError_t sweep_configure();
 
 // ---- kernel launchers (fire_mg.cu) ----
@@ -207,6 +212,7 @@ cudaError_t mg_configure(size_t max_tail_smem);
 dim3 smooth_grid(const MGLevel& L);
 dim3 coarse_grid(const MGLevel& C);   // restriction into / prolongation from level C
 void launch_smooth_batch(const BatchMap& m, const LevelBatch& L, int color, cudaStream_t st);
+// A level with a sweep plan is read (restriction) or corrected (prolongation) in p2, and its pressure is not cleared.
 void launch_restrict_batch(const BatchMap& m, const LevelBatch& F, const LevelBatch& C, cudaStream_t st);
 void launch_prolong_batch(const BatchMap& m, const LevelBatch& F, const LevelBatch& C, cudaStream_t st);
 // Tails of many simulations in one launch: kind 0 = single-CTA form, 1 = cluster form.  The host fills

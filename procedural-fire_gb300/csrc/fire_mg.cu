@@ -183,13 +183,16 @@ __global__ void __launch_bounds__(LX * LY * LZ) k_restrict_b(const __grid_consta
                                                              const __grid_constant__ LevelBatch C) {
   uint3 blk; int i;
   batch_locate(m, blk, i);
-  restrict_march<TRANSFER_DEPTH, true>((const float*)F.l[i].p, (const float*)F.l[i].b, F.l[i].nx, F.l[i].ny, F.l[i].nz, F.l[i].h, C.l[i].b, C.l[i].p, blk);
+  const MGLevel &f = F.l[i], &c = C.l[i];
+  restrict_march<TRANSFER_DEPTH, true>((const float*)(f.sweep.px ? f.p2 : f.p), (const float*)f.b, f.nx, f.ny, f.nz, f.h, c.b,
+                                       c.sweep.px ? (float*)nullptr : c.p, blk);
 }
 __global__ void __launch_bounds__(LX * LY * LZ) k_prolong_b(const __grid_constant__ BatchMap m, const __grid_constant__ LevelBatch F,
                                                             const __grid_constant__ LevelBatch C) {
   uint3 blk; int i;
   batch_locate(m, blk, i);
-  prolong_march<TRANSFER_DEPTH, true, false>(F.l[i].p, (const float*)C.l[i].p, F.l[i].nx, F.l[i].ny, F.l[i].nz, blk);
+  const MGLevel& f = F.l[i];
+  prolong_march<TRANSFER_DEPTH, true, false>(f.sweep.px ? f.p2 : f.p, (const float*)C.l[i].p, f.nx, f.ny, f.nz, blk);
 }
 
 // ---------------- single-CTA tail V-cycle out of shared memory ----------------

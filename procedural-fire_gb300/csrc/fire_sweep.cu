@@ -234,10 +234,25 @@ __global__ void __launch_bounds__(SW_THREADS, 1) k_sweep2(const T* __restrict__ 
   sweep2_body<T, kZero, kRelax>(p, b, out, nx, ny, nz, h, omega, P.px, P.ty, tile_of(P, nx, ny, nz, blockIdx.x));
 }
 
+// Measured (GB300, ensemble of 16 grids from 32x64x32 to 128x256x128, 4 cycles): 16 launches per level and cycle of batched colour
+// sweeps, 1245 us of a step's 2978, became 4 and the step takes 2486; CTAs of 256 or 448 threads give the same within 1 %.
+// A level of every simulation of a batch: down from p (kZero: from zero) into p2, else back from p2 into p.
+template <bool kZero>
+__global__ void __launch_bounds__(SW_THREADS, 1) k_sweep2_b(const __grid_constant__ BatchMap m, const __grid_constant__ LevelBatch L, int down) {
+  uint3 blk; int i;
+  batch_locate(m, blk, i);
+  const MGLevel& v = L.l[i];
+  const SweepTile t = tile_of(v.sweep, v.nx, v.ny, v.nz, blk.x);
+  const float* p = down ? v.p : v.p2;
+  float* out = down ? v.p2 : v.p;
+  if (v.omega == 1.0f) sweep2_body<float, kZero, false>(p, v.b, out, v.nx, v.ny, v.nz, v.h, v.omega, v.sweep.px, v.sweep.ty, t);
+  else sweep2_body<float, kZero, true>(p, v.b, out, v.nx, v.ny, v.nz, v.h, v.omega, v.sweep.px, v.sweep.ty, t);
+}
+
 constexpr size_t SW_SMEM = 200 * 1024;
 int sweep_threads(const SweepPlan& P) { return std::max(64, (P.px * P.ty + 31) / 32 * 32); }
-size_t sweep_smem(const SweepPlan& P) {
-  return sizeof(float4) * 2 * (size_t)(P.px + 2) * (SW_ROWS * P.ty + 2) + sizeof(float2) * 2 * SW_ROWS * SW_RING * (size_t)sweep_threads(P);
+size_t sweep_smem(const SweepPlan& P, int threads) {
+  return sizeof(float4) * 2 * (size_t)(P.px + 2) * (SW_ROWS * P.ty + 2) + sizeof(float2) * 2 * SW_ROWS * SW_RING * (size_t)threads;
 }
 
 }  // namespace
@@ -246,7 +261,7 @@ size_t sweep_smem(const SweepPlan& P) {
 // warp's chain of four updates, the shared-memory reads and the barrier) and SW_WARP cycles per resident warp (its instructions
 // on one of four schedulers); a CTA runs its planes and eight more, and about SW_START cycles around them.
 constexpr double SW_STEP = 300.0, SW_WARP = 30.0, SW_START = 1500.0;
-SweepPlan plan_sweep(const MGLevel& L, int sms) {
+SweepPlan plan_sweep(const MGLevel& L, int sms, int block) {
   const int nx = L.nx, ny = L.ny, nz = L.nz;
   SweepPlan best{};
   if (L.study || nx % 2 || nx < 8 || ny < 4 || nz < 4) return best;   // odd rows have no aligned pairs: colour launches
@@ -262,9 +277,10 @@ SweepPlan plan_sweep(const MGLevel& L, int sms) {
       if ((ny + cy - 1) / cy != nty) continue;
       const int ty = (std::min(ny, cy + SW_HALO * std::min(nty - 1, 2)) + SW_ROWS - 1) / SW_ROWS;
       SweepPlan P{px, ty, ntx, nty, 1, cx, cy, nz};
-      if (px * ty > SW_THREADS || sweep_smem(P) > SW_SMEM) continue;
-      const int threads = sweep_threads(P);
-      const int occ = std::max(1, std::min({65536 / (128 * threads), (int)(SW_SMEM / sweep_smem(P)), 8}));
+      if (px * ty > (block ? block : SW_THREADS)) continue;
+      const int threads = block ? block : sweep_threads(P);
+      if (sweep_smem(P, threads) > SW_SMEM) continue;
+      const int occ = std::max(1, std::min({65536 / (128 * threads), (int)(SW_SMEM / sweep_smem(P, threads)), 8}));
       int last = 0;
       for (int waves = 1; waves <= 8; ++waves) {   // chunks in z that fill whole waves of the SMs
         const int want = std::max(1, std::min(sms * occ * waves / (ntx * nty), nz / 4));
@@ -287,7 +303,7 @@ cudaError_t launch_sweep2_t(const T* p, const T* b, T* out, const SweepPlan& P, 
                             cudaStream_t st) {
   if (P.px == 0) return cudaErrorInvalidValue;
   const dim3 grid(P.ntx * P.nty * P.ntz), block(sweep_threads(P));
-  const size_t smem = sweep_smem(P);
+  const size_t smem = sweep_smem(P, (int)block.x);
   auto go = [&](auto kernel) { return launch_pdl(kernel, grid, block, smem, st, p, b, out, nx, ny, nz, h, omega, P); };
   if (omega == 1.0f) return zero ? go(k_sweep2<T, true, false>) : go(k_sweep2<T, false, false>);
   if constexpr (sizeof(T) != sizeof(float)) return cudaErrorInvalidValue;   // the refinement's sweeps are Gauss-Seidel
@@ -295,6 +311,12 @@ cudaError_t launch_sweep2_t(const T* p, const T* b, T* out, const SweepPlan& P, 
 }
 cudaError_t launch_sweep2(const MGLevel& L, const float* p, float* out, bool zero, cudaStream_t st) {
   return launch_sweep2_t<float>(p, L.b, out, L.sweep, L.nx, L.ny, L.nz, L.h, L.omega, zero, st);
+}
+
+cudaError_t launch_sweep2_batch(const BatchMap& m, const LevelBatch& L, bool down, bool zero, cudaStream_t st) {
+  size_t smem = 0;
+  for (int k = 0; k < m.n; ++k) smem = std::max(smem, sweep_smem(L.l[m.inst[k]].sweep, SW_BATCH_THREADS));
+  return launch_pdl(zero ? k_sweep2_b<true> : k_sweep2_b<false>, dim3(m.prefix[m.n]), dim3(SW_BATCH_THREADS), smem, st, m, L, (int)down);
 }
 
 template cudaError_t launch_sweep2_t<float>(const float*, const float*, float*, const SweepPlan&, int, int, int, float, float, bool, cudaStream_t);
@@ -350,6 +372,8 @@ cudaError_t sweep_configure() {
   opt_in(k_sweep2<float, true, false>);
   opt_in(k_sweep2<float, false, true>);
   opt_in(k_sweep2<float, true, true>);
+  opt_in(k_sweep2_b<false>);
+  opt_in(k_sweep2_b<true>);
   opt_in(k_sweep2<__half, false, false>);
   opt_in(k_sweep2<__half, true, false>);
   opt_in(k_sweep2<__nv_bfloat16, false, false>);

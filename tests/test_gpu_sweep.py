@@ -68,3 +68,27 @@ def test_refinement_forms_reach_the_tolerance(precision, res):
     assert abs(rel - out["rel_residual"]) <= 1e-5 * out["rel_residual"] + 1e-12
     assert out["rel_residual"] <= (0.9 * out["rel_residual_initial"] if single else 1e-6)
     ps.close()
+
+
+def test_batched_sweeps_match_members_alone():
+    """Members of very different sizes share each batched two-sweep launch (tiles cut for a share of the SMs), one whose
+    second level only it has outside its coarse end: after the first step from rest their
+    pressures equal those of the same simulations stepped alone (same operations, same order)."""
+    import fire_sim as F
+    import test_gpu_ensemble as E
+    members = [dict(res=r, size=tuple(0.0125 * k for k in r), seed=20 + i, spots=4)
+               for i, r in enumerate([(46, 92, 44), (64, 128, 64), (200, 60, 100), (160, 200, 120)])]
+    ens = F.Ensemble(members, vcycles=2)
+    alone = [F.FireSim(res=m["res"], size=m["size"], vcycles=2) for m in members]
+    for k, m in enumerate(members):
+        for s in (ens.members[k], alone[k]):
+            E._configure(s, m)
+    ens.step(E.DT, 1)
+    ens.sync()
+    for a, b in zip(ens.members, alone):
+        b.step(E.DT, 1)
+        b.sync()
+        assert float(np.abs(b.level(0, "p")).max()) > 0.0
+        np.testing.assert_array_equal(a.level(0, "p"), b.level(0, "p"))
+        b.close()
+    ens.close()
