@@ -202,14 +202,22 @@ __device__ __forceinline__ float4 h4(uint2 v) {
   float2 fa = __half22float2(a), fb = __half22float2(b);
   return make_float4(fa.x, fa.y, fb.x, fb.y);
 }
-__device__ __forceinline__ int wrapN(long long i) { long long m = i % TABLE_N; return (int)(m < 0 ? m + TABLE_N : m); }
+// Entry below u in the repeating table and the next one.  floor(u) mod TABLE_N without 64-bit arithmetic: in 32 bits the low
+// bits are those of the exact integer, and beyond 2^31 every float is a multiple of TABLE_N (a power of two).
+__device__ __forceinline__ void wrap_axis(float u, int& i0, int& i1, float& f) {
+  static_assert((TABLE_N & (TABLE_N - 1)) == 0 && TABLE_N <= 256, "a mask wraps");
+  const float fl = floorf(u);
+  f = u - fl;
+  i0 = fabsf(u) < 2147483648.0f ? (int)fl & (TABLE_N - 1) : 0;
+  i1 = (i0 + 1) & (TABLE_N - 1);
+}
 __device__ __forceinline__ float4 sample_table(const uint2* __restrict__ tab, f3 q) {
   const float N = (float)TABLE_N;
-  float ux = q.x * N - 0.5f, uy = q.y * N - 0.5f, uz = q.z * N - 0.5f;
-  float flx = floorf(ux), fly = floorf(uy), flz = floorf(uz);
-  float fx = ux - flx, fy = uy - fly, fz = uz - flz;
-  long long ix = (long long)flx, iy = (long long)fly, iz = (long long)flz;
-  int x0 = wrapN(ix), x1 = wrapN(ix + 1), y0 = wrapN(iy), y1 = wrapN(iy + 1), z0 = wrapN(iz), z1 = wrapN(iz + 1);
+  int x0, x1, y0, y1, z0, z1;
+  float fx, fy, fz;
+  wrap_axis(q.x * N - 0.5f, x0, x1, fx);
+  wrap_axis(q.y * N - 0.5f, y0, y1, fy);
+  wrap_axis(q.z * N - 0.5f, z0, z1, fz);
   auto T = [&](int x, int y, int z) { return h4(__ldg(tab + x + TABLE_N * (y + TABLE_N * z))); };
   float4 c00 = lerp4(T(x0, y0, z0), T(x1, y0, z0), fx);
   float4 c10 = lerp4(T(x0, y1, z0), T(x1, y1, z0), fx);

@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(SW_THREADS, 1) k_sweep2(const T* __restrict__ 
   sweep2_body<T, kZero, kRelax>(p, b, out, nx, ny, nz, h, omega, P.px, P.ty, tile_of(P, nx, ny, nz, blockIdx.x));
 }
 
-// Measured (GB300, ensemble of 16 grids from 32x64x32 to 128x256x128, 4 cycles): 16 launches per level and cycle of batched colour
+// Measured (GB300, ensemble of 16 grids from 32x64x32 to 96x192x96, 4 cycles): 16 launches per level and cycle of batched colour
 // sweeps, 1245 us of a step's 2978, became 4 and the step takes 2486; CTAs of 256 or 448 threads give the same within 1 %.
 // A level of every simulation of a batch: down from p (kZero: from zero) into p2, else back from p2 into p.
 template <bool kZero>
