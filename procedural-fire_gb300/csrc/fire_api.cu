@@ -1167,7 +1167,8 @@ int ens_top(const FireSim* s) {
 // and the multigrid's per-level maps and level tables.
 struct EnsCtx {
   StepBatch SB;
-  BatchMap cell[CELL_TILES], forces[FORCES_TILES];
+  BatchMap adv1[CELL_TILES], cell[CELL_TILES], flow[CELL_TILES], forces[FORCES_TILES];   // adv1; adv2; div and project; forces
+  int adv1Depth = 1, flowDepth = 1;
   int depth = 0;
   std::vector<BatchMap> sweepMap, smoothMap, coarseMap;   // two-sweep tiles; colour launches (levels without a plan); transfers
   std::vector<LevelBatch> LB;
@@ -1175,17 +1176,25 @@ struct EnsCtx {
 void ens_context(FireEnsemble* e, EnsCtx& c) {
   const int n = (int)e->sims.size();
   std::memset(&c.SB, 0, sizeof c.SB);
+  for (auto& m : c.adv1) m = map_empty();
   for (auto& m : c.cell) m = map_empty();
+  for (auto& m : c.flow) m = map_empty();
   for (auto& m : c.forces) m = map_empty();
   c.depth = 0;
   double cells = 0.0;
+  for (const FireSim* s : e->sims) cells += (double)s->d.nx * s->d.ny * s->d.nz;
+  c.adv1Depth = adv1_depth((long)cells);
+  c.flowDepth = flow_depth((long)cells);
   for (int i = 0; i < n; ++i) {
     FireSim* s = e->sims[i];
     c.SB.s[i] = StepInst{e->dBlocks + (size_t)i * BLOCK_FLOATS, s->f, s->d, s->levels[0].b, s->levels[0].p};
-    for (int v = 0; v < CELL_TILES; ++v) map_add(c.cell[v], i, step_grid(s->d, v));
+    for (int v = 0; v < CELL_TILES; ++v) {
+      map_add(c.adv1[v], i, step_grid(s->d, v, c.adv1Depth));
+      map_add(c.cell[v], i, step_grid(s->d, v));
+      map_add(c.flow[v], i, step_grid(s->d, v, c.flowDepth));
+    }
     for (int v = 0; v < FORCES_TILES; ++v) map_add(c.forces[v], i, forces_grid(s->d, v));
     c.depth = std::max(c.depth, ens_top(s));
-    cells += (double)s->d.nx * s->d.ny * s->d.nz;
   }
   // per level: the members that have it outside their tail, and every member's level l and l + 1
   c.sweepMap.assign(c.depth, map_empty());
@@ -1214,11 +1223,11 @@ void ens_context(FireEnsemble* e, EnsCtx& c) {
 }
 void ens_stage(FireEnsemble* e, const EnsCtx& c, int stage, int tile, cudaStream_t st) {
   switch (stage) {
-    case 0: launch_adv1_batch(c.cell[tile], c.SB, tile, st); break;
+    case 0: launch_adv1_batch(c.adv1[tile], c.SB, tile, c.adv1Depth, st); break;
     case 1: launch_adv2_batch(c.cell[tile], c.SB, tile, st); break;
     case 2: launch_forces_batch(c.forces[tile], c.SB, e->sims[0]->noise, e->sims[0]->curl, tile, st); break;
-    case 3: launch_div_batch(c.cell[tile], c.SB, tile, st); break;
-    default: launch_project_batch(c.cell[tile], c.SB, tile, st); break;
+    case 3: launch_div_batch(c.flow[tile], c.SB, tile, c.flowDepth, st); break;
+    default: launch_project_batch(c.flow[tile], c.SB, tile, c.flowDepth, st); break;
   }
 }
 // Two sweeps of level l of every member that smooths it by launches.

@@ -139,13 +139,17 @@ void launch_project(const float* P, Fields f, const float* p0, Dims d, cudaStrea
 // tile (16, 8, 32).  Every candidate computes the same per-cell arithmetic.
 constexpr int CELL_TILES = 4, FORCES_TILES = 3;
 // Block grids of the per-cell stages (adv1, adv2, div, project) and of the tiled forces stage, per candidate.
-dim3 step_grid(Dims d, int tile = 0);
+dim3 step_grid(Dims d, int tile = 0, int depth = 1);
+// Cells a thread of adv1, or of div and project, takes along z: for a grid (or a batch) of so many cells.
+constexpr int ADV1_DEPTH = 2, FLOW_DEPTH = 4;
+int adv1_depth(long cells);
+int flow_depth(long cells);
 dim3 forces_grid(Dims d, int tile = 0);
-void launch_adv1_batch(const BatchMap& m, const StepBatch& I, int tile, cudaStream_t st);
+void launch_adv1_batch(const BatchMap& m, const StepBatch& I, int tile, int depth, cudaStream_t st);
 void launch_adv2_batch(const BatchMap& m, const StepBatch& I, int tile, cudaStream_t st);
 void launch_forces_batch(const BatchMap& m, const StepBatch& I, const uint2* noise, const uint2* curl, int tile, cudaStream_t st);
-void launch_div_batch(const BatchMap& m, const StepBatch& I, int tile, cudaStream_t st);
-void launch_project_batch(const BatchMap& m, const StepBatch& I, int tile, cudaStream_t st);
+void launch_div_batch(const BatchMap& m, const StepBatch& I, int tile, int depth, cudaStream_t st);
+void launch_project_batch(const BatchMap& m, const StepBatch& I, int tile, int depth, cudaStream_t st);
 
 // ---- kernel launchers (fire_sweep.cu) ----
 // Two red-black sweeps from p (zero: from zero) into out; bit-identical to the four colour launches.

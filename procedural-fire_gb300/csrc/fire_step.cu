@@ -29,19 +29,22 @@ struct CellId { int i, j, k; bool ok; };
 // instantiated for every CELL_TILES entry and the ensemble's autotuner picks one per stage.
 template <int TX, int TY, int TZ> struct Tile { static constexpr int X = TX, Y = TY, Z = TZ; };
 using Tile0 = Tile<BX, BY, BZ>;
-template <class T = Tile0>
+// K: consecutive z cells of a thread (id.k is the first).
+template <class T = Tile0, int K = 1>
 __device__ __forceinline__ CellId cell_id(Dims d, uint3 blk) {
   pdl_wait();
   pdl_trigger();
   CellId c;
   c.i = blk.x * T::X + threadIdx.x;
   c.j = blk.y * T::Y + threadIdx.y;
-  c.k = blk.z * T::Z + threadIdx.z;
+  c.k = (blk.z * T::Z + threadIdx.z) * K;
   c.ok = c.i < d.nx && c.j < d.ny && c.k < d.nz;
   return c;
 }
 __device__ __forceinline__ CellId cell_id(Dims d) { return cell_id<Tile0>(d, blockIdx); }
-static dim3 grid_for(Dims d) { return dim3((d.nx + BX - 1) / BX, (d.ny + BY - 1) / BY, (d.nz + BZ - 1) / BZ); }
+static dim3 grid_for(Dims d, int depth = 1) {
+  return dim3((d.nx + BX - 1) / BX, (d.ny + BY - 1) / BY, (d.nz + BZ * depth - 1) / (BZ * depth));
+}
 static dim3 block_shape() { return dim3(BX, BY, BZ); }
 
 
@@ -62,6 +65,104 @@ __device__ __forceinline__ void adv1_body(const float* __restrict__ P, const Fie
   f.velX[ci] = make_float4(mixf(wind.x, sv.x, fade), mixf(wind.y, sv.y, fade), mixf(wind.z, sv.z, fade), 0.0f);
   f.SX[ci] = mul4(sample(f.S, t, d), fade);
   f.S2X[ci] = mul4(sample(f.S2, t, d), fade);
+}
+
+// ---- adv1 with two cells a thread ----
+// adv1 is bound by the L1's data path (177 wavefronts per warp and cell, 72 % of its rate, at 128x256x128): a float4 texel of
+// a row costs four to five, and a trilinear sample eight texels.  A thread with two cells, one above the other, mostly samples
+// points one cell apart, so the upper four texels of the first sample are the lower four of the second: they are kept, and
+// loaded again only where the two floors differ.  A sample is formed from the same texels by the same operations as sample() in
+// adv1_body, plane by plane; which product of a lerp the compiler rounds there (measured: of a x lerp of velocities the
+// first, elsewhere the second) is written out, so the results are the same bits.
+// adv2, whose stencils' ranges double the arithmetic, gains nothing from it (256x512x256: 1469 -> 1508 us).
+struct Corner { int o, dx, dy, dz; };   // offset of a 2 x 2 x 2 stencil's first cell and the steps to the second ones (0 at a clamped edge)
+struct Weights { float x, y, z; };
+__device__ __forceinline__ void corner_of(const Tap& t, Dims d, Corner& c, Weights& w) {
+  const int sy = d.nx, sz = d.nx * d.ny;
+  c.o = t.x0 + t.y0 * sy + t.z0 * sz;
+  c.dx = t.x1 - t.x0;
+  c.dy = (t.y1 - t.y0) * sy;
+  c.dz = (t.z1 - t.z0) * sz;
+  w.x = t.fx; w.y = t.fy; w.z = t.fz;
+}
+struct Quad { float4 a, b, c, e; };     // (x0, y0), (x1, y0), (x0, y1), (x1, y1) of one plane
+__device__ __forceinline__ void load_quad(Quad& q, const float4* __restrict__ f, int o, const Corner& c) {
+  q.a = __ldg(f + o);
+  q.b = __ldg(f + (o + c.dx));
+  q.c = __ldg(f + (o + c.dy));
+  q.e = __ldg(f + (o + c.dy + c.dx));
+}
+// Whether the upper plane of stencil a is the lower plane of stencil b.
+__device__ __forceinline__ bool same_plane(const Corner& a, const Corner& b) { return a.o + a.dz == b.o && a.dx == b.dx && a.dy == b.dy; }
+// a (1 - t) + b t with one product inside an FMA: the first one, or (kSecond) the second.
+template <bool kSecond>
+__device__ __forceinline__ float4 lerp_as(const float4& a, const float4& b, float t) {
+  const float s = 1.0f - t;
+  auto one = [&](float p, float q) { return kSecond ? __fmaf_rn(q, t, __fmul_rn(p, s)) : __fmaf_rn(p, s, __fmul_rn(q, t)); };
+  return make_float4(one(a.x, b.x), one(a.y, b.y), one(a.z, b.z), one(a.w, b.w));
+}
+template <bool kVel>
+__device__ __forceinline__ float4 bilinear(const Quad& q, const Weights& w) {
+  return lerp_as<false>(lerp_as<kVel>(q.a, q.b, w.x), lerp_as<kVel>(q.c, q.e, w.x), w.y);
+}
+// K samples of a field, K stencils one above the other.
+template <bool kVel, int K>
+__device__ __forceinline__ void sample_column(float4 (&out)[K], const float4* __restrict__ f, const Corner (&c)[K], const Weights (&w)[K]) {
+  Quad q;
+  load_quad(q, f, c[0].o, c[0]);
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    if (k > 0 && !same_plane(c[k > 0 ? k - 1 : 0], c[k])) load_quad(q, f, c[k].o, c[k]);
+    const float4 lo = bilinear<kVel>(q, w[k]);
+    load_quad(q, f, c[k].o + c[k].dz, c[k]);
+    out[k] = lerp_as<false>(lo, bilinear<kVel>(q, w[k]), w[k].z);
+  }
+}
+template <class TileT, int K>
+__device__ __forceinline__ void adv1_column(const float* __restrict__ P, const Fields& f, Dims d, uint3 blk) {
+  CellId id = cell_id<TileT, K>(d, blk);
+  if (!id.ok) return;
+  const float dt = __ldg(P + P_dt), dx = __ldg(P + P_dx);
+  const unsigned plane = (unsigned)(d.nx * d.ny), c0 = (unsigned)(id.i + d.nx * id.j) + plane * (unsigned)id.k;
+  unsigned ci[K];   // a cell above the domain repeats the top one and is not stored
+  f3 c[K], v[K], b[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int z = min(id.k + k, d.nz - 1);
+    ci[k] = c0 + plane * (unsigned)(z - id.k);
+    c[k] = mk3((float)id.i + 0.5f, (float)id.j + 0.5f, (float)z + 0.5f);
+    v[k] = xyz(__ldg(f.vel + ci[k]));
+  }
+  Corner at[K];
+  Weights w[K];
+  float4 s[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) corner_of(make_tap(c[k] - v[k] * (0.5f * dt) / dx, d), d, at[k], w[k]);
+  sample_column<true>(s, f.vel, at, w);
+  float fade[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    b[k] = c[k] - xyz(s[k]) * dt / dx;
+    fade[k] = outside_fade(b[k], d);
+    corner_of(make_tap(b[k], d), d, at[k], w[k]);
+  }
+  sample_column<true>(s, f.vel, at, w);
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const float ws = sstep(0.03f, 0.4f, b[k].y * dx);
+    const f3 wind = mk3(__ldg(P + P_windX) * ws, 0.0f * ws, __ldg(P + P_windZ) * ws);
+    const f3 sv = xyz(s[k]);
+    if (id.k + k < d.nz)
+      f.velX[ci[k]] = make_float4(mixf(wind.x, sv.x, fade[k]), mixf(wind.y, sv.y, fade[k]), mixf(wind.z, sv.z, fade[k]), 0.0f);
+  }
+  sample_column<false>(s, f.S, at, w);
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+    if (id.k + k < d.nz) f.SX[ci[k]] = mul4(s[k], fade[k]);
+  sample_column<false>(s, f.S2, at, w);
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+    if (id.k + k < d.nz) f.S2X[ci[k]] = mul4(s[k], fade[k]);
 }
 
 // ---------------- adv2 (src/sim.js:159-197) ----------------
@@ -532,50 +633,71 @@ __device__ __forceinline__ void forces_tiled_body(const float* __restrict__ P, c
 constexpr size_t FORCES_TILED_SMEM = sizeof(float4) * 5 * VX * VY + sizeof(float) * 3 * WX * WY;
 
 // ---------------- divergence minus the expansion target (src/sim.js:399-413) ----------------
-template <class TileT = Tile0>
+// The z neighbours of a thread's K cells are its own cells.
+template <class TileT = Tile0, int K = 1>
 __device__ __forceinline__ void div_body(const float* __restrict__ P, const float4* __restrict__ velX, float* __restrict__ b0, Dims d,
                                          uint3 blk) {
-  CellId id = cell_id<TileT>(d, blk);
+  CellId id = cell_id<TileT, K>(d, blk);
   if (!id.ok) return;
-  const int i = id.i, j = id.j, k = id.k;
-  const size_t ci = cell(i, j, k, d.nx, d.ny);
+  const int i = id.i, j = id.j;
   const float dx = __ldg(P + P_dx);
+  const int plane = d.nx * d.ny;
+  int ci = i + d.nx * j + plane * id.k;
+  const int xm = i > 0 ? -1 : 0, xp = i < d.nx - 1 ? 1 : 0, ym = j > 0 ? -d.nx : 0, yp = j < d.ny - 1 ? d.nx : 0;
   float4 me = __ldg(velX + ci);
-  float L = ldc(velX, i - 1, j, k, d).x, R = ldc(velX, i + 1, j, k, d).x;
-  float B = ldc(velX, i, j - 1, k, d).y, T = ldc(velX, i, j + 1, k, d).y;
-  float K = ldc(velX, i, j, k - 1, d).z, F = ldc(velX, i, j, k + 1, d).z;
-  if (j == 0) B = -me.y;   // solid floor
-  b0[ci] = ((R - L) + (T - B) + (F - K)) / (2.0f * dx) - me.w;
+  float below = id.k > 0 ? __ldg(velX + (ci - plane)).z : me.z;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    if (k > 0 && id.k + k >= d.nz) break;
+    const float4 above = id.k + k < d.nz - 1 ? __ldg(velX + (ci + plane)) : me;
+    const float L = __ldg(velX + (ci + xm)).x, R = __ldg(velX + (ci + xp)).x;
+    float B = __ldg(velX + (ci + ym)).y;
+    const float T = __ldg(velX + (ci + yp)).y;
+    if (j == 0) B = -me.y;   // solid floor
+    b0[ci] = ((R - L) + (T - B) + (above.z - below)) / (2.0f * dx) - me.w;
+    below = me.z;
+    me = above;
+    ci += plane;
+  }
 }
 
 // ---------------- projection (src/sim.js:526-550) ----------------
-__device__ __forceinline__ float pr(const float* __restrict__ p, int x, int y, int z, Dims d, float me) {
-  if (x < 0 || z < 0 || x >= d.nx || z >= d.nz || y >= d.ny) return -me;   // open sides/top: p = 0 on the face
-  if (y < 0) return me;                                                    // floor: Neumann
-  return __ldg(p + cell(x, y, z, d.nx, d.ny));
-}
-template <class TileT = Tile0>
+// Ghosts: open sides and top, p = 0 on the face (-me); floor, Neumann (me).  The z neighbours of a thread's K cells are its own.
+template <class TileT = Tile0, int K = 1>
 __device__ __forceinline__ void project_body(const float* __restrict__ P, const float4* __restrict__ velX, const float* __restrict__ p0,
                                              const unsigned char* __restrict__ solid, float4* __restrict__ vel, Dims d, uint3 blk) {
-  CellId id = cell_id<TileT>(d, blk);
+  CellId id = cell_id<TileT, K>(d, blk);
   if (!id.ok) return;
-  const int i = id.i, j = id.j, k = id.k;
-  const size_t ci = cell(i, j, k, d.nx, d.ny);
+  const int i = id.i, j = id.j;
   const float dx = __ldg(P + P_dx);
+  const int plane = d.nx * d.ny;
+  int ci = i + d.nx * j + plane * id.k;
   float me = __ldg(p0 + ci);
-  f3 g = mk3(pr(p0, i + 1, j, k, d, me) - pr(p0, i - 1, j, k, d, me),
-             pr(p0, i, j + 1, k, d, me) - pr(p0, i, j - 1, k, d, me),
-             pr(p0, i, j, k + 1, d, me) - pr(p0, i, j, k - 1, d, me)) / (2.0f * dx);
-  f3 v = xyz(__ldg(velX + ci)) - g;
-  if (__ldg(solid + ci)) v = mk3(0.0f, 0.0f, 0.0f);   // geo.b > 0.5
-  if (j == 0) v.y = fmaxf(v.y, 0.0f);
-  float vl = len3(v);
-  if (vl > 20.0f || isnan(vl)) v = isnan(vl) ? mk3(0.0f, 0.0f, 0.0f) : v * 20.0f / vl;
-  vel[ci] = make_float4(v.x, v.y, v.z, 0.0f);
+  float below = id.k > 0 ? __ldg(p0 + (ci - plane)) : -me;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    if (k > 0 && id.k + k >= d.nz) break;
+    const float above = id.k + k < d.nz - 1 ? __ldg(p0 + (ci + plane)) : -me;
+    const float xm = i > 0 ? __ldg(p0 + (ci - 1)) : -me, xp = i < d.nx - 1 ? __ldg(p0 + (ci + 1)) : -me;
+    const float ym = j > 0 ? __ldg(p0 + (ci - d.nx)) : me, yp = j < d.ny - 1 ? __ldg(p0 + (ci + d.nx)) : -me;
+    const f3 g = mk3(xp - xm, yp - ym, above - below) / (2.0f * dx);
+    f3 v = xyz(__ldg(velX + ci)) - g;
+    if (__ldg(solid + ci)) v = mk3(0.0f, 0.0f, 0.0f);   // geo.b > 0.5
+    if (j == 0) v.y = fmaxf(v.y, 0.0f);
+    float vl = len3(v);
+    if (vl > 20.0f || isnan(vl)) v = isnan(vl) ? mk3(0.0f, 0.0f, 0.0f) : v * 20.0f / vl;
+    vel[ci] = make_float4(v.x, v.y, v.z, 0.0f);
+    below = me;
+    me = above;
+    ci += plane;
+  }
 }
 
 // ---------------- per-simulation kernels ----------------
 __global__ void __launch_bounds__(256, FIRE_ADV_MIN_CTAS) k_adv1(const float* __restrict__ P, Fields f, Dims d) { adv1_body(P, f, d, blockIdx); }
+__global__ void __launch_bounds__(256, FIRE_ADV_MIN_CTAS) k_adv1_column(const float* __restrict__ P, Fields f, Dims d) {
+  adv1_column<Tile0, ADV1_DEPTH>(P, f, d, blockIdx);
+}
 __global__ void __launch_bounds__(256, FIRE_ADV_MIN_CTAS) k_adv2(const float* __restrict__ P, Fields f, Dims d) { adv2_body(P, f, d, blockIdx); }
 // One wave of resident CTAs.  The (column tile, plane) units, planes fastest, are split into gridDim.x equal
 // contiguous ranges, so every SM marches the same number of planes (a grid of fixed-depth chunks leaves its
@@ -611,25 +733,28 @@ __global__ void __launch_bounds__(FT_X * FT_Y, FIRE_FORCES_MIN_CTAS) k_forces_ti
 }
 // mg_counter (the residual-driven step graph only, else null): the solve that follows counts its V-cycles
 // from zero, so this kernel clears the count instead of a separate launch.
+template <int K>
 __global__ void __launch_bounds__(256) k_div(const float* __restrict__ P, const float4* __restrict__ velX, float* __restrict__ b0, Dims d,
                                              int* __restrict__ mg_counter) {
-  div_body(P, velX, b0, d, blockIdx);
+  div_body<Tile0, K>(P, velX, b0, d, blockIdx);
   if (mg_counter && (blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x | threadIdx.y | threadIdx.z) == 0) *mg_counter = 0;
 }
+template <int K>
 __global__ void __launch_bounds__(256) k_project(const float* __restrict__ P, const float4* __restrict__ velX, const float* __restrict__ p0,
                                                  const unsigned char* __restrict__ solid, float4* __restrict__ vel, Dims d) {
-  project_body(P, velX, p0, solid, vel, d, blockIdx);
+  project_body<Tile0, K>(P, velX, p0, solid, vel, d, blockIdx);
 }
 
 // ---------------- batched kernels: one grid over many independent simulations ----------------
 // Each CTA finds its simulation and its position in that simulation's grid from the flat block index
 // (BatchMap), then runs the same body as the per-simulation kernel: the arithmetic, and so the results,
 // are those of stepping each simulation alone.
-template <class T>
+template <class T, int K>
 __global__ void __launch_bounds__(256, FIRE_ADV_MIN_CTAS) k_adv1_b(const __grid_constant__ BatchMap m, const __grid_constant__ StepBatch I) {
   uint3 blk; int i;
   batch_locate(m, blk, i);
-  adv1_body<T>(I.s[i].P, I.s[i].f, I.s[i].d, blk);
+  if (K > 1) adv1_column<T, K>(I.s[i].P, I.s[i].f, I.s[i].d, blk);
+  else adv1_body<T>(I.s[i].P, I.s[i].f, I.s[i].d, blk);
 }
 template <class T>
 __global__ void __launch_bounds__(256, FIRE_ADV_MIN_CTAS) k_adv2_b(const __grid_constant__ BatchMap m, const __grid_constant__ StepBatch I) {
@@ -645,17 +770,17 @@ __global__ void __launch_bounds__(FT_X * FT_Y, FIRE_FORCES_MIN_CTAS) k_forces_b(
   batch_locate(m, blk, i);
   forces_tiled_body<ZD>(I.s[i].P, I.s[i].f, noiseT, curlT, I.s[i].d, blk, fsm);
 }
-template <class T>
+template <class T, int K>
 __global__ void __launch_bounds__(256) k_div_b(const __grid_constant__ BatchMap m, const __grid_constant__ StepBatch I) {
   uint3 blk; int i;
   batch_locate(m, blk, i);
-  div_body<T>(I.s[i].P, I.s[i].f.velX, I.s[i].b0, I.s[i].d, blk);
+  div_body<T, K>(I.s[i].P, I.s[i].f.velX, I.s[i].b0, I.s[i].d, blk);
 }
-template <class T>
+template <class T, int K>
 __global__ void __launch_bounds__(256) k_project_b(const __grid_constant__ BatchMap m, const __grid_constant__ StepBatch I) {
   uint3 blk; int i;
   batch_locate(m, blk, i);
-  project_body<T>(I.s[i].P, I.s[i].f.velX, I.s[i].p0, I.s[i].f.solid, I.s[i].f.vel, I.s[i].d, blk);
+  project_body<T, K>(I.s[i].P, I.s[i].f.velX, I.s[i].p0, I.s[i].f.solid, I.s[i].f.vel, I.s[i].d, blk);
 }
 
 // The tile candidates of the batched stages: CELL_TILES cell tiles (256 threads each; x stays 32 or 64 wide
@@ -679,7 +804,19 @@ template <class F> void with_forces_depth(int v, F&& f) {
 }
 
 // ---------------- launchers ----------------
-void launch_adv1(const float* P, Fields f, Dims d, cudaStream_t st) { launch_pdl(k_adv1, grid_for(d), block_shape(), 0, st, P, f, d); }
+// A thread takes several cells along z where enough threads remain to fill the SMs.  Measured (GB300, us, one cell -> several):
+// adv1 50x98x50 16.8 -> 17.5, 64x128x64 22.0 -> 22.5, 80x120x80 30.5 -> 29.1, 96x192x96 56.1 -> 51.4, 128x256x128 119 -> 106,
+// 256x512x256 873 -> 755; div and project together 64x128x64 16.4 -> 18.3, 80x120x80 20.4 -> 18.8, 128x256x128 61.4 -> 57.5,
+// 256x512x256 390 -> 354.  In a batch all members count: a CTA of one cell a thread is short against finding its
+// simulation (64x128x64 and 96x192x96 together: adv1 75 -> 63, div 19 -> 12.5, project 31 -> 16).
+constexpr long ADV1_DEEP_CELLS = 600000, FLOW_DEEP_CELLS = 700000;
+static long cells_of(Dims d) { return (long)d.nx * d.ny * d.nz; }
+int adv1_depth(long cells) { return cells >= ADV1_DEEP_CELLS ? ADV1_DEPTH : 1; }
+int flow_depth(long cells) { return cells >= FLOW_DEEP_CELLS ? FLOW_DEPTH : 1; }
+void launch_adv1(const float* P, Fields f, Dims d, cudaStream_t st) {
+  const int K = adv1_depth(cells_of(d));
+  launch_pdl(K > 1 ? k_adv1_column : k_adv1, grid_for(d, K), block_shape(), 0, st, P, f, d);
+}
 void launch_adv2(const float* P, Fields f, Dims d, cudaStream_t st) { launch_pdl(k_adv2, grid_for(d), block_shape(), 0, st, P, f, d); }
 void launch_curl(Fields f, Dims d, cudaStream_t st) { launch_pdl(k_curl, grid_for(d), block_shape(), 0, st, f, d); }
 // Resident k_forces_tiled CTAs of each device (CTAs per SM x SMs), set by step_configure.
@@ -727,11 +864,11 @@ cudaError_t step_configure() {
   return e;
 }
 // Block grids of the batched stages for a simulation of dims d with tile candidate `tile`.
-dim3 step_grid(Dims d, int tile) {
+dim3 step_grid(Dims d, int tile, int depth) {
   dim3 g;
   with_cell_tile(tile, [&](auto t) {
     using T = decltype(t);
-    g = dim3((d.nx + T::X - 1) / T::X, (d.ny + T::Y - 1) / T::Y, (d.nz + T::Z - 1) / T::Z);
+    g = dim3((d.nx + T::X - 1) / T::X, (d.ny + T::Y - 1) / T::Y, (d.nz + T::Z * depth - 1) / (T::Z * depth));
   });
   return g;
 }
@@ -739,10 +876,10 @@ dim3 forces_grid(Dims d, int tile) {
   const int zd = kForcesDepth[tile >= 0 && tile < FORCES_TILES ? tile : 0];
   return dim3((d.nx + FT_X - 1) / FT_X, (d.ny + FT_Y - 1) / FT_Y, (d.nz + zd - 1) / zd);
 }
-void launch_adv1_batch(const BatchMap& m, const StepBatch& I, int tile, cudaStream_t st) {
+void launch_adv1_batch(const BatchMap& m, const StepBatch& I, int tile, int depth, cudaStream_t st) {
   with_cell_tile(tile, [&](auto t) {
     using T = decltype(t);
-    launch_pdl(k_adv1_b<T>, dim3(m.prefix[m.n]), dim3(T::X, T::Y, T::Z), 0, st, m, I);
+    launch_pdl(depth > 1 ? k_adv1_b<T, ADV1_DEPTH> : k_adv1_b<T, 1>, dim3(m.prefix[m.n]), dim3(T::X, T::Y, T::Z), 0, st, m, I);
   });
 }
 void launch_adv2_batch(const BatchMap& m, const StepBatch& I, int tile, cudaStream_t st) {
@@ -756,26 +893,28 @@ void launch_forces_batch(const BatchMap& m, const StepBatch& I, const uint2* noi
     launch_pdl(k_forces_b<decltype(z)::value>, dim3(m.prefix[m.n]), dim3(FT_X, FT_Y), FORCES_TILED_SMEM, st, m, I, noise, curl);
   });
 }
-void launch_div_batch(const BatchMap& m, const StepBatch& I, int tile, cudaStream_t st) {
+void launch_div_batch(const BatchMap& m, const StepBatch& I, int tile, int depth, cudaStream_t st) {
   with_cell_tile(tile, [&](auto t) {
     using T = decltype(t);
-    launch_pdl(k_div_b<T>, dim3(m.prefix[m.n]), dim3(T::X, T::Y, T::Z), 0, st, m, I);
+    launch_pdl(depth > 1 ? k_div_b<T, FLOW_DEPTH> : k_div_b<T, 1>, dim3(m.prefix[m.n]), dim3(T::X, T::Y, T::Z), 0, st, m, I);
   });
 }
-void launch_project_batch(const BatchMap& m, const StepBatch& I, int tile, cudaStream_t st) {
+void launch_project_batch(const BatchMap& m, const StepBatch& I, int tile, int depth, cudaStream_t st) {
   with_cell_tile(tile, [&](auto t) {
     using T = decltype(t);
-    launch_pdl(k_project_b<T>, dim3(m.prefix[m.n]), dim3(T::X, T::Y, T::Z), 0, st, m, I);
+    launch_pdl(depth > 1 ? k_project_b<T, FLOW_DEPTH> : k_project_b<T, 1>, dim3(m.prefix[m.n]), dim3(T::X, T::Y, T::Z), 0, st, m, I);
   });
 }
 void launch_forces_unfused(const float* P, Fields f, const uint2* noise, const uint2* curl, Dims d, cudaStream_t st) {
   launch_pdl(k_forces<false>, grid_for(d), block_shape(), 0, st, P, f, noise, curl, d);
 }
 void launch_div(const float* P, Fields f, float* b0, Dims d, cudaStream_t st, int* mg_counter) {
-  launch_pdl(k_div, grid_for(d), block_shape(), 0, st, P, (const float4*)f.velX, b0, d, mg_counter);
+  const int K = flow_depth(cells_of(d));
+  launch_pdl(K > 1 ? k_div<FLOW_DEPTH> : k_div<1>, grid_for(d, K), block_shape(), 0, st, P, (const float4*)f.velX, b0, d, mg_counter);
 }
 void launch_project(const float* P, Fields f, const float* p0, Dims d, cudaStream_t st) {
-  launch_pdl(k_project, grid_for(d), block_shape(), 0, st, P, (const float4*)f.velX, p0, (const unsigned char*)f.solid, f.vel, d);
+  const int K = flow_depth(cells_of(d));
+  launch_pdl(K > 1 ? k_project<FLOW_DEPTH> : k_project<1>, grid_for(d, K), block_shape(), 0, st, P, (const float4*)f.velX, p0, (const unsigned char*)f.solid, f.vel, d);
 }
 
 }  // namespace fire
@@ -784,6 +923,6 @@ namespace fire {
 // Verifies that this library carries a kernel image for the current device.
 cudaError_t kernels_probe() {
   cudaFuncAttributes a;
-  return cudaFuncGetAttributes(&a, k_div);
+  return cudaFuncGetAttributes(&a, k_div<1>);
 }
 }  // namespace fire
