@@ -146,7 +146,11 @@ __device__ __forceinline__ void scatter_tap(float4* __restrict__ g, const Tap& t
 // =====================================================================================================
 // adv1 (src/sim.js:142-157): velX = mix(wind, vel(bt), fade), SX = S(bt) fade, S2X = S2(bt) fade with
 // bt = c - vel(mid) dt/dx, mid = c - vel(c) dt/(2 dx).
-__global__ void __launch_bounds__(256) k_adv1_adj(const float* __restrict__ P, TapeStep T, AdjFields a, Dims d) {
+// The three large kernels need 173 to 182 registers, which leaves an SM one CTA: eight warps against chains of dependent gathers.
+// Two CTAs (128 registers, some spilled) hide more.  Measured (GB300, 64x128x64, us, one CTA, two, three): k_forces_adj1 110, 85,
+// 85; k_adv2_adj 96, 70, 88; k_adv1_adj 74, 63, 79; a 10-step backward 8.30 ms, 7.68, 7.97.
+constexpr int ADJ_CTAS = 2;
+__global__ void __launch_bounds__(256, ADJ_CTAS) k_adv1_adj(const float* __restrict__ P, TapeStep T, AdjFields a, Dims d) {
   const ACell id = acell(d);
   if (!id.ok) return;
   const size_t ci = cell(id.i, id.j, id.k, d.nx, d.ny);
@@ -223,7 +227,7 @@ __device__ __forceinline__ LimCh limiter_adj(float lr, float x, float H, float m
 __device__ __forceinline__ float ch4(float4 v, int c) { return c == 0 ? v.x : c == 1 ? v.y : c == 2 ? v.z : v.w; }
 __device__ __forceinline__ void set4(float4& v, int c, float s) { if (c == 0) v.x = s; else if (c == 1) v.y = s; else if (c == 2) v.z = s; else v.w = s; }
 
-__global__ void __launch_bounds__(256) k_adv2_adj(const float* __restrict__ P, TapeStep T, AdjFields a, Dims d) {
+__global__ void __launch_bounds__(256, ADJ_CTAS) k_adv2_adj(const float* __restrict__ P, TapeStep T, AdjFields a, Dims d) {
   const ACell id = acell(d);
   if (!id.ok) return;
   const size_t ci = cell(id.i, id.j, id.k, d.nx, d.ny);
@@ -676,7 +680,7 @@ __device__ __forceinline__ float forces_adj_cell(const float* __restrict__ P, co
 // Pass 1 of the forces adjoint: per-cell reverse, then the spot-flux cotangents reduced per warp.  Consumes
 // the output cotangents (S, S2 are zeroed for the advection adjoints that accumulate into them next) and
 // clears the hat cotangents the advection adjoints accumulate into.
-__global__ void __launch_bounds__(256) k_forces_adj1(const float* __restrict__ P, TapeStep T, AdjFields a, const uint2* __restrict__ noiseT,
+__global__ void __launch_bounds__(256, ADJ_CTAS) k_forces_adj1(const float* __restrict__ P, TapeStep T, AdjFields a, const uint2* __restrict__ noiseT,
                                                      const uint2* __restrict__ curlT, Dims d, int consume) {
   const ACell id = acell(d);
   float lacc = 0.0f;
