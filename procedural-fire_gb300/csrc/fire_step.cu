@@ -228,6 +228,12 @@ __global__ void __launch_bounds__(256) k_curl(Fields f, Dims d) {
 // velY Laplacian (only evaluated when visc > 0).
 // The cell's own SY, S2Y and geometry values are passed in (the z-marching kernel prefetches them a plane
 // ahead).
+// Most cells of a domain are cold and burn nothing, and the kernel is bound by its instructions (870 a cell, 65 % of the issue
+// slots at 128x256x128).  Where a factor is exactly 0, what it multiplies is left out: combustion below the ignition window,
+// confinement and turbulence below 450 K without heat release, the age of gas that has none, the speed limit's root.  Only
+// the sign of a zero can differ.  Measured (GB300, us, everything evaluated -> this): 50x98x50 30.3 -> 28.9, 80x120x80 50.6
+// -> 50.1, 128x256x128 185 -> 184 (a fire that fills it), 256x512x256 1103 -> 990; gates on the soot oxidation and the cooling
+// cost more in a burning warp than they save (128x256x128 184 -> 192).
 // Readers of the per-step parameter block for the forces physics: from global memory (batched, eager and
 // adjoint launches), or from the kernel's own parameter space (the step graph's launch, whose block is set on
 // the instantiated graph before every step), where each read is a constant-bank operand instead of a load.
@@ -309,20 +315,29 @@ __device__ __forceinline__ void forces_cell(const PA& pa, const Fields& f, const
     s2.w *= 1.0f - bw;
     s2.y = fmaxf(s2.y, 0.05f * bw * clampf(s.y + s2.x, 0.0f, 1.0f));
   }
-  float ageF = s2.y / fmaxf(s.y + s2.x, 1e-4f);
+  float ageF = s2.y != 0.0f ? s2.y / fmaxf(s.y + s2.x, 1e-4f) : s2.y;
 
   // ---- mixing-limited combustion (src/sim.js:299-309)
   const float T0 = 293.0f + 1000.0f * s.x;
   const float o = clampf(1.0f - s.y - s2.x, 0.0f, 1.0f);
   const float ignT = pa[P_ignT], rs = pa[P_rs];
   const float ign = sstep_inv(ignT - 50.0f, pa[P_STRIDE + E_invIgn], T0);
-  const float b = fminf(s.y, o / rs) * (1.0f - expf(-pa[P_kMix] * ign * dt));
-  s.y -= b;
-  s2.x = fminf(s2.x + (1.0f + rs) * b, 1.0f);
-  const float dT = fminf(pa[P_heatOut] * b, fmaxf(2100.0f - T0, 0.0f));
-  float T = T0 + dT;
-  const float q = dT / dt;
-  const float phi = geo.z > 0.5f ? 0.0f : fminf(pa[P_expansion] * q / T, 60.0f);
+  const float kMix = pa[P_kMix], heatOut = pa[P_heatOut], expansion = pa[P_expansion];
+  auto finite = [](float x) { return fabsf(x) <= 3.4028235e38f; };
+  // without finite uniforms a product with an exact 0 need not be 0
+  const bool plain = finite(kMix) && finite(heatOut) && finite(expansion) && rs > 0.0f && dt > 0.0f && finite(dt);
+  float b = 0.0f, T = T0, q = 0.0f, phi = 0.0f;
+  if (plain && ign == 0.0f && T0 > 0.0f) {
+    s2.x = fminf(s2.x, 1.0f);
+  } else {
+    b = fminf(s.y, o / rs) * (1.0f - expf(-kMix * ign * dt));
+    s.y -= b;
+    s2.x = fminf(s2.x + (1.0f + rs) * b, 1.0f);
+    const float dT = fminf(heatOut * b, fmaxf(2100.0f - T0, 0.0f));
+    T = T0 + dT;
+    q = dT / dt;
+    phi = geo.z > 0.5f ? 0.0f : fminf(expansion * q / T, 60.0f);
+  }
 
   // ---- soot (src/sim.js:312-318); the age gate bounds come from the extension block
   const float sootOx = pa[P_sootOx];
@@ -354,28 +369,30 @@ __device__ __forceinline__ void forces_cell(const PA& pa, const Fields& f, const
     float nu = visc * 1.5e-5f * powf(fmaxf(T, 293.0f) / 293.0f, 1.7f);
     v = v + lapV * fminf(nu * dt / (dx * dx), 0.15f);
   }
-  // ---- laminar flame base (src/sim.js:350)
-  const float lamAge = pa[P_lamAge];
-  const float lam = lamAge > 0.0f ? sstep(0.5f * lamAge, fmaxf(lamAge, 1e-3f), ageF) : 1.0f;
+  // ---- laminar flame base (src/sim.js:350); both gates below are 0 in cold gas without heat release
+  if (T > 450.0f || s.w != 0.0f) {
+    const float lamAge = pa[P_lamAge];
+    const float lam = lamAge > 0.0f ? sstep(0.5f * lamAge, fmaxf(lamAge, 1e-3f), ageF) : 1.0f;
 
-  // ---- vorticity confinement (src/sim.js:353-361).  Where the gate is exactly 0 (gas below 450 K, the
-  // sources, the floor layer) the increment is a signed zero, so it is skipped; only the sign of a zero
-  // velocity component can differ.
-  const float gate = sstep(450.0f, 900.0f, T) * (1.0f - srcAll) * sstep(0.02f, 0.08f, p.y) * lam;
-  if (gate != 0.0f) {
-    const f3 g = nb.grad_w();
-    const float gl = len3(g);
-    if (gl > 1e-6f) v = v + cross3(g / gl, xyz(nb.vort_center())) * (pa[P_vortEps] * gate) * dt;
-  }
+    // ---- vorticity confinement (src/sim.js:353-361).  Where the gate is exactly 0 (gas below 450 K, the
+    // sources, the floor layer) the increment is a signed zero, so it is skipped; only the sign of a zero
+    // velocity component can differ.
+    const float gate = sstep(450.0f, 900.0f, T) * (1.0f - srcAll) * sstep(0.02f, 0.08f, p.y) * lam;
+    if (gate != 0.0f) {
+      const f3 g = nb.grad_w();
+      const float gl = len3(g);
+      if (gl > 1e-6f) v = v + cross3(g / gl, xyz(nb.vort_center())) * (pa[P_vortEps] * gate) * dt;
+    }
 
-  // ---- sub-grid turbulence: rising, evolving curl noise (src/sim.js:364-368); skipped the same way where
-  // its gate is exactly 0 (below 500 K with no heat release: most of the domain), which saves the table sample
-  const float tgate = fmaxf(sstep(500.0f, 1100.0f, T), sstep(0.0f, 3.0f, s.w)) * (1.0f - srcAll) *
-                      mixf(0.6f, 1.8f, sstep(0.2f, 0.75f, p.y)) * lam;
-  if (tgate != 0.0f) {
-    f3 tq = (p - mk3(0.0f, time * pa[P_turbRise], 0.0f)) * pa[P_turbFreq] + mk3(0.0f, 0.0f, time * pa[P_turbEvolve]);
-    f3 cn = xyz(sample_table(curlT, tq));
-    v = v + cn * pa[P_STRIDE + E_turbK] * tgate * dt * 10.0f;   // E_turbK = turbAmp / 12
+    // ---- sub-grid turbulence: rising, evolving curl noise (src/sim.js:364-368); skipped the same way where
+    // its gate is exactly 0 (below 500 K with no heat release: most of the domain), which saves the table sample
+    const float tgate = fmaxf(sstep(500.0f, 1100.0f, T), sstep(0.0f, 3.0f, s.w)) * (1.0f - srcAll) *
+                        mixf(0.6f, 1.8f, sstep(0.2f, 0.75f, p.y)) * lam;
+    if (tgate != 0.0f) {
+      f3 tq = (p - mk3(0.0f, time * pa[P_turbRise], 0.0f)) * pa[P_turbFreq] + mk3(0.0f, 0.0f, time * pa[P_turbEvolve]);
+      f3 cn = xyz(sample_table(curlT, tq));
+      v = v + cn * pa[P_STRIDE + E_turbK] * tgate * dt * 10.0f;   // E_turbK = turbAmp / 12
+    }
   }
 
   // ---- wind above the logs (src/sim.js:372-375)
@@ -401,8 +418,11 @@ __device__ __forceinline__ void forces_cell(const PA& pa, const Fields& f, const
   s.z *= kt;
   s2.z *= kt;
 
-  float vl = len3(v);
-  if (vl > 15.0f) v = v * (15.0f / vl);
+  const float vv = dot3(v, v);
+  if (vv > 224.0f) {   // sqrt(224) < 15
+    const float vl = sqrtf(vv);
+    if (vl > 15.0f) v = v * (15.0f / vl);
+  }
   bool bad = isnan(s.x) || isnan(s.y) || isnan(s.z) || isnan(s.w) || isnan(s2.x) || isnan(s2.y) || isnan(s2.z) ||
              isnan(s2.w) || isnan(v.x) || isnan(v.y) || isnan(v.z);
   if (bad) {
@@ -684,8 +704,11 @@ __device__ __forceinline__ void project_body(const float* __restrict__ P, const 
     f3 v = xyz(__ldg(velX + ci)) - g;
     if (__ldg(solid + ci)) v = mk3(0.0f, 0.0f, 0.0f);   // geo.b > 0.5
     if (j == 0) v.y = fmaxf(v.y, 0.0f);
-    float vl = len3(v);
-    if (vl > 20.0f || isnan(vl)) v = isnan(vl) ? mk3(0.0f, 0.0f, 0.0f) : v * 20.0f / vl;
+    const float vv = dot3(v, v);
+    if (!(vv <= 399.0f)) {   // sqrt(399) < 20
+      const float vl = sqrtf(vv);
+      if (vl > 20.0f || isnan(vl)) v = isnan(vl) ? mk3(0.0f, 0.0f, 0.0f) : v * 20.0f / vl;
+    }
     vel[ci] = make_float4(v.x, v.y, v.z, 0.0f);
     below = me;
     me = above;
