@@ -108,11 +108,11 @@ struct PState {
 };
 
 // Writes the CTA's (x, y, z, w) partial (df64 pairs (rr, bb)) into slot `slot`.
-__device__ __forceinline__ void cta_partial(float rrf, float bbf, float4* partials, int slot) {
+__device__ __forceinline__ void cta_partial(df64 rr, df64 bb, float4* partials, int slot) {
   __shared__ df64 sr[NT / 32], sb[NT / 32];
   const int tid = threadIdx.x + GX * (threadIdx.y + GY * threadIdx.z);
-  df64 rr = df_warp_sum(df_make(rrf));
-  df64 bb = df_warp_sum(df_make(bbf));
+  rr = df_warp_sum(rr);
+  bb = df_warp_sum(bb);
   if ((tid & 31) == 0) { sr[tid >> 5] = rr; sb[tid >> 5] = bb; }
   __syncthreads();
   if (tid < 32) {
@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(NT) k_sumsq(const float* __restrict__ b, long 
     const float v = __ldg(b + i);
     s += v * v;
   }
-  cta_partial(0.0f, s, partials, blockIdx.x);
+  cta_partial(df_make(0.0f), df_make(s), partials, blockIdx.x);
 }
 
 // Laplacian numerator of one cell written as a sum of neighbour differences, (nb - me) per face with the
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(NT) k_pres(const float* __restrict__ xh, const
       }
     }
   }
-  cta_partial(rr, bb, partials, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z));
+  cta_partial(df_make(rr), df_make(bb), partials, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z));
 }
 
 // k_pres for even nx with one thread per x pair (2 gx, 2 gx + 1) and RZ planes: every load of xh, xl and b
@@ -249,7 +249,74 @@ __global__ void __launch_bounds__(NT) k_pres2(const float* __restrict__ xh, cons
       }
     }
   }
-  cta_partial(rr, bb, partials, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z));
+  cta_partial(df_make(rr), df_make(bb), partials, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z));
+}
+
+// k_pres2 with four cells of a row per thread, for rows that fill whole warps of them: one 16-byte load where the pair form has two
+// 8-byte ones, and the x neighbours of the four come from the neighbouring lanes, so a cell costs three quarters of the L1
+// traffic and two thirds of the instructions.  Same arithmetic and order within a cell; the partials' cells are grouped differently.
+// Measured (GB300, whole solves, pairs -> this): 256x512x256 with FP32 storage 4.99 -> 4.83 ms, 128x256x128 with half 1.043 -> 1.030.
+template <typename TR>
+__global__ void __launch_bounds__(NT) k_pres4(const float* __restrict__ xh, const float* __restrict__ xl, const float* __restrict__ b,
+                                              TR* __restrict__ rT, const PState* __restrict__ ps, int nx, int ny, int nz, float ih2,
+                                              float4* __restrict__ partials) {
+  pdl_wait();
+  pdl_trigger();
+  const int gx = blockIdx.x * GX + threadIdx.x, y = blockIdx.y * GY + threadIdx.y;
+  const int z0 = (blockIdx.z * GZ + threadIdx.z) * RZ;
+  float rr = 0.0f, rr2 = 0.0f, bb = 0.0f, bb2 = 0.0f;   // as many cells in each FP32 sum as the pair form
+  if (y < ny && z0 < nz) {   // uniform over a warp: its 32 lanes share y and z
+    const float s = rT ? ps->sc[1] : 1.0f;
+    const int sy = nx, sz = nx * ny;
+    const bool hxm = gx > 0, hxp = gx < (nx >> 2) - 1, hym = y > 0, hyp = y < ny - 1;
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    auto ld4 = [](const float* q) { return __ldg(reinterpret_cast<const float4*>(q)); };
+    int t = 4 * gx + sy * y + sz * z0;
+    float4 hp = z0 > 0 ? ld4(xh + t - sz) : zero, hc = ld4(xh + t), lp = zero, lc = zero;
+    if (xl) { lp = z0 > 0 ? ld4(xl + t - sz) : zero; lc = ld4(xl + t); }
+    const int lane = threadIdx.x;
+    auto sides = [&](const float* q, float4 c, float& l, float& r) {
+      l = __shfl_up_sync(0xffffffffu, c.w, 1);
+      r = __shfl_down_sync(0xffffffffu, c.x, 1);
+      if (lane == 0) l = hxm ? __ldg(q + t - 1) : 0.0f;
+      if (lane == 31) r = hxp ? __ldg(q + t + 4) : 0.0f;
+    };
+    auto laps = [&](float4 c, float l, float r, float4 ym, float4 yp, float4 zm, float4 zp, bool hzm, bool hzp) {
+      return make_float4(lap_diff(c.x, l, c.y, ym.x, yp.x, zm.x, zp.x, hxm, true, hym, hyp, hzm, hzp),
+                         lap_diff(c.y, c.x, c.z, ym.y, yp.y, zm.y, zp.y, true, true, hym, hyp, hzm, hzp),
+                         lap_diff(c.z, c.y, c.w, ym.z, yp.z, zm.z, zp.z, true, true, hym, hyp, hzm, hzp),
+                         lap_diff(c.w, c.z, r, ym.w, yp.w, zm.w, zp.w, true, hxp, hym, hyp, hzm, hzp));
+    };
+#pragma unroll
+    for (int k = 0; k < RZ; ++k) {
+      const int z = z0 + k;
+      if (z >= nz) break;
+      const bool hzm = z > 0, hzp = z + 1 < nz;
+      const float4 hn = hzp ? ld4(xh + t + sz) : zero, ln = xl && hzp ? ld4(xl + t + sz) : zero, bv = ld4(b + t);
+      const float4 hym4 = hym ? ld4(xh + t - sy) : zero, hyp4 = hyp ? ld4(xh + t + sy) : zero;
+      float l, r;
+      sides(xh, hc, l, r);
+      const float4 d = laps(hc, l, r, hym4, hyp4, hp, hn, hzm, hzp);
+      float4 dl = zero;
+      if (xl) {
+        const float4 lym = hym ? ld4(xl + t - sy) : zero, lyp = hyp ? ld4(xl + t + sy) : zero;
+        sides(xl, lc, l, r);
+        dl = laps(lc, l, r, lym, lyp, lp, ln, hzm, hzp);
+      }
+      const float4 res = make_float4((bv.x - d.x * ih2) - dl.x * ih2, (bv.y - d.y * ih2) - dl.y * ih2, (bv.z - d.z * ih2) - dl.z * ih2,
+                                     (bv.w - d.w * ih2) - dl.w * ih2);
+      if (rT) {
+        st2<true>(rT + t, make_float2(res.x * s, res.y * s));
+        st2<true>(rT + t + 2, make_float2(res.z * s, res.w * s));
+      }
+      rr += res.x * res.x; rr += res.y * res.y; rr2 += res.z * res.z; rr2 += res.w * res.w;
+      bb += bv.x * bv.x; bb += bv.y * bv.y; bb2 += bv.z * bv.z; bb2 += bv.w * bv.w;
+      hp = hc; hc = hn;
+      lp = lc; lc = ln;
+      t += sz;
+    }
+  }
+  cta_partial(df_add(df_make(rr), df_make(rr2)), df_add(df_make(bb), df_make(bb2)), partials, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z));
 }
 
 // (xh, xl) += e * sc[0] as a double-float (FP32 pair) update: Knuth's TwoSum then renormalisation, so the
@@ -335,7 +402,7 @@ __global__ void __launch_bounds__(NT) k_rhs(float* __restrict__ b, int nx, int n
     v += noise * sqrtf(-2.0f * logf(u1)) * cosf(6.283185307179586f * u2);
     b[x + nx * (y + ny * z)] = v;
   }
-  cta_partial(0.0f, v, partials, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z));
+  cta_partial(df_make(0.0f), df_make(v), partials, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z));
 }
 __global__ void __launch_bounds__(NT) k_mean(const float4* __restrict__ partials, int count, double ncells, double* __restrict__ mean) {
   __shared__ df64 sa[SUMV / 32], sb[SUMV / 32];
@@ -462,9 +529,11 @@ void pprolong(const PLevel& F, void* p, const PLevel& C, cudaStream_t st) {
   });
 }
 
-// The residual kernel's grid: x pairs for even nx (k_pres2), single cells otherwise (k_pres).
+// The residual kernel's grid: four cells a thread where rows are whole warps of them (k_pres4), x pairs for even nx (k_pres2), single
+// cells otherwise (k_pres).
+bool pres_four(const PLevel& L) { return L.nx % (4 * GX) == 0; }
 dim3 pres_grid(const PLevel& L) {
-  const int cols = (L.nx % 2 == 0) ? L.nx / 2 : L.nx;
+  const int cols = pres_four(L) ? L.nx / 4 : (L.nx % 2 == 0) ? L.nx / 2 : L.nx;
   return dim3((cols + GX - 1) / GX, (L.ny + GY - 1) / GY, (L.nz + GZ * RZ - 1) / (GZ * RZ));
 }
 
@@ -473,7 +542,7 @@ void pres(FirePoisson* ps, const PState* state, const float* b, const float* xh,
   const PLevel& L = ps->levels[0];
   with_type(write ? L.sto : STO_F32, [&](auto t) {
     using TR = decltype(t);
-    auto kernel = L.nx % 2 ? k_pres<TR> : L.nz % (GZ * RZ) ? k_pres2<TR, false> : k_pres2<TR, true>;
+    auto kernel = pres_four(L) ? k_pres4<TR> : L.nx % 2 ? k_pres<TR> : L.nz % (GZ * RZ) ? k_pres2<TR, false> : k_pres2<TR, true>;
     launch_pdl(kernel, pres_grid(L), kBlock, 0, st, xh, xl, b, write ? (TR*)L.b : (TR*)nullptr, state, L.nx, L.ny, L.nz, 1.0f / (L.h * L.h),
                ps->partials);
   });

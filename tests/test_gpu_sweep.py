@@ -92,3 +92,25 @@ def test_batched_sweeps_match_members_alone():
         np.testing.assert_array_equal(a.level(0, "p"), b.level(0, "p"))
         b.close()
     ens.close()
+
+
+@pytest.mark.parametrize("res", [(128, 42, 30), (256, 20, 17), (128, 7, 5)])
+def test_refinement_residual_on_whole_warp_rows(res):
+    """The residual of a pair (x, x_lo) with four cells a thread (rows of a multiple of 128 cells; rows and planes that leave ragged
+    CTAs, fewer planes than one thread marches) against its FP64 form.  A residual is a sum of 14 rounded terms of at most
+    |b| + 12 max|x| / h^2 and the norm adds about as much again, so 64 x 2^-24 of that size over the norm bounds the error."""
+    torch = pytest.importorskip("torch")
+    import fire_sim as F
+    import oracle as O
+    n = (res[2], res[1], res[0])
+    rng = np.random.default_rng(res[0] + res[1])
+    b, x = (rng.standard_normal(n).astype(np.float32) for _ in range(2))
+    lo = (1e-8 * rng.standard_normal(n)).astype(np.float32)
+    h = 0.5
+    ps = F.Poisson(res, h, "ir32")
+    got = ps.residual(*(torch.from_numpy(v).cuda() for v in (b, x, lo)))
+    r = b.astype(np.float64) - O.pressure_apply(x.astype(np.float64) + lo, h)
+    want = np.linalg.norm(r) / np.linalg.norm(b)
+    size = np.sqrt(r.size) * (np.abs(b).max() + 12 * np.abs(x).max() / h ** 2) / np.linalg.norm(b)
+    assert abs(got - want) <= 64 * 2.0 ** -24 * size
+    ps.close()
