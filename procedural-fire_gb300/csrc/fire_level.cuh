@@ -6,8 +6,8 @@
 // thread that needs it (10 pair or side loads per coarse cell and plane pair where a gather per child takes 64), and what two
 // coarse planes share stays in registers.
 // Measured (GB300, back to back, us, gather per coarse cell -> this; restriction, prolongation): 64x128x64 3.0 -> 1.8,
-// 3.2 -> 2.5; 80x120x80 4.5 -> 2.3, 5.2 -> 4.5; 128x256x128 10.1 -> 5.4, 8.9 -> 8.0; 256x512x256 101 -> 63, 72 -> 54 (4.5 and
-// 5.3 TB/s).
+// 3.2 -> 2.5; 80x120x80 4.5 -> 2.3, 5.2 -> 4.5; 128x256x128 10.1 -> 5.4, 8.9 -> 8.0; 256x512x256 101 -> 56, 72 -> 53 (5.0 and
+// 5.4 TB/s).
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -202,7 +202,9 @@ __device__ __forceinline__ void prolong_march(TF* __restrict__ p, const TC* __re
   }
 }
 
-// Coarse planes a thread marches: four where that still leaves each of the 152 SMs eight CTAs, else one.
+// Coarse planes a thread marches: the prolongation four where that still leaves each of the 152 SMs eight CTAs, else one
+// (256x512x256: 63 us with one, 55 with two, 53 with four, 57 with eight); the restriction one (56, 56, 62, 65: the compiler
+// spreads a longer march's loads out); in a batch both four, since a CTA first has to find its simulation.
 constexpr int TRANSFER_DEPTH = 4;
 constexpr long TRANSFER_DEEP_CELLS = 152L * 8 * LX * LY * LZ * TRANSFER_DEPTH;
 inline dim3 transfer_grid(int cnx, int cny, int cnz, int depth) {

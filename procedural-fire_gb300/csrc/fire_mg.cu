@@ -159,10 +159,10 @@ __global__ void __launch_bounds__(GX * GY * GZ) k_smooth1(float* __restrict__ p,
   if (omega == 1.0f) smooth_body_t<false, false, 1>(p, b, nx, ny, nz, h, color, blockIdx, omega);
   else smooth_body_t<true, false, 1>(p, b, nx, ny, nz, h, color, blockIdx, omega);
 }
-template <int kDepth, bool kPair>
+template <bool kPair>
 __global__ void __launch_bounds__(LX * LY * LZ) k_restrict(const float* __restrict__ p, const float* __restrict__ b, int nx, int ny, int nz,
                                                            float h, float* __restrict__ bc, float* __restrict__ pc) {
-  restrict_march<kDepth, kPair>(p, b, nx, ny, nz, h, bc, pc, blockIdx);
+  restrict_march<1, kPair>(p, b, nx, ny, nz, h, bc, pc, blockIdx);
 }
 template <int kDepth, bool kPair, bool kClamp>
 __global__ void __launch_bounds__(LX * LY * LZ) k_prolong(float* __restrict__ p, const float* __restrict__ pc, int nx, int ny, int nz) {
@@ -998,10 +998,8 @@ cudaError_t launch_smooth(const MGLevel& L, int color, cudaStream_t st) {
 static bool pair_aligned(const void* p, const void* b) { return ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(b)) & 7u) == 0; }
 static bool transfer_deep(const MGLevel& C) { return (long)C.nx * C.ny * C.nz >= TRANSFER_DEEP_CELLS; }
 cudaError_t launch_restrict(const MGLevel& F, const MGLevel& C, cudaStream_t st, bool clear) {
-  const bool deep = transfer_deep(C), pairs = pair_aligned(F.p, F.b);
-  return launch_pdl(!pairs ? k_restrict<1, false> : deep ? k_restrict<TRANSFER_DEPTH, true> : k_restrict<1, true>,
-                    transfer_grid(C.nx, C.ny, C.nz, pairs && deep ? TRANSFER_DEPTH : 1), kBlock, 0, st, (const float*)F.p, (const float*)F.b, F.nx,
-                    F.ny, F.nz, F.h, C.b, clear ? C.p : (float*)nullptr);
+  return launch_pdl(pair_aligned(F.p, F.b) ? k_restrict<true> : k_restrict<false>, transfer_grid(C.nx, C.ny, C.nz, 1), kBlock, 0, st, (const float*)F.p,
+                    (const float*)F.b, F.nx, F.ny, F.nz, F.h, C.b, clear ? C.p : (float*)nullptr);
 }
 cudaError_t launch_prolong(const MGLevel& F, const MGLevel& C, cudaStream_t st) {
   const bool deep = transfer_deep(C), pairs = pair_aligned(F.p, nullptr);

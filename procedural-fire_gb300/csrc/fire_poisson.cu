@@ -87,10 +87,10 @@ __global__ void __launch_bounds__(NT) k_psmooth(T* __restrict__ p, const T* __re
   }
 }
 // The transfers between levels of any two storage types (fire_level.cuh).
-template <int kDepth, typename TF, typename TC>
+template <typename TF, typename TC>
 __global__ void __launch_bounds__(NT) k_prestrict(const TF* __restrict__ p, const TF* __restrict__ b, int nx, int ny, int nz, float h,
                                                   TC* __restrict__ bc, TC* __restrict__ pc) {
-  restrict_march<kDepth, true>(p, b, nx, ny, nz, h, bc, pc, blockIdx);
+  restrict_march<1, true>(p, b, nx, ny, nz, h, bc, pc, blockIdx);
 }
 template <int kDepth, typename TF, typename TC>
 __global__ void __launch_bounds__(NT) k_pprolong(TF* __restrict__ p, const TC* __restrict__ pc, int nx, int ny, int nz) {
@@ -512,9 +512,8 @@ void prestrict(const PLevel& F, const void* p, const PLevel& C, bool clear, cuda
     with_type(C.sto, [&](auto c) {
       using TF = decltype(f);
       using TC = decltype(c);
-      launch_pdl(deep(C) ? k_prestrict<TRANSFER_DEPTH, TF, TC> : k_prestrict<1, TF, TC>,
-                 transfer_grid(C.nx, C.ny, C.nz, deep(C) ? TRANSFER_DEPTH : 1), kBlock, 0, st, (const TF*)p, (const TF*)F.b, F.nx, F.ny, F.nz,
-                 F.h, (TC*)C.b, clear ? (TC*)C.p : (TC*)nullptr);
+      launch_pdl(k_prestrict<TF, TC>, transfer_grid(C.nx, C.ny, C.nz, 1), kBlock, 0, st, (const TF*)p, (const TF*)F.b, F.nx, F.ny, F.nz, F.h,
+                 (TC*)C.b, clear ? (TC*)C.p : (TC*)nullptr);
     });
   });
 }
