@@ -890,21 +890,65 @@ __device__ __forceinline__ void residual_column(const float* __restrict__ p, con
     }
   }
 }
+// The same for the pair of columns x, x + 1 (even x and nx): pairs move as one load and each column keeps its own sums, so a
+// column's FP32 sums are residual_column's.
+__device__ __forceinline__ void residual_pair(const float* __restrict__ p, const float* __restrict__ b, int x, int y, int z0, int nx, int ny,
+                                              int nz, float ih2, float2& rr, float2& bb) {
+  const int sy = nx, sz = nx * ny;
+  const bool hxm = x > 0, hxp = x < nx - 2, hym = y > 0, hyp = y < ny - 1;
+  auto ld = [](const float* q) { return __ldg(reinterpret_cast<const float2*>(q)); };
+  const float2 none = make_float2(0.0f, 0.0f);
+  int t = x + sy * y + sz * z0;
+  float2 prev = z0 > 0 ? ld(p + t - sz) : none, cur = ld(p + t);
+#pragma unroll
+  for (int k = 0; k < RZ; ++k) {
+    const int z = z0 + k;
+    if (z < nz) {
+      const bool hzp = z + 1 < nz;
+      const float2 next = hzp ? ld(p + t + sz) : none, me = cur;
+      const float left = hxm ? __ldg(p + t - 1) : -me.x, right = hxp ? __ldg(p + t + 2) : -me.y;
+      const float2 ym = hym ? ld(p + t - sy) : me, yp = hyp ? ld(p + t + sy) : make_float2(-me.x, -me.y);
+      const float2 zm = z > 0 ? prev : make_float2(-me.x, -me.y), zp = hzp ? next : make_float2(-me.x, -me.y);
+      const float2 bv = ld(b + t);
+      const float lx = (left + me.y + ym.x + yp.x + zm.x + zp.x - 6.0f * me.x) * ih2;
+      const float ly = (me.x + right + ym.y + yp.y + zm.y + zp.y - 6.0f * me.y) * ih2;
+      const float rx = bv.x - lx, ry = bv.y - ly;
+      rr.x += rx * rx;
+      rr.y += ry * ry;
+      bb.x += bv.x * bv.x;
+      bb.y += bv.y * bv.y;
+      prev = cur;
+      cur = next;
+      t += sz;
+    }
+  }
+}
 // gate (residual-driven loop only, else null): the loop's counters; the norm is skipped while the cycle
 // about to complete (gate[0] + 1) is below the first cycle at which this step tests convergence (gate[3]).
+// kPair: a thread takes two columns (even nx): half the loads and CTAs.  Measured (GB300, norm and sum, us, single columns -> pairs):
+// 64x128x64 7.3 -> 6.8, 80x120x80 7.7 -> 7.6, 128x256x128 15.8 -> 12.6, 256x512x256 117 -> 80.
+template <bool kPair>
 __global__ void __launch_bounds__(RB) k_residual(const float* __restrict__ p, const float* __restrict__ b, int nx, int ny, int nz,
                                                  float ih2, float4* __restrict__ partials, const int* __restrict__ gate) {
   __shared__ df64 sr[RB / 32], sb[RB / 32];
   pdl_wait();
   pdl_trigger();
   if (gate && gate[0] + 1 < mg_first_test(gate[3])) return;   // uniform over the grid
-  const int x = blockIdx.x * GX + threadIdx.x, y = blockIdx.y * GY + threadIdx.y;
+  const int x = (blockIdx.x * GX + threadIdx.x) * (kPair ? 2 : 1), y = blockIdx.y * GY + threadIdx.y;
   const int z0 = (blockIdx.z * GZ + threadIdx.z) * RZ;
   const int tid = threadIdx.x + GX * (threadIdx.y + GY * threadIdx.z);
-  float rrf = 0.0f, bbf = 0.0f;   // this thread's RZ cells in FP32, widened to df64 once below
-  if (x < nx && y < ny && z0 < nz) residual_column(p, b, x, y, z0, nx, ny, nz, ih2, rrf, bbf);
-  df64 rr = df_warp_sum(df_make(rrf));
-  df64 bb = df_warp_sum(df_make(bbf));
+  float2 rrf = make_float2(0.0f, 0.0f), bbf = rrf;   // RZ cells of a column in FP32, widened to df64 once below
+  if (x < nx && y < ny && z0 < nz) {
+    if (kPair) residual_pair(p, b, x, y, z0, nx, ny, nz, ih2, rrf, bbf);
+    else residual_column(p, b, x, y, z0, nx, ny, nz, ih2, rrf.x, bbf.x);
+  }
+  df64 rr = df_make(rrf.x), bb = df_make(bbf.x);
+  if (kPair) {
+    rr = df_add(rr, df_make(rrf.y));
+    bb = df_add(bb, df_make(bbf.y));
+  }
+  rr = df_warp_sum(rr);
+  bb = df_warp_sum(bb);
   if ((tid & 31) == 0) { sr[tid >> 5] = rr; sb[tid >> 5] = bb; }
   __syncthreads();
   if (tid < 32) {
@@ -1173,21 +1217,21 @@ void launch_tail_batch(int kind, const void* dev_descs, int count, size_t smem, 
   cfg.numAttrs = 2;
   cudaLaunchKernelEx(&cfg, k_ctail_b, (const CTailLevels*)dev_descs, pre, post);
 }
-static dim3 residual_grid(const MGLevel& L) { return grid3(L.nx, L.ny, (L.nz + RZ - 1) / RZ); }
+static dim3 residual_grid(const MGLevel& L) { return grid3(L.nx % 2 ? L.nx : L.nx / 2, L.ny, (L.nz + RZ - 1) / RZ); }
 int residual_partials_count(const MGLevel& L) {
   dim3 g = residual_grid(L);
   return (int)(g.x * g.y * g.z);
 }
 void launch_residual(const MGLevel& L, double* partials, double* out2, cudaStream_t st) {
   float4* part4 = reinterpret_cast<float4*>(partials);   // 16 bytes per CTA (the buffer holds 128 per CTA)
-  launch_pdl(k_residual, residual_grid(L), kBlock, 0, st, (const float*)L.p, (const float*)L.b, L.nx, L.ny, L.nz,
+  launch_pdl(L.nx % 2 ? k_residual<false> : k_residual<true>, residual_grid(L), kBlock, 0, st, (const float*)L.p, (const float*)L.b, L.nx, L.ny, L.nz,
              1.0f / (L.h * L.h), part4, (const int*)nullptr);
   launch_pdl(k_sum_pairs, dim3(1), dim3(RB), 0, st, (const float4*)part4, residual_partials_count(L), out2);
 }
 void launch_residual_decide(const MGLevel& L, double* partials, double* sums2, double tol, int max_cycles, int* counter,
                             double* rel_out, cudaGraphConditionalHandle h, cudaStream_t st) {
   float4* part4 = reinterpret_cast<float4*>(partials);
-  launch_pdl(k_residual, residual_grid(L), kBlock, 0, st, (const float*)L.p, (const float*)L.b, L.nx, L.ny, L.nz,
+  launch_pdl(L.nx % 2 ? k_residual<false> : k_residual<true>, residual_grid(L), kBlock, 0, st, (const float*)L.p, (const float*)L.b, L.nx, L.ny, L.nz,
              1.0f / (L.h * L.h), part4, (const int*)counter);
   launch_pdl(k_sum_decide, dim3(1), dim3(RB), 0, st, (const float4*)part4, residual_partials_count(L), sums2, tol, max_cycles,
              counter, rel_out, h);

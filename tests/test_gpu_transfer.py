@@ -62,3 +62,23 @@ def test_four_byte_aligned_level():
         assert rc == 0
         got.append(p[shift:shift + n].cpu().numpy())
     np.testing.assert_array_equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("res", [(10, 9, 7), (66, 50, 41), (25, 30, 27)])
+def test_residual_norm_matches_float64(res):
+    """The residual's norm with two columns a thread (even rows; ragged ends in every direction) and with one (odd rows).  A residual
+    is 9 rounded terms of at most s = max|b| + 12 max|p| / h^2 and each square and column sum of 8 adds 9 roundings, so
+    32 u s sqrt(cells) / ||b|| bounds the relative norm's error."""
+    nx, ny, nz = res
+    rng = np.random.default_rng(ny)
+    sim = F.FireSim(res=res, size=tuple(0.5 * r for r in res))
+    p, b = (rng.standard_normal((nz, ny, nx)).astype(np.float32) for _ in range(2))
+    h = float(np.float32(sim.levels[0]["h"]))
+    sim.set_level(0, "p", p)
+    sim.set_level(0, "b", b)
+    q = [v.astype(np.float64) for v in NF.neighbours(p.astype(np.float64))]
+    r = b - (sum(q) - 6.0 * p.astype(np.float64)) / h ** 2
+    norm = np.linalg.norm(b.astype(np.float64))
+    s = np.abs(b).max() + 12 * np.abs(p).max() / h ** 2
+    assert abs(sim.residual() - np.linalg.norm(r) / norm) <= 32 * U * s * np.sqrt(b.size) / norm
+    sim.close()
