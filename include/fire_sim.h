@@ -327,7 +327,7 @@ int fire_ensemble_step(FireEnsemble* e, float dt, int n_steps, void* stream);
 int fire_ensemble_sync(FireEnsemble* e);
 const char* fire_ensemble_last_error(FireEnsemble* e);
 /* Tile candidates of the batched stages (adv1, adv2, forces, div, project): cell tiles 0-3 (32x4x2, 32x8x1,
- * 32x2x4, 64x4x1 threads) for the per-cell stages, z-march depths 0-2 (16, 8, 32 planes) for forces.
+ * 32x2x4, 64x4x1 threads), for forces the first three.
  * fire_ensemble_tiles reports the chosen ones (FIRE_ERR_STATE before the tuning step) and, if ms is not
  * NULL, the measured mean launch time of each candidate (5 x 4 floats, ms; unused entries 0).          */
 #define FIRE_ENSEMBLE_STAGES 5

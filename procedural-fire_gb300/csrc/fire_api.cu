@@ -492,7 +492,6 @@ int fire_sim_create(const FireConfig* cfg, const float* logs, int n_logs, FireSi
       cudaEventCreateWithFlags(&sim->joinEv, cudaEventDisableTiming) != cudaSuccess)
     return fail(FIRE_ERR_CUDA);
   if (mg_configure(TAIL_SMEM_BUDGET) != cudaSuccess || coarse_configure() != cudaSuccess || sweep_configure() != cudaSuccess) return fail(set_err(sim, FIRE_ERR_CUDA, "tail kernel smem opt-in failed"));
-  if (step_configure() != cudaSuccess) return fail(set_err(sim, FIRE_ERR_CUDA, "forces kernel smem opt-in failed"));
 
   // zero state (reset semantics), bake the tables (src/noise.js), upload logs
   cudaStream_t st = sim->capStream;
@@ -1167,7 +1166,7 @@ int ens_top(const FireSim* s) {
 // and the multigrid's per-level maps and level tables.
 struct EnsCtx {
   StepBatch SB;
-  BatchMap adv1[CELL_TILES], cell[CELL_TILES], flow[CELL_TILES], forces[FORCES_TILES];   // adv1; adv2; div and project; forces
+  BatchMap adv1[CELL_TILES], cell[CELL_TILES], flow[CELL_TILES];   // adv1; adv2 and forces; div and project
   int adv1Depth = 1, flowDepth = 1;
   int depth = 0;
   std::vector<BatchMap> sweepMap, smoothMap, coarseMap;   // two-sweep tiles; colour launches (levels without a plan); transfers
@@ -1179,7 +1178,6 @@ void ens_context(FireEnsemble* e, EnsCtx& c) {
   for (auto& m : c.adv1) m = map_empty();
   for (auto& m : c.cell) m = map_empty();
   for (auto& m : c.flow) m = map_empty();
-  for (auto& m : c.forces) m = map_empty();
   c.depth = 0;
   double cells = 0.0;
   for (const FireSim* s : e->sims) cells += (double)s->d.nx * s->d.ny * s->d.nz;
@@ -1193,7 +1191,6 @@ void ens_context(FireEnsemble* e, EnsCtx& c) {
       map_add(c.cell[v], i, step_grid(s->d, v));
       map_add(c.flow[v], i, step_grid(s->d, v, c.flowDepth));
     }
-    for (int v = 0; v < FORCES_TILES; ++v) map_add(c.forces[v], i, forces_grid(s->d, v));
     c.depth = std::max(c.depth, ens_top(s));
   }
   // per level: the members that have it outside their tail, and every member's level l and l + 1
@@ -1225,7 +1222,7 @@ void ens_stage(FireEnsemble* e, const EnsCtx& c, int stage, int tile, cudaStream
   switch (stage) {
     case 0: launch_adv1_batch(c.adv1[tile], c.SB, tile, c.adv1Depth, st); break;
     case 1: launch_adv2_batch(c.cell[tile], c.SB, tile, st); break;
-    case 2: launch_forces_batch(c.forces[tile], c.SB, e->sims[0]->noise, e->sims[0]->curl, tile, st); break;
+    case 2: launch_forces_batch(c.cell[tile], c.SB, e->sims[0]->noise, e->sims[0]->curl, tile, st); break;
     case 3: launch_div_batch(c.flow[tile], c.SB, tile, c.flowDepth, st); break;
     default: launch_project_batch(c.flow[tile], c.SB, tile, c.flowDepth, st); break;
   }

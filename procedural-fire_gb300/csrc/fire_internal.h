@@ -128,23 +128,18 @@ struct ParamBlock { float v[BLOCK_FLOATS]; };
 void launch_forces_pb(const ParamBlock& pb, Fields f, const uint2* noise, const uint2* curl, Dims d, cudaStream_t st);
 cudaError_t forces_pb_set(cudaGraphExec_t exec, cudaGraphNode_t node, const ParamBlock& pb, Fields f, const uint2* noise,
                           const uint2* curl, Dims d);
-void launch_forces_unfused(const float* P, Fields f, const uint2* noise, const uint2* curl, Dims d, cudaStream_t st);
-void launch_forces_recompute(const float* P, Fields f, const uint2* noise, const uint2* curl, Dims d, cudaStream_t st);
-// Opts the shared-memory kernels of fire_step.cu into their dynamic shared memory on the current device.
-cudaError_t step_configure();
 void launch_div(const float* P, Fields f, float* b0, Dims d, cudaStream_t st, int* mg_counter = nullptr);
 void launch_project(const float* P, Fields f, const float* p0, Dims d, cudaStream_t st);
 // Tile candidates of the batched stages: CELL_TILES cell tiles for adv1, adv2, div and project (0 is the
-// per-simulation kernels' 32x4x2; then 32x8x1, 32x2x4, 64x4x1) and FORCES_TILES z-march depths of the forces
-// tile (16, 8, 32).  Every candidate computes the same per-cell arithmetic.
+// per-simulation kernels' 32x4x2; then 32x8x1, 32x2x4, 64x4x1), the first FORCES_TILES of them for forces.  Every candidate
+// computes the same per-cell arithmetic.
 constexpr int CELL_TILES = 4, FORCES_TILES = 3;
-// Block grids of the per-cell stages (adv1, adv2, div, project) and of the tiled forces stage, per candidate.
+// Block grids of the stages, per candidate.
 dim3 step_grid(Dims d, int tile = 0, int depth = 1);
 // Cells a thread of adv1, or of div and project, takes along z: for a grid (or a batch) of so many cells.
 constexpr int ADV1_DEPTH = 2, FLOW_DEPTH = 4;
 int adv1_depth(long cells);
 int flow_depth(long cells);
-dim3 forces_grid(Dims d, int tile = 0);
 void launch_adv1_batch(const BatchMap& m, const StepBatch& I, int tile, int depth, cudaStream_t st);
 void launch_adv2_batch(const BatchMap& m, const StepBatch& I, int tile, cudaStream_t st);
 void launch_forces_batch(const BatchMap& m, const StepBatch& I, const uint2* noise, const uint2* curl, int tile, cudaStream_t st);

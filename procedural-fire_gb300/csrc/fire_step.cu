@@ -1,8 +1,7 @@
 // Per-step stencil kernels of the fire simulation: MacCormack advection, curl + forces (fused),
 // divergence and projection.  Each kernel restates one WGSL compute shader of src/sim.js; the line
 // ranges are given per kernel.  One thread per cell; CTAs cover 32 x 4 x 2 bricks so the gathers of
-// the semi-Lagrangian back-trace and the 7-point stencils hit L1 (the forces stage instead marches 32 x 8
-// column tiles up z, one wave of resident CTAs).  Fields are dense float4 arrays, x fastest, so every warp
+// the semi-Lagrangian back-trace and the 7-point stencils hit L1.  Fields are dense float4 arrays, x fastest, so every warp
 // reads and writes 512 contiguous bytes per field.
 #include <type_traits>
 #include "fire_device.cuh"
@@ -222,18 +221,16 @@ __global__ void __launch_bounds__(256) k_curl(Fields f, Dims d) {
 // ---------------- forces (src/sim.js:214-396), with the curl recomputed in place ----------------
 // The reference runs a separate curl dispatch into a vorticity texture and reads 7 taps of it here.
 // This kernel computes those 7 vorticity values from velY directly (the taps are clamped to the
-// domain exactly as `ld` clamps them), so the vorticity field never round-trips through HBM.
-// Per-cell physics of the forces kernel.  `nb` supplies the velY/vorticity neighbourhood: the centre
-// velY value, the centre vorticity, the gradient of |w| from the 6 clamped vorticity taps, and the
-// velY Laplacian (only evaluated when visc > 0).
-// The cell's own SY, S2Y and geometry values are passed in (the z-marching kernel prefetches them a plane
-// ahead).
-// Most cells of a domain are cold and burn nothing, and the kernel is bound by its instructions (870 a cell, 65 % of the issue
-// slots at 128x256x128).  Where a factor is exactly 0, what it multiplies is left out: combustion below the ignition window,
-// confinement and turbulence below 450 K without heat release, the age of gas that has none, the speed limit's root.  Only
-// the sign of a zero can differ.  Measured (GB300, us, everything evaluated -> this): 50x98x50 30.3 -> 28.9, 80x120x80 50.6
-// -> 50.1, 128x256x128 185 -> 184 (a fire that fills it), 256x512x256 1103 -> 990; gates on the soot oxidation and the cooling
-// cost more in a burning warp than they save (128x256x128 184 -> 192).
+// domain exactly as `ld` clamps them), and only in the cells whose confinement gate is open.
+// Most cells of a domain are cold and burn nothing, and the kernel is bound by its instructions.  Where a factor is exactly 0,
+// what it multiplies is left out: combustion below the ignition window, confinement and turbulence below 450 K without heat
+// release, the age of gas that has none, the speed limit's root.  Only the sign of a zero can differ.  (Gates on the soot
+// oxidation and the cooling cost more in a burning warp than they save.)
+// A column march through shared memory, which formed every cell's vorticity once (870 instructions a cell, 65 % of the issue slots),
+// lost to this as soon as the gates were there.  Measured (GB300, us, march without gates, with, this): 50x98x50 30.3, 28.9,
+// 21.2; 80x120x80 50.6, 50.1, 39.3; 96x192x96 91.8, 90.8, 60.3; 128x256x128 185, 184, 103; 256x512x256 1103, 990, 621.  Where hot
+// cells are strewn over the whole domain (82 % of 128x256x128 at random) it is 222 against 209.
+// Per-cell physics.  The cell's own SY, S2Y and geometry values are passed in.
 // Readers of the per-step parameter block for the forces physics: from global memory (batched, eager and
 // adjoint launches), or from the kernel's own parameter space (the step graph's launch, whose block is set on
 // the instantiated graph before every step), where each read is a constant-bank operand instead of a load.
@@ -245,10 +242,61 @@ struct ParamsByValue {
   const ParamBlock& b;
   __device__ __forceinline__ float operator[](int i) const { return b.v[i]; }
 };
-template <class PA, class Nb>
+// The cell's neighbourhood of velY.  The vorticity and its gradient are wanted only where confinement acts, in hot gas, a small
+// part of a domain; there the seven curls are formed from their 42 velY cells, which the L1 holds.  Offsets along an axis: the
+// clamped cells at -2, -1, 0, +1, +2, and what lies above the clamped -1 and below the clamped +1 (the cell itself, or at
+// an edge its only neighbour: a tap outside the domain is the clamped cell's, with that cell's own neighbours).
+struct Axis { int m2, m1, c, p1, p2, above_m1, below_p1; };
+__device__ __forceinline__ Axis axis_of(int i, int n, int stride) {
+  const int m1 = max(i - 1, 0), p1 = min(i + 1, n - 1);
+  return Axis{stride * max(m1 - 1, 0), stride * m1, stride * i, stride * p1, stride * min(p1 + 1, n - 1),
+              stride * min(m1 + 1, n - 1), stride * max(p1 - 1, 0)};
+}
+// sqrt(x^2 + y^2 + z^2) with the first (kSecond: the second) of the inner two squares rounded before it is added.
+template <bool kSecond>
+__device__ __forceinline__ float length_as(f3 a) {
+  return sqrtf(__fmaf_rn(a.z, a.z, kSecond ? __fmaf_rn(a.x, a.x, __fmul_rn(a.y, a.y)) : __fmaf_rn(a.y, a.y, __fmul_rn(a.x, a.x))));
+}
+__device__ __forceinline__ f3 cross_as(f3 a, f3 b) {
+  return mk3(__fmaf_rn(a.y, b.z, -__fmul_rn(a.z, b.y)), __fmaf_rn(a.z, b.x, -__fmul_rn(a.x, b.z)), __fmaf_rn(a.x, b.y, -__fmul_rn(a.y, b.x)));
+}
+struct VelNb {
+  const float4* __restrict__ v;
+  Dims d;
+  int i, j, k;
+  __device__ f3 at(int o) const { return xyz(__ldg(v + o)); }
+  // the curl from the six neighbours' offsets
+  __device__ f3 curl(int xm, int xp, int ym, int yp, int zm, int zp) const {
+    const f3 L = at(xm), R = at(xp), B = at(ym), T = at(yp), K = at(zm), F = at(zp);
+    return mk3((T.z - B.z) - (F.y - K.y), (F.x - K.x) - (R.z - L.z), (R.y - L.y) - (T.x - B.x)) * 0.5f;
+  }
+  __device__ float4 vel_center() const { return __ldg(v + cell(i, j, k, d.nx, d.ny)); }
+  // The vorticity w, and in g the gradient of its length.
+  __device__ f3 vorticity(f3& g) const {
+    const Axis X = axis_of(i, d.nx, 1), Y = axis_of(j, d.ny, d.nx), Z = axis_of(k, d.nz, d.nx * d.ny);
+    const int yz = Y.c + Z.c, xz = X.c + Z.c, xy = X.c + Y.c;
+    auto side = [&](int xm, int xp, int ym, int yp, int zm, int zp) { return length_as<false>(curl(xm, xp, ym, yp, zm, zp)); };
+    g.x = side(X.below_p1 + yz, X.p2 + yz, X.p1 + Y.m1 + Z.c, X.p1 + Y.p1 + Z.c, X.p1 + Y.c + Z.m1, X.p1 + Y.c + Z.p1) -
+          side(X.m2 + yz, X.above_m1 + yz, X.m1 + Y.m1 + Z.c, X.m1 + Y.p1 + Z.c, X.m1 + Y.c + Z.m1, X.m1 + Y.c + Z.p1);
+    g.y = side(X.m1 + Y.p1 + Z.c, X.p1 + Y.p1 + Z.c, Y.below_p1 + xz, Y.p2 + xz, X.c + Y.p1 + Z.m1, X.c + Y.p1 + Z.p1) -
+          side(X.m1 + Y.m1 + Z.c, X.p1 + Y.m1 + Z.c, Y.m2 + xz, Y.above_m1 + xz, X.c + Y.m1 + Z.m1, X.c + Y.m1 + Z.p1);
+    g.z = side(X.m1 + Y.c + Z.p1, X.p1 + Y.c + Z.p1, X.c + Y.m1 + Z.p1, X.c + Y.p1 + Z.p1, Z.below_p1 + xy, Z.p2 + xy) -
+          side(X.m1 + Y.c + Z.m1, X.p1 + Y.c + Z.m1, X.c + Y.m1 + Z.m1, X.c + Y.p1 + Z.m1, Z.m2 + xy, Z.above_m1 + xy);
+    return curl(X.m1 + yz, X.p1 + yz, Y.m1 + xz, Y.p1 + xz, Z.m1 + xy, Z.p1 + xy);
+  }
+  __device__ f3 lap_v() const {   // src/sim.js:340-343, same summation order
+    f3 l = xyz(ldc(v, i + 1, j, k, d)) + xyz(ldc(v, i - 1, j, k, d));
+    l = l + xyz(ldc(v, i, j + 1, k, d));
+    l = l + xyz(ldc(v, i, j - 1, k, d));
+    l = l + xyz(ldc(v, i, j, k + 1, d));
+    l = l + xyz(ldc(v, i, j, k - 1, d));
+    return l - xyz(vel_center()) * 6.0f;
+  }
+};
+template <class PA>
 __device__ __forceinline__ void forces_cell(const PA& pa, const Fields& f, const uint2* __restrict__ noiseT,
                                             const uint2* __restrict__ curlT, Dims d, int i, int j, int k, unsigned ci,
-                                            const Nb& nb, float4 s, float4 s2, const float4 geo) {
+                                            const VelNb& nb, float4 s, float4 s2, const float4 geo) {
   const float dt = pa[P_dt], dx = pa[P_dx], I = pa[P_intensity];
   const float seed = pa[P_seed], time = pa[P_time];
   f3 p = mk3(pa[P_ox], pa[P_oy], pa[P_oz]) + mk3((float)i + 0.5f, (float)j + 0.5f, (float)k + 0.5f) * dx;
@@ -379,9 +427,10 @@ __device__ __forceinline__ void forces_cell(const PA& pa, const Fields& f, const
     // velocity component can differ.
     const float gate = sstep(450.0f, 900.0f, T) * (1.0f - srcAll) * sstep(0.02f, 0.08f, p.y) * lam;
     if (gate != 0.0f) {
-      const f3 g = nb.grad_w();
-      const float gl = len3(g);
-      if (gl > 1e-6f) v = v + cross3(g / gl, xyz(nb.vort_center())) * (pa[P_vortEps] * gate) * dt;
+      f3 g;
+      const f3 w = nb.vorticity(g);
+      const float gl = length_as<true>(g);
+      if (gl > 1e-6f) v = v + cross_as(g / gl, w) * (pa[P_vortEps] * gate) * dt;
     }
 
     // ---- sub-grid turbulence: rising, evolving curl noise (src/sim.js:364-368); skipped the same way where
@@ -435,222 +484,15 @@ __device__ __forceinline__ void forces_cell(const PA& pa, const Fields& f, const
   f.S2[ci] = s2;
 }
 
-// Neighbourhood from global memory: either the vorticity field written by the curl stage, or (fused)
-// the 7 vorticity taps recomputed from clamped velY loads.
-template <bool kFusedCurl>
-struct GlobalNb {
-  const Fields& f;
-  Dims d;
-  int i, j, k;
-  __device__ float4 vel_center() const { return __ldg(f.velY + cell(i, j, k, d.nx, d.ny)); }
-  __device__ float4 vort_center() const {
-    return kFusedCurl ? curl_at(f.velY, i, j, k, d) : __ldg(f.vort + cell(i, j, k, d.nx, d.ny));
-  }
-  __device__ f3 grad_w() const {
-    if (kFusedCurl)
-      return mk3(curl_at(f.velY, min(i + 1, d.nx - 1), j, k, d).w - curl_at(f.velY, max(i - 1, 0), j, k, d).w,
-                 curl_at(f.velY, i, min(j + 1, d.ny - 1), k, d).w - curl_at(f.velY, i, max(j - 1, 0), k, d).w,
-                 curl_at(f.velY, i, j, min(k + 1, d.nz - 1), d).w - curl_at(f.velY, i, j, max(k - 1, 0), d).w);
-    return mk3(ldc(f.vort, i + 1, j, k, d).w - ldc(f.vort, i - 1, j, k, d).w,
-               ldc(f.vort, i, j + 1, k, d).w - ldc(f.vort, i, j - 1, k, d).w,
-               ldc(f.vort, i, j, k + 1, d).w - ldc(f.vort, i, j, k - 1, d).w);
-  }
-  __device__ f3 lap_v() const {   // src/sim.js:340-343, same summation order
-    f3 l = xyz(ldc(f.velY, i + 1, j, k, d)) + xyz(ldc(f.velY, i - 1, j, k, d));
-    l = l + xyz(ldc(f.velY, i, j + 1, k, d));
-    l = l + xyz(ldc(f.velY, i, j - 1, k, d));
-    l = l + xyz(ldc(f.velY, i, j, k + 1, d));
-    l = l + xyz(ldc(f.velY, i, j, k - 1, d));
-    return l - xyz(vel_center()) * 6.0f;
-  }
-};
-template <bool kFusedCurl>
-__global__ void __launch_bounds__(256) k_forces(const float* __restrict__ P, Fields f, const uint2* __restrict__ noiseT,
-                                                const uint2* __restrict__ curlT, Dims d) {
-  CellId id = cell_id(d);
+template <class TileT = Tile0, class PA>
+__device__ __forceinline__ void forces_body(const PA& pa, const Fields& f, const uint2* __restrict__ noiseT, const uint2* __restrict__ curlT,
+                                            Dims d, uint3 blk) {
+  CellId id = cell_id<TileT>(d, blk);
   if (!id.ok) return;
-  GlobalNb<kFusedCurl> nb{f, d, id.i, id.j, id.k};
+  const VelNb nb{f.velY, d, id.i, id.j, id.k};
   const size_t ci = cell(id.i, id.j, id.k, d.nx, d.ny);
-  forces_cell(ParamsGlobal{P}, f, noiseT, curlT, d, id.i, id.j, id.k, (unsigned)ci, nb, __ldg(f.SY + ci), __ldg(f.S2Y + ci),
-              __ldg(f.geo + ci));
+  forces_cell(pa, f, noiseT, curlT, d, id.i, id.j, id.k, (unsigned)ci, nb, __ldg(f.SY + ci), __ldg(f.S2Y + ci), __ldg(f.geo + ci));
 }
-
-// ---- z-marching shared-memory variant of curl + forces ----
-// A CTA of 32 x 8 threads owns a 32 x 8 column tile and marches through a run of planes (FZ planes per CTA
-// in the batched kernel; an equal share of all (column, plane) units in the one-wave kernel).  Shared memory holds a
-// ring of 5 velY planes (tile + 2-cell halo, clamped to the domain like `ld`) and a ring of 3 planes of the
-// vorticity magnitude |w| (tile + 1-cell halo), which is all the confinement gradient reads; the vorticity
-// vector itself is needed only at the cell, where confinement acts, and is formed there from the velY ring
-// with the same arithmetic.  |w| at a halo position outside the domain is that of the clamped position,
-// which is what `ld(vortT, c +- e)` returns.  Each velY value is loaded ~2x per cell (halo overhead) instead
-// of the 42 gathers of the per-cell recompute.
-constexpr int FT_X = 32, FT_Y = 8, FZ = 16;
-constexpr int VX = FT_X + 4, VY = FT_Y + 4;      // velY plane with 2-cell halo
-constexpr int WX = FT_X + 2, WY = FT_Y + 2;      // vorticity plane with 1-cell halo
-// Ring slots are addressed by logical z (z >= -2): velY plane z lives in slot (z + 10) % 5, vorticity
-// plane z in slot (z + 9) % 3.
-__device__ __forceinline__ float4* vslot(float4* vbuf, int z) { return vbuf + ((z + 10) % 5) * (VX * VY); }
-__device__ __forceinline__ float* wslot(float* wbuf, int z) { return wbuf + ((z + 9) % 3) * (WX * WY); }
-// The curl of velY at tile position c (a VX*VY offset) from planes K (z-1), P0 (z), F (z+1), given the
-// positions of its x and y neighbours (clamped to the domain by the caller); the arithmetic of curl_at.
-__device__ __forceinline__ f3 curl_tile(const float4* K, const float4* P0, const float4* F, int c, int cxm, int cxp, int cym,
-                                        int cyp) {
-  f3 L = xyz(P0[cxm]), R = xyz(P0[cxp]);
-  f3 B = xyz(P0[cym]), T = xyz(P0[cyp]);
-  f3 Kv = xyz(K[c]), Fv = xyz(F[c]);
-  return mk3((T.z - B.z) - (Fv.y - Kv.y), (Fv.x - Kv.x) - (R.z - L.z), (R.y - L.y) - (T.x - B.x)) * 0.5f;
-}
-struct TileNb {
-  const float4 *vm, *v0, *vp;   // velY planes z-1, z, z+1 (VX*VY each)
-  const float *wm, *w0, *wp;    // |w| planes z-1, z, z+1 (WX*WY each)
-  int tx, ty;                   // thread position in the tile
-  __device__ float4 vel_center() const { return v0[(ty + 2) * VX + tx + 2]; }
-  // The cell is inside the domain and the ring's halo holds clamped positions, so its four in-plane
-  // neighbours in the ring are the clamped neighbours; vm / vp are the clamped planes z -+ 1.
-  __device__ float4 vort_center() const {
-    const int c = (ty + 2) * VX + tx + 2;
-    const f3 w = curl_tile(vm, v0, vp, c, c - 1, c + 1, c - VX, c + VX);
-    return make_float4(w.x, w.y, w.z, 0.0f);
-  }
-  __device__ f3 grad_w() const {
-    const int c = (ty + 1) * WX + tx + 1;
-    return mk3(w0[c + 1] - w0[c - 1], w0[c + WX] - w0[c - WX], wp[c] - wm[c]);
-  }
-  __device__ f3 lap_v() const {   // src/sim.js:340-343, same summation order
-    const int c = (ty + 2) * VX + tx + 2;
-    f3 l = xyz(v0[c + 1]) + xyz(v0[c - 1]);
-    l = l + xyz(v0[c + VX]);
-    l = l + xyz(v0[c - VX]);
-    l = l + xyz(vp[c]);
-    l = l + xyz(vm[c]);
-    return l - xyz(v0[c]) * 6.0f;
-  }
-};
-__device__ __forceinline__ int clampi(int v, int n) { return min(max(v, 0), n - 1); }
-// 16-byte asynchronous global -> shared copy (cached in L2 only), and its group commit / wait.
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-// The plane-independent part of a thread's share of the ring traffic for one column tile, worked out once
-// per march: each thread copies velY elements t = tid and tid + 256 of a plane and forms vorticity elements
-// t = tid and tid + 256.
-//  * vsrc[k]: x + nx * y of velY element k's source, clamped to the domain as `ld` does (-1: no element);
-//  * wtap[k]: vorticity element k's velY ring offset (bits 0-9) and which of its x-, x+, y-, y+ neighbours lie
-//    inside the domain (bits 10-13; a clamped neighbour is the centre itself) (-1: no element).
-constexpr int FT_N = FT_X * FT_Y;
-static_assert(VX * VY <= 2 * FT_N && WX * WY <= 2 * FT_N && VX * VY < 1024, "two ring elements per thread, 10-bit offsets");
-struct MarchPlan {
-  int vsrc[2], wtap[2];
-};
-__device__ __forceinline__ MarchPlan march_plan(int x0, int y0, Dims d) {
-  MarchPlan m;
-  const int tid = threadIdx.y * FT_X + threadIdx.x;
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const int t = tid + k * FT_N;
-    m.vsrc[k] = -1;
-    m.wtap[k] = -1;
-    if (t < VX * VY) {
-      const int lx = t % VX, ly = t / VX;
-      m.vsrc[k] = clampi(x0 + lx - 2, d.nx) + d.nx * clampi(y0 + ly - 2, d.ny);
-    }
-    if (t < WX * WY) {
-      const int lx = t % WX, ly = t / WX;
-      // clamp the position to the domain, then express it in tile coordinates (velY tile origin at -2)
-      const int gx = clampi(x0 + lx - 1, d.nx), gy = clampi(y0 + ly - 1, d.ny);
-      const int c = (gy - y0 + 2) * VX + (gx - x0 + 2);
-      m.wtap[k] = c | (gx > 0) << 10 | (gx < d.nx - 1) << 11 | (gy > 0) << 12 | (gy < d.ny - 1) << 13;
-    }
-  }
-  return m;
-}
-// Starts the copy of logical plane z (clamped) of velY for the march's tile into `dst`; the caller commits and
-// waits.
-__device__ __forceinline__ void load_vplane(float4* dst, const float4* __restrict__ velY, const MarchPlan& m, int z, Dims d) {
-  const unsigned zo = (unsigned)clampi(z, d.nz) * (unsigned)(d.nx * d.ny);
-  const int tid = threadIdx.y * FT_X + threadIdx.x;
-#pragma unroll
-  for (int k = 0; k < 2; ++k)
-    if (m.vsrc[k] >= 0) cp_async16(dst + tid + k * FT_N, velY + (zo + (unsigned)m.vsrc[k]));
-}
-// |w| of logical plane zlog into `dst` (positions clamped to the domain), from the velY ring.  The planes it
-// reads (clamp(zlog) and its clamped z neighbours) are resident in the ring when this is called.
-__device__ __forceinline__ void curl_plane(float* dst, float4* vbuf, const MarchPlan& m, int zlog, Dims d) {
-  const int zc = clampi(zlog, d.nz);
-  const float4* PK = vslot(vbuf, clampi(zc - 1, d.nz));
-  const float4* P0 = vslot(vbuf, zc);
-  const float4* PF = vslot(vbuf, clampi(zc + 1, d.nz));
-  const int tid = threadIdx.y * FT_X + threadIdx.x;
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const int tap = m.wtap[k];
-    if (tap < 0) continue;
-    const int c = tap & 1023;
-    const f3 w = curl_tile(PK, P0, PF, c, c - ((tap >> 10) & 1), c + ((tap >> 11) & 1), c - ((tap >> 12) & 1) * VX,
-                           c + ((tap >> 13) & 1) * VX);
-    dst[tid + k * FT_N] = len3(w);
-  }
-}
-// Marches the column tile at (x0, y0) through planes [z0, z1), z1 > z0.  The copy of the next velY plane is
-// started before the current plane's source terms and completes behind them: it goes to the slot of plane
-// z - 2, which nothing reads any more (the vorticity of z - 1 was formed three planes ago, and the previous
-// plane's Laplacian finished before the last barrier).
-template <class PA>
-__device__ __forceinline__ void forces_march(const PA& pa, const Fields& f, const uint2* __restrict__ noiseT,
-                                             const uint2* __restrict__ curlT, Dims d, int x0, int y0, int z0, int z1,
-                                             float4* fsm) {
-  float4* vbuf = fsm;                                        // 5 * VX * VY
-  float* wbuf = reinterpret_cast<float*>(fsm + 5 * VX * VY);  // 3 * WX * WY
-  const MarchPlan m = march_plan(x0, y0, d);
-  for (int z = z0 - 2; z <= z0 + 2; ++z) load_vplane(vslot(vbuf, z), f.velY, m, z, d);
-  cp_async_commit();
-  cp_async_wait_all();
-  __syncthreads();
-  for (int z = z0 - 1; z <= z0 + 1; ++z) curl_plane(wslot(wbuf, z), vbuf, m, z, d);
-  __syncthreads();
-  const int i = x0 + threadIdx.x, j = y0 + threadIdx.y;
-  const bool mine = i < d.nx && j < d.ny;
-  const unsigned plane = (unsigned)(d.nx * d.ny);
-  unsigned ci = mine ? (unsigned)i + (unsigned)d.nx * ((unsigned)j + (unsigned)d.ny * (unsigned)z0) : 0u;
-  // this thread's SY, S2Y, geo for the current plane, loaded one plane ahead
-  float4 s_n = make_float4(0.0f, 0.0f, 0.0f, 0.0f), s2_n = s_n, g_n = s_n;
-  if (mine) { s_n = __ldg(f.SY + ci); s2_n = __ldg(f.S2Y + ci); g_n = __ldg(f.geo + ci); }
-  for (int z = z0; z < z1; ++z, ci += plane) {
-    const float4 s = s_n, s2 = s2_n, g = g_n;
-    const bool more = z + 1 < z1;
-    if (more) {
-      load_vplane(vslot(vbuf, z + 3), f.velY, m, z + 3, d);   // into the slot of plane z - 2
-      cp_async_commit();
-    }
-    if (mine && more) { s_n = __ldg(f.SY + ci + plane); s2_n = __ldg(f.S2Y + ci + plane); g_n = __ldg(f.geo + ci + plane); }
-    if (mine) {
-      TileNb nb;
-      nb.vm = vslot(vbuf, z - 1); nb.v0 = vslot(vbuf, z); nb.vp = vslot(vbuf, z + 1);
-      nb.wm = wslot(wbuf, z - 1); nb.w0 = wslot(wbuf, z); nb.wp = wslot(wbuf, z + 1);
-      nb.tx = threadIdx.x;
-      nb.ty = threadIdx.y;
-      forces_cell(pa, f, noiseT, curlT, d, i, j, z, ci, nb, s, s2, g);
-    }
-    if (more) {
-      cp_async_wait_all();
-      __syncthreads();          // plane z + 3 is visible; everyone is done with vorticity plane z - 1
-      curl_plane(wslot(wbuf, z + 2), vbuf, m, z + 2, d);       // replaces vorticity plane z - 1
-      __syncthreads();
-    }
-  }
-}
-// The batched kernel's CTA: column tile (blk.x, blk.y), planes [blk.z * ZD, blk.z * ZD + ZD).
-template <int ZD = FZ>   // planes one CTA marches through
-__device__ __forceinline__ void forces_tiled_body(const float* __restrict__ P, const Fields& f, const uint2* __restrict__ noiseT,
-                                                  const uint2* __restrict__ curlT, Dims d, uint3 blk, float4* fsm) {
-  pdl_wait();
-  pdl_trigger();
-  const int z0 = blk.z * ZD;
-  forces_march(ParamsGlobal{P}, f, noiseT, curlT, d, blk.x * FT_X, blk.y * FT_Y, z0, min(z0 + ZD, d.nz), fsm);
-}
-constexpr size_t FORCES_TILED_SMEM = sizeof(float4) * 5 * VX * VY + sizeof(float) * 3 * WX * WY;
 
 // ---------------- divergence minus the expansion target (src/sim.js:399-413) ----------------
 // The z neighbours of a thread's K cells are its own cells.
@@ -722,37 +564,14 @@ __global__ void __launch_bounds__(256, FIRE_ADV_MIN_CTAS) k_adv1_column(const fl
   adv1_column<Tile0, ADV1_DEPTH>(P, f, d, blockIdx);
 }
 __global__ void __launch_bounds__(256, FIRE_ADV_MIN_CTAS) k_adv2(const float* __restrict__ P, Fields f, Dims d) { adv2_body(P, f, d, blockIdx); }
-// One wave of resident CTAs.  The (column tile, plane) units, planes fastest, are split into gridDim.x equal
-// contiguous ranges, so every SM marches the same number of planes (a grid of fixed-depth chunks leaves its
-// last wave partly idle); a range that runs into the next column restarts the march there.
-template <class PA>
-__device__ __forceinline__ void forces_persistent(const PA& pa, const Fields& f, const uint2* __restrict__ noiseT,
-                                                  const uint2* __restrict__ curlT, Dims d, float4* fsm) {
-  pdl_wait();
-  pdl_trigger();
-  const int gx = (d.nx + FT_X - 1) / FT_X, gy = (d.ny + FT_Y - 1) / FT_Y;
-  const long long units = (long long)gx * gy * d.nz;
-  long long u = units * blockIdx.x / gridDim.x;
-  const long long end = units * (blockIdx.x + 1) / gridDim.x;
-  while (u < end) {
-    const int col = (int)(u / d.nz), z0 = (int)(u % d.nz);
-    const int z1 = (int)min((long long)d.nz, z0 + (end - u));
-    forces_march(pa, f, noiseT, curlT, d, (col % gx) * FT_X, (col / gx) * FT_Y, z0, z1, fsm);
-    u += z1 - z0;
-    if (u < end) __syncthreads();   // the next march refills the rings
-  }
+__global__ void __launch_bounds__(256, FIRE_FORCES_MIN_CTAS) k_forces(const float* __restrict__ P, Fields f, const uint2* __restrict__ noiseT,
+                                                                      const uint2* __restrict__ curlT, Dims d) {
+  forces_body(ParamsGlobal{P}, f, noiseT, curlT, d, blockIdx);
 }
-__global__ void __launch_bounds__(FT_X * FT_Y, FIRE_FORCES_MIN_CTAS) k_forces_tiled(const float* __restrict__ P, Fields f,
-                                                                                     const uint2* __restrict__ noiseT,
-                                                                                     const uint2* __restrict__ curlT, Dims d) {
-  extern __shared__ float4 fsm[];
-  forces_persistent(ParamsGlobal{P}, f, noiseT, curlT, d, fsm);
-}
-__global__ void __launch_bounds__(FT_X * FT_Y, FIRE_FORCES_MIN_CTAS) k_forces_tiled_pb(const __grid_constant__ ParamBlock pb, Fields f,
-                                                                                        const uint2* __restrict__ noiseT,
-                                                                                        const uint2* __restrict__ curlT, Dims d) {
-  extern __shared__ float4 fsm[];
-  forces_persistent(ParamsByValue{pb}, f, noiseT, curlT, d, fsm);
+__global__ void __launch_bounds__(256, FIRE_FORCES_MIN_CTAS) k_forces_pb(const __grid_constant__ ParamBlock pb, Fields f,
+                                                                         const uint2* __restrict__ noiseT, const uint2* __restrict__ curlT,
+                                                                         Dims d) {
+  forces_body(ParamsByValue{pb}, f, noiseT, curlT, d, blockIdx);
 }
 // mg_counter (the residual-driven step graph only, else null): the solve that follows counts its V-cycles
 // from zero, so this kernel clears the count instead of a separate launch.
@@ -785,13 +604,12 @@ __global__ void __launch_bounds__(256, FIRE_ADV_MIN_CTAS) k_adv2_b(const __grid_
   batch_locate(m, blk, i);
   adv2_body<T>(I.s[i].P, I.s[i].f, I.s[i].d, blk);
 }
-template <int ZD>
-__global__ void __launch_bounds__(FT_X * FT_Y, FIRE_FORCES_MIN_CTAS) k_forces_b(const __grid_constant__ BatchMap m, const __grid_constant__ StepBatch I,
-                                                                                 const uint2* __restrict__ noiseT, const uint2* __restrict__ curlT) {
-  extern __shared__ float4 fsm[];
+template <class T>
+__global__ void __launch_bounds__(256, FIRE_FORCES_MIN_CTAS) k_forces_b(const __grid_constant__ BatchMap m, const __grid_constant__ StepBatch I,
+                                                                        const uint2* __restrict__ noiseT, const uint2* __restrict__ curlT) {
   uint3 blk; int i;
   batch_locate(m, blk, i);
-  forces_tiled_body<ZD>(I.s[i].P, I.s[i].f, noiseT, curlT, I.s[i].d, blk, fsm);
+  forces_body<T>(ParamsGlobal{I.s[i].P}, I.s[i].f, noiseT, curlT, I.s[i].d, blk);
 }
 template <class T, int K>
 __global__ void __launch_bounds__(256) k_div_b(const __grid_constant__ BatchMap m, const __grid_constant__ StepBatch I) {
@@ -807,7 +625,7 @@ __global__ void __launch_bounds__(256) k_project_b(const __grid_constant__ Batch
 }
 
 // The tile candidates of the batched stages: CELL_TILES cell tiles (256 threads each; x stays 32 or 64 wide
-// for coalescing) and FORCES_TILES z-march depths of the forces tile.
+// for coalescing); the forces stage takes the first FORCES_TILES of them.
 template <class F> void with_cell_tile(int v, F&& f) {
   switch (v) {
     case 1: f(Tile<32, 8, 1>{}); break;
@@ -817,14 +635,7 @@ template <class F> void with_cell_tile(int v, F&& f) {
   }
 }
 static_assert(CELL_TILES == 4, "with_cell_tile lists every cell tile");
-constexpr int kForcesDepth[FORCES_TILES] = {FZ, 8, 32};
-template <class F> void with_forces_depth(int v, F&& f) {
-  switch (v) {
-    case 1: f(std::integral_constant<int, 8>{}); break;
-    case 2: f(std::integral_constant<int, 32>{}); break;
-    default: f(std::integral_constant<int, FZ>{}); break;
-  }
-}
+static_assert(FORCES_TILES <= CELL_TILES, "the forces stage's candidates are cell tiles");
 
 // ---------------- launchers ----------------
 // A thread takes several cells along z where enough threads remain to fill the SMs.  Measured (GB300, us, one cell -> several):
@@ -842,49 +653,22 @@ void launch_adv1(const float* P, Fields f, Dims d, cudaStream_t st) {
 }
 void launch_adv2(const float* P, Fields f, Dims d, cudaStream_t st) { launch_pdl(k_adv2, grid_for(d), block_shape(), 0, st, P, f, d); }
 void launch_curl(Fields f, Dims d, cudaStream_t st) { launch_pdl(k_curl, grid_for(d), block_shape(), 0, st, f, d); }
-// Resident k_forces_tiled CTAs of each device (CTAs per SM x SMs), set by step_configure.
-constexpr int kMaxDevices = 64;
-static int g_forces_wave[kMaxDevices];
-static dim3 forces_wave_grid(Dims d) {
-  const long long units = (long long)((d.nx + FT_X - 1) / FT_X) * ((d.ny + FT_Y - 1) / FT_Y) * d.nz;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  const int wave = dev >= 0 && dev < kMaxDevices && g_forces_wave[dev] > 0 ? g_forces_wave[dev] : 4 * 152;
-  return dim3((unsigned)(units < wave ? units : wave));
-}
 void launch_forces(const float* P, Fields f, const uint2* noise, const uint2* curl, Dims d, cudaStream_t st) {
-  launch_pdl(k_forces_tiled, forces_wave_grid(d), dim3(FT_X, FT_Y), FORCES_TILED_SMEM, st, P, f, noise, curl, d);
+  launch_pdl(k_forces, grid_for(d), block_shape(), 0, st, P, f, noise, curl, d);
 }
 void launch_forces_pb(const ParamBlock& pb, Fields f, const uint2* noise, const uint2* curl, Dims d, cudaStream_t st) {
-  launch_pdl(k_forces_tiled_pb, forces_wave_grid(d), dim3(FT_X, FT_Y), FORCES_TILED_SMEM, st, pb, f, noise, curl, d);
+  launch_pdl(k_forces_pb, grid_for(d), block_shape(), 0, st, pb, f, noise, curl, d);
 }
 cudaError_t forces_pb_set(cudaGraphExec_t exec, cudaGraphNode_t node, const ParamBlock& pb, Fields f, const uint2* noise,
                           const uint2* curl, Dims d) {
   void* args[] = {(void*)&pb, (void*)&f, (void*)&noise, (void*)&curl, (void*)&d};
   cudaKernelNodeParams kp = {};
-  kp.func = (void*)k_forces_tiled_pb;
-  kp.gridDim = forces_wave_grid(d);
-  kp.blockDim = dim3(FT_X, FT_Y);
-  kp.sharedMemBytes = (unsigned)FORCES_TILED_SMEM;
+  kp.func = (void*)k_forces_pb;
+  kp.gridDim = grid_for(d);
+  kp.blockDim = block_shape();
+  kp.sharedMemBytes = 0;
   kp.kernelParams = args;
   return cudaGraphExecKernelNodeSetParams(exec, node, &kp);
-}
-void launch_forces_recompute(const float* P, Fields f, const uint2* noise, const uint2* curl, Dims d, cudaStream_t st) {
-  launch_pdl(k_forces<true>, grid_for(d), block_shape(), 0, st, P, f, noise, curl, d);
-}
-cudaError_t step_configure() {
-  cudaError_t e = cudaFuncSetAttribute(k_forces_tiled, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FORCES_TILED_SMEM);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_forces_tiled_pb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FORCES_TILED_SMEM);
-  int dev = 0, sms = 0, per_sm = 0;
-  if (e == cudaSuccess) e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_forces_tiled, FT_X * FT_Y, FORCES_TILED_SMEM);
-  if (e == cudaSuccess && dev >= 0 && dev < kMaxDevices) g_forces_wave[dev] = (per_sm > 0 ? per_sm : 1) * sms;
-  for (int v = 0; v < FORCES_TILES && e == cudaSuccess; ++v)
-    with_forces_depth(v, [&](auto z) {
-      e = cudaFuncSetAttribute(k_forces_b<decltype(z)::value>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FORCES_TILED_SMEM);
-    });
-  return e;
 }
 // Block grids of the batched stages for a simulation of dims d with tile candidate `tile`.
 dim3 step_grid(Dims d, int tile, int depth) {
@@ -894,10 +678,6 @@ dim3 step_grid(Dims d, int tile, int depth) {
     g = dim3((d.nx + T::X - 1) / T::X, (d.ny + T::Y - 1) / T::Y, (d.nz + T::Z * depth - 1) / (T::Z * depth));
   });
   return g;
-}
-dim3 forces_grid(Dims d, int tile) {
-  const int zd = kForcesDepth[tile >= 0 && tile < FORCES_TILES ? tile : 0];
-  return dim3((d.nx + FT_X - 1) / FT_X, (d.ny + FT_Y - 1) / FT_Y, (d.nz + zd - 1) / zd);
 }
 void launch_adv1_batch(const BatchMap& m, const StepBatch& I, int tile, int depth, cudaStream_t st) {
   with_cell_tile(tile, [&](auto t) {
@@ -912,8 +692,9 @@ void launch_adv2_batch(const BatchMap& m, const StepBatch& I, int tile, cudaStre
   });
 }
 void launch_forces_batch(const BatchMap& m, const StepBatch& I, const uint2* noise, const uint2* curl, int tile, cudaStream_t st) {
-  with_forces_depth(tile, [&](auto z) {
-    launch_pdl(k_forces_b<decltype(z)::value>, dim3(m.prefix[m.n]), dim3(FT_X, FT_Y), FORCES_TILED_SMEM, st, m, I, noise, curl);
+  with_cell_tile(tile, [&](auto t) {
+    using T = decltype(t);
+    launch_pdl(k_forces_b<T>, dim3(m.prefix[m.n]), dim3(T::X, T::Y, T::Z), 0, st, m, I, noise, curl);
   });
 }
 void launch_div_batch(const BatchMap& m, const StepBatch& I, int tile, int depth, cudaStream_t st) {
@@ -927,9 +708,6 @@ void launch_project_batch(const BatchMap& m, const StepBatch& I, int tile, int d
     using T = decltype(t);
     launch_pdl(depth > 1 ? k_project_b<T, FLOW_DEPTH> : k_project_b<T, 1>, dim3(m.prefix[m.n]), dim3(T::X, T::Y, T::Z), 0, st, m, I);
   });
-}
-void launch_forces_unfused(const float* P, Fields f, const uint2* noise, const uint2* curl, Dims d, cudaStream_t st) {
-  launch_pdl(k_forces<false>, grid_for(d), block_shape(), 0, st, P, f, noise, curl, d);
 }
 void launch_div(const float* P, Fields f, float* b0, Dims d, cudaStream_t st, int* mg_counter) {
   const int K = flow_depth(cells_of(d));
