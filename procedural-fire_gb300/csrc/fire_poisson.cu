@@ -801,7 +801,8 @@ int fire_poisson_create(const int res[3], float h, int precision, int device, Fi
     L.nx = M.nx; L.ny = M.ny; L.nz = M.nz; L.h = M.h;
     L.sto = (ps->ir && l < ps->tailFirst) ? sto : STO_F32;
     // every level that launches smooth: all above the coarse end, and the coarsest itself where none takes it
-    if (l < ps->tailFirst) L.sweep = ps->mg[l].sweep = plan_sweep(ps->mg[l]);
+    // (not of 16-bit rows of an odd length)
+    if (l < ps->tailFirst && (L.sto == STO_F32 || M.nx % 2 == 0)) L.sweep = ps->mg[l].sweep = plan_sweep(ps->mg[l]);
     const size_t bytes = align_up((size_t)M.nx * M.ny * M.nz * elem_bytes(L.sto));
     if (L.sweep.px > 0) { p2Off[l] = off; off += bytes; }
     if (l == 0 && !ps->ir) { pOff[l] = bOff[l] = (size_t)-1; continue; }

@@ -19,6 +19,10 @@
 // 96x192x96 19.0 -> 10.7, 128x256x128 28.0 -> 18.3, 256x512x256 270 -> 120 (402 MB there: 3.4 TB/s).  A step costs 0.3-0.5 us
 // whatever the tile: about 130 instructions a warp behind a chain of reads, four dependent updates, a write and a barrier;
 // registers and the halo keep it to one or two CTAs an SM.
+// Grids without coarser levels (an odd side) run all their sweeps here; rows of an odd length copy their cells one by one.  Steps of two
+// cycles with 64 sweeps each, us, colour launches -> this: 101x90x95 886 -> 731, 131x211x120 2491 -> 1709.
+// Tried and slower: loads into register slots two planes ahead instead of the ring (16x16x16 2.9 -> 4.8, 256x512x256 123 -> 152:
+// two steps do not cover a load, and 16 unrolled steps miss the instruction cache), four rows a thread (123 -> 134: spills).
 #include <algorithm>
 #include "fire_device.cuh"
 #include "fire_launch.cuh"
@@ -33,10 +37,19 @@ constexpr int SW_THREADS = 512;   // 128 registers a thread
 constexpr int SW_AHEAD = 4;       // planes of p and b in flight: a step takes about 0.3 us, a load from L2 0.4 and more
 constexpr int SW_RING = 7;        // entries a thread's ring is long: six planes, and one more so that 32 lanes hit all banks
 
-// Asynchronous copy of one pair; zeros where it lies outside the domain.
-template <typename V>
-__device__ __forceinline__ void copy_pair(V* dst, const void* src, bool in) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "n"((int)sizeof(V)), "r"(in ? (int)sizeof(V) : 0) : "memory");
+// Asynchronous copy of one pair, or (kOdd: rows of an odd length, whose pairs are not aligned) of its two cells one by one; zeros
+// where it lies outside the domain, and for the second cell where only that does.
+template <bool kOdd, typename V>
+__device__ __forceinline__ void copy_pair(V* dst, const void* src, bool in, bool second) {
+  if (kOdd) {
+    static_assert(!kOdd || sizeof(V) == 8, "cells of four bytes");
+    const unsigned to = (unsigned)__cvta_generic_to_shared(dst);
+    const char* from = static_cast<const char*>(src);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to), "l"(from), "r"(in ? 4 : 0) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to + 4), "l"(in && second ? from + 4 : from), "r"(in && second ? 4 : 0) : "memory");
+  } else {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "n"((int)sizeof(V)), "r"(in ? (int)sizeof(V) : 0) : "memory");
+  }
 }
 
 // A column of a thread as rings over the planes: plane k - j of the march's step k = i (mod 6) sits at slot (i - j) mod 6, so
@@ -105,7 +118,7 @@ __device__ __forceinline__ void step(const Sweeper& w, Col (&c)[SW_ROWS][2], int
 
 // One tile: [x0, x1) x [y0, y1) x [z0, z1) is written; block of px pairs x ty thread rows.
 struct SweepTile { int lx, ly, x0, x1, y0, y1, z0, z1; };
-template <typename T, bool kZero, bool kRelax>
+template <typename T, bool kZero, bool kRelax, bool kOdd = false>
 __device__ __forceinline__ void sweep2_body(const T* __restrict__ p, const T* __restrict__ b, T* __restrict__ out, int nx, int ny, int nz,
                                             float h, float omega, int PX, int TY, const SweepTile& t) {
   extern __shared__ float4 sw_smem[];
@@ -120,7 +133,8 @@ __device__ __forceinline__ void sweep2_body(const T* __restrict__ p, const T* __
   w.S = sw_smem + w.pitch * (SW_ROWS * ty + 1) + px + 1;
   for (int i = tid; i < 2 * w.par; i += blockDim.x) sw_smem[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   const int x = t.lx + 2 * px, y = t.ly + SW_ROWS * ty;
-  w.live = work && x < nx && y < ny;   // nx is even; of an odd ny the last thread row has one row in the domain
+  w.live = work && x < nx && y < ny;   // of an odd nx or ny the last pair or thread row has one column or row in the domain
+  const bool wide = !kOdd || x + 1 < nx;
   const bool both = y + 1 < ny;
   const bool core = w.live && x >= t.x0 && x < t.x1 && y >= t.y0 && y < t.y1;
   Col c[SW_ROWS][2];
@@ -131,7 +145,7 @@ __device__ __forceinline__ void sweep2_body(const T* __restrict__ p, const T* __
       const float d = 6.0f + (x + q == 0 ? 1.0f : 0.0f) + (x + q == nx - 1 ? 1.0f : 0.0f) + (y + r == ny - 1 ? 1.0f : 0.0f) - (y + r == 0 ? 1.0f : 0.0f);
       asm("rcp.approx.f32 %0, %1;" : "=f"(w.rd[r][q]) : "f"(d));
       asm("rcp.approx.f32 %0, %1;" : "=f"(w.rdz[r][q]) : "f"(d + 1.0f));
-      if (r == 1 && !both) w.rd[r][q] = w.rdz[r][q] = 0.0f;   // a row outside stays zero
+      if ((r == 1 && !both) || (q == 1 && !wide)) w.rd[r][q] = w.rdz[r][q] = 0.0f;   // a row or column outside stays zero
 #pragma unroll
       for (int j = 0; j < 6; ++j) c[r][q].v[j] = c[r][q].b[j] = 0.0f;
     }
@@ -154,8 +168,8 @@ __device__ __forceinline__ void sweep2_body(const T* __restrict__ p, const T* __
 #pragma unroll
     for (int r = 0; r < SW_ROWS; ++r) {
       const bool here = in && (r == 0 || both);
-      if (!kZero) copy_pair(ring[r] + entry, pq + r * row, here);
-      copy_pair(ring[SW_ROWS + r] + entry, bq + r * row, here);
+      if (!kZero) copy_pair<kOdd>(ring[r] + entry, pq + r * row, here, wide);
+      copy_pair<kOdd>(ring[SW_ROWS + r] + entry, bq + r * row, here, wide);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
     if (q + 1 < nz) { pq += ahead; bq += ahead; }
@@ -190,7 +204,15 @@ __device__ __forceinline__ void sweep2_body(const T* __restrict__ p, const T* __
       if (core && k - SW_HALO >= t.z0)
 #pragma unroll
         for (int r = 0; r < SW_ROWS; ++r)
-          if (r == 0 || both) *reinterpret_cast<V*>(oq + r * nx) = Cells2<T>::put(make_float2(c[r][0].v[slot(I, 4)], c[r][1].v[slot(I, 4)]));
+          if (r == 0 || both) {
+            const float2 v = make_float2(c[r][0].v[slot(I, 4)], c[r][1].v[slot(I, 4)]);
+            if (!kOdd) {
+              *reinterpret_cast<V*>(oq + r * nx) = Cells2<T>::put(v);
+            } else {
+              oq[r * nx] = Cells2<T>::back(v.x);
+              if (wide) oq[r * nx + 1] = Cells2<T>::back(v.y);
+            }
+          }
       oq += plane;
     }
     ++k;
@@ -228,10 +250,10 @@ __device__ __forceinline__ SweepTile tile_of(const SweepPlan& P, int nx, int ny,
   t.ly = max(0, t.y0 - SW_HALO);
   return t;
 }
-template <typename T, bool kZero, bool kRelax>
+template <typename T, bool kZero, bool kRelax, bool kOdd = false>
 __global__ void __launch_bounds__(SW_THREADS, 1) k_sweep2(const T* __restrict__ p, const T* __restrict__ b, T* __restrict__ out, int nx, int ny,
                                                           int nz, float h, float omega, SweepPlan P) {
-  sweep2_body<T, kZero, kRelax>(p, b, out, nx, ny, nz, h, omega, P.px, P.ty, tile_of(P, nx, ny, nz, blockIdx.x));
+  sweep2_body<T, kZero, kRelax, kOdd>(p, b, out, nx, ny, nz, h, omega, P.px, P.ty, tile_of(P, nx, ny, nz, blockIdx.x));
 }
 
 // Measured (GB300, ensemble of 16 grids from 32x64x32 to 96x192x96, 4 cycles): 16 launches per level and cycle of batched colour
@@ -264,13 +286,13 @@ constexpr double SW_STEP = 300.0, SW_WARP = 30.0, SW_START = 1500.0;
 SweepPlan plan_sweep(const MGLevel& L, int sms, int block) {
   const int nx = L.nx, ny = L.ny, nz = L.nz;
   SweepPlan best{};
-  if (L.study || nx % 2 || nx < 8 || ny < 4 || nz < 4) return best;   // odd rows have no aligned pairs: colour launches
+  if (L.study || nx < 8 || ny < 4 || nz < 4) return best;
   double cost = 1e30;
   auto even = [](int v) { return (v + 1) & ~1; };
   for (int ntx = 1; ntx <= 16; ++ntx) {
     const int cx = even((nx + ntx - 1) / ntx);
     if ((nx + cx - 1) / cx != ntx || (cx < 16 && ntx > 1)) continue;
-    const int px = std::min(nx, cx + SW_HALO * std::min(ntx - 1, 2)) / 2;
+    const int px = (std::min(nx, cx + SW_HALO * std::min(ntx - 1, 2)) + 1) / 2;
     for (int nty = 1; nty <= 128; ++nty) {
       const int cy = even((ny + nty - 1) / nty);
       if (cy < 8 && nty > 1) break;
@@ -305,6 +327,11 @@ cudaError_t launch_sweep2_t(const T* p, const T* b, T* out, const SweepPlan& P, 
   const dim3 grid(P.ntx * P.nty * P.ntz), block(sweep_threads(P));
   const size_t smem = sweep_smem(P, (int)block.x);
   auto go = [&](auto kernel) { return launch_pdl(kernel, grid, block, smem, st, p, b, out, nx, ny, nz, h, omega, P); };
+  if (nx % 2) {
+    if constexpr (sizeof(T) != sizeof(float)) return cudaErrorInvalidValue;   // 16-bit rows of an odd length: colour launches
+    else if (omega == 1.0f) return zero ? go(k_sweep2<T, true, false, true>) : go(k_sweep2<T, false, false, true>);
+    else return zero ? go(k_sweep2<T, true, true, true>) : go(k_sweep2<T, false, true, true>);
+  }
   if (omega == 1.0f) return zero ? go(k_sweep2<T, true, false>) : go(k_sweep2<T, false, false>);
   if constexpr (sizeof(T) != sizeof(float)) return cudaErrorInvalidValue;   // the refinement's sweeps are Gauss-Seidel
   else return zero ? go(k_sweep2<T, true, true>) : go(k_sweep2<T, false, true>);
@@ -372,6 +399,10 @@ cudaError_t sweep_configure() {
   opt_in(k_sweep2<float, true, false>);
   opt_in(k_sweep2<float, false, true>);
   opt_in(k_sweep2<float, true, true>);
+  opt_in(k_sweep2<float, false, false, true>);
+  opt_in(k_sweep2<float, true, false, true>);
+  opt_in(k_sweep2<float, false, true, true>);
+  opt_in(k_sweep2<float, true, true, true>);
   opt_in(k_sweep2_b<false>);
   opt_in(k_sweep2_b<true>);
   opt_in(k_sweep2<__half, false, false>);

@@ -36,10 +36,11 @@ def test_cycle_matches_colour_launches(res, omega):
     b.close()
 
 
-@pytest.mark.parametrize("res", [(120, 101, 90), (150, 100, 77)])
+@pytest.mark.parametrize("res", [(120, 101, 90), (150, 100, 77), (101, 90, 95), (151, 103, 64)])
 def test_single_large_level_matches_colour_launches(res):
     """A grid without coarser levels and too large for the on-chip kernel: all its sweeps are two-sweep launches, in place by
-    pairs, with the odd remainder by colour; an odd row count leaves a thread row with one row in the domain."""
+    pairs, with the odd remainder by colour; an odd row count leaves a thread row with one row in the domain.  An odd row length leaves a pair
+    with one column, and pairs that are not aligned."""
     a, b = C._sim(res, 1.0), C._sim(res, 1.0)
     a.run_stage("vcycle", 0.01)
     b.run_mg("sweeps", 0, a.info().coarse_iters)
