@@ -420,7 +420,7 @@ def run_ensemble(dev: int, steps: int = 20):
             "tiles": {"stages": ["adv1", "adv2", "forces", "div", "project"],
                       "chosen": tuned[0].tolist() if tuned else None,
                       "candidate_ms": tuned[1].round(5).tolist() if tuned else None,
-                      "cell_tiles": ["32x4x2", "32x8x1", "32x2x4", "64x4x1"], "forces_depths": [16, 8, 32],
+                      "cell_tiles": ["32x4x2", "32x8x1", "32x2x4", "64x4x1"], "forces_tiles": ["32x4x2", "32x8x1", "32x2x4"],
                       "ms_per_step_untuned_tiles": ms_untuned}}
 
 
