@@ -305,7 +305,7 @@ int fire_poisson_noalloc_status(void* stream);
 /* ---- ensembles of independent simulations ------------------------------------------------------
  * n (<= 64) simulations of possibly different grids advanced together: each stage of a step is one
  * kernel launch over all members, the multigrid levels are batched level by level and the members'
- * shared-memory tails run in one launch per tail form, all captured in one CUDA graph per step.  The
+ * on-chip coarse ends run in one launch per form, all captured in one CUDA graph per step.  The
  * members are FireSim handles owned by the ensemble: configure them (params, spots, soot age, events) and
  * read them (fields, stats) with the fire_sim_* functions, but step them only through the ensemble and do
  * not destroy them.  Every member must use fixed V-cycles (mg_max_cycles = 0) with the same count, the

@@ -491,7 +491,7 @@ int fire_sim_create(const FireConfig* cfg, const float* logs, int n_logs, FireSi
       cudaEventCreateWithFlags(&sim->forkEv, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&sim->joinEv, cudaEventDisableTiming) != cudaSuccess)
     return fail(FIRE_ERR_CUDA);
-  if (mg_configure(TAIL_SMEM_BUDGET) != cudaSuccess || coarse_configure() != cudaSuccess || sweep_configure() != cudaSuccess) return fail(set_err(sim, FIRE_ERR_CUDA, "tail kernel smem opt-in failed"));
+  if (mg_configure(TAIL_SMEM_BUDGET) != cudaSuccess || coarse_configure() != cudaSuccess || sweep_configure() != cudaSuccess) return fail(set_err(sim, FIRE_ERR_CUDA, "multigrid kernels' shared-memory opt-in failed"));
 
   // zero state (reset semantics), bake the tables (src/noise.js), upload logs
   cudaStream_t st = sim->capStream;

@@ -6,12 +6,12 @@
 // update, exactly as mgSmooth does.
 //
 // GB300 mapping:
-//  * the fine levels run one launch per colour sweep, restriction and prolongation on 3D grids of
-//    32 x 4 x 2 CTAs (32-bit index arithmetic, no integer division); at 128x256x128 the level-0 arrays
-//    (p and b, 33.5 MB) stay resident in the 129 MB L2 across the cycle;
-//  * every level small enough to fit, with all coarser ones, in one CTA's shared memory is solved by a
-//    single-CTA kernel that runs the rest of the V-cycle out of shared memory; levels of <= 256 cells
-//    inside it run on one warp with __syncwarp, so the coarsest sweeps cost no CTA-wide barriers;
+//  * the fine levels take two sweeps per pass (fire_sweep.cu) and one launch per transfer (fire_level.cuh); the kernels of one
+//    colour sweep here serve the levels those do not take, the convergence studies and the allocation-free solve, on
+//    3D grids of 32 x 4 x 2 CTAs (32-bit index arithmetic, no integer division);
+//  * the levels below run in one launch on chip (fire_coarse.cu).  The tail kernels here, out of shared memory that
+//    bulk copies fill, serve what that does not take: the studies' variant, FP64 coarsest sweeps, coarsest levels that
+//    fit no cluster's registers;
 //  * every kernel uses programmatic dependent launch (fire_launch.cuh) so consecutive launches overlap.
 #include <algorithm>
 #include <cstring>

@@ -3,7 +3,7 @@
 //
 // Mixed-precision form (FIRE_POISSON_FP16 / FIRE_POISSON_BF16):
 //   x, b and every residual are FP32; the correction equation A e = r is solved approximately by V(2,2)
-//   cycles whose level arrays (p and b of every level above the shared-memory tail) are stored in IEEE half
+//   cycles whose level arrays (p and b of every level above the on-chip coarse end) are stored in IEEE half
 //   or bfloat16, with all arithmetic in FP32 registers.  Halving the bytes of the fine levels is the point:
 //   at 256x512x256 the level-0 arrays of the FP32 form (268 MB) do not fit the 129 MB L2 and every sweep is
 //   HBM-bound.  The residual handed to the correction solve is scaled by 1/RMS of the previous residual, so
