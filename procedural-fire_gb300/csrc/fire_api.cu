@@ -440,7 +440,6 @@ int fire_sim_create(const FireConfig* cfg, const float* logs, int n_logs, FireSi
     size_t c = (size_t)sim->levels[l].nx * sim->levels[l].ny * sim->levels[l].nz;
     pOff[l] = off; off = align_up(off + c * sizeof(float));
     bOff[l] = off; off = align_up(off + c * sizeof(float));
-    if (sim->levels[l].sweep.px > 0) { p2Off[l] = off; off = align_up(off + c * sizeof(float)); }
   }
   const size_t tabBytes = (size_t)TABLE_N * TABLE_N * TABLE_N * sizeof(uint2);
   size_t solidOff = off; off = align_up(off + cells);
@@ -453,8 +452,18 @@ int fire_sim_create(const FireConfig* cfg, const float* logs, int n_logs, FireSi
   size_t diagPartOff = off; off = align_up(off + sizeof(double) * 16 * (size_t)stats_partials_count(sim->d));
   size_t smallOff = off; off = align_up(off + sizeof(double) * 48);
   size_t cntOff = off; off = align_up(off + sizeof(int) * 4);
-  sim->arenaBytes = off;
+  // last, the second pressure arrays of the two-sweep kernel: where only they do not fit, the levels take colour launches
+  const size_t without = off;
+  for (size_t l = 0; l < sim->levels.size(); ++l)
+    if (sim->levels[l].sweep.px > 0) { p2Off[l] = off; off = align_up(off + (size_t)sim->levels[l].nx * sim->levels[l].ny * sim->levels[l].nz * sizeof(float)); }
   cudaError_t e = cudaMalloc(&sim->arena, off);
+  if (e != cudaSuccess && off > without) {
+    cudaGetLastError();
+    for (MGLevel& L : sim->levels) L.sweep = SweepPlan{};
+    off = without;
+    e = cudaMalloc(&sim->arena, off);
+  }
+  sim->arenaBytes = off;
   if (e != cudaSuccess) { delete sim; return FIRE_ERR_OOM; }
   char* A = (char*)sim->arena;
   float4** fp[11] = {&sim->f.vel, &sim->f.velX, &sim->f.velY, &sim->f.S, &sim->f.SX, &sim->f.SY,

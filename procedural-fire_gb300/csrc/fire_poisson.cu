@@ -19,7 +19,7 @@
 // storage type where a colour launch would have stored it), marched transfers (fire_level.cuh), the coarse kernel.  All
 // levels are in the plain layout: with one pass per two sweeps a red-black split saves no bytes, and plain pairs serve every
 // kernel.  Measured (GB300, whole solves, colour launches on a split level 0 -> this): 256x512x256 with FP32 storage 7.20 ->
-// 4.98 ms, 128x256x128 with half 1.38 -> 1.06 ms; FP32 form at 64x128x64 296 -> 283 us.
+// 4.81 ms, 128x256x128 with half 1.38 -> 1.05 ms; FP32 form at 64x64x64 296 -> 280 us.
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
 #include <cmath>
@@ -804,7 +804,6 @@ int fire_poisson_create(const int res[3], float h, int precision, int device, Fi
     // (not of 16-bit rows of an odd length)
     if (l < ps->tailFirst && (L.sto == STO_F32 || M.nx % 2 == 0)) L.sweep = ps->mg[l].sweep = plan_sweep(ps->mg[l]);
     const size_t bytes = align_up((size_t)M.nx * M.ny * M.nz * elem_bytes(L.sto));
-    if (L.sweep.px > 0) { p2Off[l] = off; off += bytes; }
     if (l == 0 && !ps->ir) { pOff[l] = bOff[l] = (size_t)-1; continue; }
     pOff[l] = off; off += bytes;
     bOff[l] = off; off += bytes;
@@ -821,7 +820,21 @@ int fire_poisson_create(const int res[3], float h, int precision, int device, Fi
   const size_t srcOff = off; off = align_up(off + sizeof(float) * MAX_SOURCES * 5);
   const size_t loOff = off; if (ps->ir) off = align_up(off + sizeof(float) * (size_t)ps->cells);
   const size_t cinvOff = off; if (direct) off = align_up(off + sizeof(double) * cinv.size());
-  if (cudaMalloc(&ps->arena, off) != cudaSuccess) { delete ps; return FIRE_ERR_OOM; }
+  // last, the second pressure arrays of the two-sweep kernel: where only they do not fit, the levels take colour launches
+  const size_t without = off;
+  for (int l = 0; l < n; ++l)
+    if (ps->levels[l].sweep.px > 0) {
+      p2Off[l] = off;
+      off += align_up((size_t)ps->mg[l].nx * ps->mg[l].ny * ps->mg[l].nz * elem_bytes(ps->levels[l].sto));
+    }
+  cudaError_t got = cudaMalloc(&ps->arena, off);
+  if (got != cudaSuccess && off > without) {
+    cudaGetLastError();
+    for (int l = 0; l < n; ++l) ps->levels[l].sweep = ps->mg[l].sweep = SweepPlan{};
+    off = without;
+    got = cudaMalloc(&ps->arena, off);
+  }
+  if (got != cudaSuccess) { delete ps; return FIRE_ERR_OOM; }
   char* A = (char*)ps->arena;
   for (int l = 0; l < n; ++l) {
     if (ps->levels[l].sweep.px > 0) {
