@@ -16,7 +16,7 @@
 // result is bit-identical to the four launches.
 //
 // Measured (GB300, two sweeps back to back, us, four colour launches -> this): 64x128x64 8.6 -> 6.5, 80x120x80 13.2 -> 7.4,
-// 96x192x96 19.0 -> 10.7, 128x256x128 28.0 -> 18.3, 256x512x256 270 -> 120 (402 MB there: 3.4 TB/s).  A step costs 0.3-0.5 us
+// 96x192x96 19.0 -> 10.7, 128x256x128 28.0 -> 18.3, 256x512x256 270 -> 111 (402 MB there: 3.6 TB/s).  A step costs 0.3-0.5 us
 // whatever the tile: about 130 instructions a warp behind a chain of reads, four dependent updates, a write and a barrier;
 // registers and the halo keep it to one or two CTAs an SM.
 // Grids without coarser levels (an odd side) run all their sweeps here; rows of an odd length copy their cells one by one.  Steps of two
@@ -279,14 +279,19 @@ size_t sweep_smem(const SweepPlan& P, int threads) {
 
 }  // namespace
 
-// The cut that costs least by a model of the kernel: a step of a resident set of CTAs takes the larger of SW_STEP cycles (one
+// The cut that costs least by a model of the kernel: a step of a resident set of CTAs takes the larger of a step's least (one
 // warp's chain of four updates, the shared-memory reads and the barrier) and SW_WARP cycles per resident warp (its instructions
-// on one of four schedulers); a CTA runs its planes and eight more, and about SW_START cycles around them.
-constexpr double SW_STEP = 300.0, SW_WARP = 30.0, SW_START = 1500.0;
+// on one of four schedulers); a CTA runs its planes and eight more, and about SW_START cycles around them.  On levels of
+// SW_LARGE_CELLS and more a step takes SW_ADD besides, and 6 % more where a row of pairs ends inside eight lanes: fitted to 9638
+// plans of ten levels, the choice is within 3.5 % of the fastest everywhere (256x512x256: 111 us, 124 without).  On small levels
+// those terms choose narrower rows, as fast back to back but slower in whole solves (64x64x64 and 50x98x50 2 %, 128x256x128 0.3 %).
+constexpr double SW_STEP = 300.0, SW_STEP_LARGE = 200.0, SW_ADD = 200.0, SW_WARP = 30.0, SW_START = 1500.0;
+constexpr long SW_LARGE_CELLS = 5000000;
 SweepPlan plan_sweep(const MGLevel& L, int sms, int block) {
   const int nx = L.nx, ny = L.ny, nz = L.nz;
   SweepPlan best{};
   if (L.study || nx < 8 || ny < 4 || nz < 4) return best;
+  const bool large = (long)nx * ny * nz >= SW_LARGE_CELLS;
   double cost = 1e30;
   auto even = [](int v) { return (v + 1) & ~1; };
   for (int ntx = 1; ntx <= 16; ++ntx) {
@@ -311,7 +316,8 @@ SweepPlan plan_sweep(const MGLevel& L, int sms, int block) {
         last = ntz;
         const long ctas = (long)ntx * nty * ntz, w = (ctas + (long)sms * occ - 1) / ((long)sms * occ);
         const int resident = (int)std::min<long>(occ, (ctas + sms - 1) / sms);
-        const double step = std::max(SW_STEP, SW_WARP * resident * threads / 32.0);
+        const double warps = SW_WARP * resident * threads / 32.0;
+        const double step = large ? (SW_ADD + std::max(SW_STEP_LARGE, warps)) * (px % 8 ? 1.06 : 1.0) : std::max(SW_STEP, warps);
         const double c = w * ((std::min(nz, cz + SW_HALO * std::min(ntz, 2)) + 1) * step + SW_START);
         if (c < cost) { cost = c; best = P; best.ntz = ntz; best.cz = cz; }
       }
