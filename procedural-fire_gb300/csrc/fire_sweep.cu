@@ -258,8 +258,10 @@ __global__ void __launch_bounds__(SW_THREADS, 1) k_sweep2(const T* __restrict__ 
 
 // Measured (GB300, ensemble of 16 grids from 32x64x32 to 96x192x96, 4 cycles): 16 launches per level and cycle of batched colour
 // sweeps, 1245 us of a step's 2978, became 4 and the step takes 2486; CTAs of 256 or 448 threads give the same within 1 %.
+// With both bodies (omega 1 and not) in one kernel 160 bytes of registers spilled: a step 2244, with one body 2032.
 // A level of every simulation of a batch: down from p (kZero: from zero) into p2, else back from p2 into p.
-template <bool kZero>
+// kMixed: some member's omega is not 1 (a second body, which costs registers).
+template <bool kZero, bool kMixed>
 __global__ void __launch_bounds__(SW_THREADS, 1) k_sweep2_b(const __grid_constant__ BatchMap m, const __grid_constant__ LevelBatch L, int down) {
   uint3 blk; int i;
   batch_locate(m, blk, i);
@@ -267,7 +269,7 @@ __global__ void __launch_bounds__(SW_THREADS, 1) k_sweep2_b(const __grid_constan
   const SweepTile t = tile_of(v.sweep, v.nx, v.ny, v.nz, blk.x);
   const float* p = down ? v.p : v.p2;
   float* out = down ? v.p2 : v.p;
-  if (v.omega == 1.0f) sweep2_body<float, kZero, false>(p, v.b, out, v.nx, v.ny, v.nz, v.h, v.omega, v.sweep.px, v.sweep.ty, t);
+  if (!kMixed || v.omega == 1.0f) sweep2_body<float, kZero, false>(p, v.b, out, v.nx, v.ny, v.nz, v.h, v.omega, v.sweep.px, v.sweep.ty, t);
   else sweep2_body<float, kZero, true>(p, v.b, out, v.nx, v.ny, v.nz, v.h, v.omega, v.sweep.px, v.sweep.ty, t);
 }
 
@@ -349,7 +351,10 @@ cudaError_t launch_sweep2(const MGLevel& L, const float* p, float* out, bool zer
 cudaError_t launch_sweep2_batch(const BatchMap& m, const LevelBatch& L, bool down, bool zero, cudaStream_t st) {
   size_t smem = 0;
   for (int k = 0; k < m.n; ++k) smem = std::max(smem, sweep_smem(L.l[m.inst[k]].sweep, SW_BATCH_THREADS));
-  return launch_pdl(zero ? k_sweep2_b<true> : k_sweep2_b<false>, dim3(m.prefix[m.n]), dim3(SW_BATCH_THREADS), smem, st, m, L, (int)down);
+  bool mixed = false;
+  for (int k = 0; k < m.n; ++k) mixed = mixed || L.l[m.inst[k]].omega != 1.0f;
+  return launch_pdl(mixed ? (zero ? k_sweep2_b<true, true> : k_sweep2_b<false, true>) : zero ? k_sweep2_b<true, false> : k_sweep2_b<false, false>,
+                    dim3(m.prefix[m.n]), dim3(SW_BATCH_THREADS), smem, st, m, L, (int)down);
 }
 
 template cudaError_t launch_sweep2_t<float>(const float*, const float*, float*, const SweepPlan&, int, int, int, float, float, bool, cudaStream_t);
@@ -409,8 +414,10 @@ cudaError_t sweep_configure() {
   opt_in(k_sweep2<float, true, false, true>);
   opt_in(k_sweep2<float, false, true, true>);
   opt_in(k_sweep2<float, true, true, true>);
-  opt_in(k_sweep2_b<false>);
-  opt_in(k_sweep2_b<true>);
+  opt_in(k_sweep2_b<false, false>);
+  opt_in(k_sweep2_b<true, false>);
+  opt_in(k_sweep2_b<false, true>);
+  opt_in(k_sweep2_b<true, true>);
   opt_in(k_sweep2<__half, false, false>);
   opt_in(k_sweep2<__half, true, false>);
   opt_in(k_sweep2<__nv_bfloat16, false, false>);

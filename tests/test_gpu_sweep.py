@@ -71,10 +71,13 @@ def test_refinement_forms_reach_the_tolerance(precision, res):
     ps.close()
 
 
-def test_batched_sweeps_match_members_alone():
+@pytest.mark.parametrize("mixed", [False, True])
+def test_batched_sweeps_match_members_alone(mixed):
     """Members of very different sizes share each batched two-sweep launch (tiles cut for a share of the SMs), one whose
     second level only it has outside its coarse end: after the first step from rest their
-    pressures equal those of the same simulations stepped alone (same operations, same order)."""
+    pressures equal those of the same simulations stepped alone (same operations, same order).  mixed: one member's launched
+    levels are over-relaxed (its coarse end is not, as descriptors are made at creation), which another kernel serves; the
+    others' pressures are still their own."""
     import fire_sim as F
     import test_gpu_ensemble as E
     members = [dict(res=r, size=tuple(0.0125 * k for k in r), seed=20 + i, spots=4)
@@ -84,13 +87,19 @@ def test_batched_sweeps_match_members_alone():
     for k, m in enumerate(members):
         for s in (ens.members[k], alone[k]):
             E._configure(s, m)
+    if mixed:
+        ens.members[1].set_mg_omega(1.2)
     ens.step(E.DT, 1)
     ens.sync()
-    for a, b in zip(ens.members, alone):
+    for k, (a, b) in enumerate(zip(ens.members, alone)):
         b.step(E.DT, 1)
         b.sync()
-        assert float(np.abs(b.level(0, "p")).max()) > 0.0
-        np.testing.assert_array_equal(a.level(0, "p"), b.level(0, "p"))
+        pa, pb = a.level(0, "p"), b.level(0, "p")
+        assert float(np.abs(pb).max()) > 0.0
+        if mixed and k == 1:   # two cycles of either smoother leave a few percent of the solution's error
+            assert (pa != pb).any() and FC.rel_l2(pa, pb) < 0.2
+        else:
+            np.testing.assert_array_equal(pa, pb)
         b.close()
     ens.close()
 
