@@ -472,7 +472,8 @@ int fire_sim_create(const FireConfig* cfg, const float* logs, int n_logs, FireSi
   for (size_t l = 0; l < sim->levels.size(); ++l) {
     sim->levels[l].p = (float*)(A + pOff[l]);
     sim->levels[l].b = (float*)(A + bOff[l]);
-    if (sim->levels[l].sweep.px > 0) sim->levels[l].p2 = (float*)(A + p2Off[l]);
+    if (sim->levels[l].sweep.px > 0) sim->levels[l].p2 = (float*)(A + p2Off[l]);   // an ensemble's batches use every one
+    if (!sweep_pays(sim->levels[l], l + 1 == sim->levels.size())) sim->levels[l].sweep = SweepPlan{};
   }
   sim->noise = (uint2*)(A + noiseOff);
   sim->curl = (uint2*)(A + curlOff);

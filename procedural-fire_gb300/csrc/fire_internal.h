@@ -150,6 +150,7 @@ void launch_project_batch(const BatchMap& m, const StepBatch& I, int tile, int d
 // Two red-black sweeps from p (zero: from zero) into out; bit-identical to the four colour launches.
 // sms: the SMs the level may count on; block: threads of a CTA (0: as many as the tile has).
 SweepPlan plan_sweep(const MGLevel& L, int sms = 152, int block = 0);
+bool sweep_pays(const MGLevel& L, bool coarsest);
 cudaError_t launch_sweep2(const MGLevel& L, const float* p, float* out, bool zero, cudaStream_t st);
 // The same on a level's arrays in storage T (float, __half, __nv_bfloat16; omega 1 for the last two).
 template <typename T>

@@ -802,7 +802,7 @@ int fire_poisson_create(const int res[3], float h, int precision, int device, Fi
     L.sto = (ps->ir && l < ps->tailFirst) ? sto : STO_F32;
     // every level that launches smooth: all above the coarse end, and the coarsest itself where none takes it
     // (not of 16-bit rows of an odd length)
-    if (l < ps->tailFirst && (L.sto == STO_F32 || M.nx % 2 == 0)) L.sweep = ps->mg[l].sweep = plan_sweep(ps->mg[l]);
+    if (l < ps->tailFirst && (L.sto == STO_F32 || M.nx % 2 == 0) && sweep_pays(M, l == n - 1)) L.sweep = ps->mg[l].sweep = plan_sweep(ps->mg[l]);
     const size_t bytes = align_up((size_t)M.nx * M.ny * M.nz * elem_bytes(L.sto));
     if (l == 0 && !ps->ir) { pOff[l] = bOff[l] = (size_t)-1; continue; }
     pOff[l] = off; off += bytes;

@@ -328,6 +328,13 @@ SweepPlan plan_sweep(const MGLevel& L, int sms, int block) {
   return best;
 }
 
+// Where a launch of this kernel is faster than the four colour launches it replaces, from whole-level times (GB300, us, this against
+// four): odd rows 61x111x57 8.5 / 7.2, 71x131x67 8.3 / 12.5; a coarsest level (odd in y or z) 50x91x49 6.9 / 6.6, 56x101x60 5.8 /
+// 7.3; a level with coarser ones 42x84x42 7.0 / 6.3, 46x92x44 5.9 / 6.4.  (In a batch all members' levels share the launch.)
+bool sweep_pays(const MGLevel& L, bool coarsest) {
+  return (long)L.nx * L.ny * L.nz >= (L.nx % 2 ? 500000 : coarsest ? 280000 : 150000);
+}
+
 template <typename T>
 cudaError_t launch_sweep2_t(const T* p, const T* b, T* out, const SweepPlan& P, int nx, int ny, int nz, float h, float omega, bool zero,
                             cudaStream_t st) {
