@@ -19,7 +19,7 @@
 // storage type where a colour launch would have stored it), marched transfers (fire_level.cuh), the coarse kernel.  All
 // levels are in the plain layout: with one pass per two sweeps a red-black split saves no bytes, and plain pairs serve every
 // kernel.  Measured (GB300, whole solves, colour launches on a split level 0 -> this): 256x512x256 with FP32 storage 7.20 ->
-// 4.81 ms, 128x256x128 with half 1.38 -> 1.05 ms; FP32 form at 64x64x64 296 -> 280 us.
+// 4.67 ms, 128x256x128 with half 1.38 -> 1.04 ms; FP32 form at 64x64x64 296 -> 285 us.
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
 #include <cmath>
