@@ -180,11 +180,12 @@ def launches_per_step(sim, cycles_per_step: float) -> float:
     """Kernels launched per step by the captured graph: 5 stencil kernels (the divergence kernel also clears
     the solve's cycle count), and per V-cycle 4 per level above the coarse kernel (two sweeps in one launch before and after,
     restriction, prolongation), the coarse kernel, the residual norm and the decision kernel.  The coarse kernel takes the
-    levels whose half-row x z columns, times their groups of four rows per CTA of a 16-CTA cluster, fit 1024 threads."""
+    levels whose half-row x z columns, times their groups of four rows per CTA of a 16-CTA cluster, fit 512 threads (1024 for
+    the finest and the coarsest level)."""
     T = len(sim.levels)
     while T > 0:
         nx, ny, nz = sim.levels[T - 1]["dims"]
-        if (nx + 1) // 2 * nz * ((ny + 63) // 64) > 1024:
+        if (nx + 1) // 2 * nz * ((ny + 63) // 64) > (1024 if T in (1, len(sim.levels)) else 512):
             break
         T -= 1
     top = min(T, len(sim.levels) - 1)

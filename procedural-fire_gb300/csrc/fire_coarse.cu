@@ -25,7 +25,7 @@
 // Measured (GB300, back to back, us; the forms this replaces: one launch per phase, the single-CTA or 8-CTA tail):
 //   one V(2,2) cycle from 32x64x32            21.2   (46: level 0 in launches, tail from 16x32x16)
 //   four cycles of it in one launch           73.6   (186)
-//   one cycle from 40x60x40, 43 coarse sweeps 42.3   (66)
+//   one cycle from 20x30x20, 43 coarse sweeps 24.3; with 40x60x40 on top 42.3 (66): that level runs in launches, see coarse_first
 //   64 sweeps of a 25x49x25 coarsest level    59.6   (190: two launches a sweep)
 // A phase costs about 0.15 us on one CTA (LDS - six adds - store - barrier) and 0.3 us on a split level, of which half is
 // the neighbours' rows in flight; nothing here is near a byte or FLOP limit.
@@ -947,7 +947,9 @@ int coarse_first(const MGLevel* levels, int n, bool direct) {
   CoDesc D;
   size_t smem;
   int threads, first = n;
-  while (first > 0 && make_plan(levels, first - 1, n, direct, D, smem, threads)) --first;
+  // A level that needs more than 512 threads a CTA leaves a thread too few registers: 40x60x40 on top of 20x30x20 costs 18 us a
+  // cycle here and 14 in launches.  Where it is the finest level, one launch for all cycles outweighs that.
+  while (first > 0 && make_plan(levels, first - 1, n, direct, D, smem, threads) && (threads <= CO_THREADS[0] || first == 1 || first == n)) --first;
   return first;
 }
 cudaError_t launch_coarse(const MGLevel* levels, int first, int n, int pre, int post, int coarse, const double* cinv, int cycles,
