@@ -648,7 +648,8 @@ __device__ __forceinline__ void prolong_level(Own<K>& o, const Slab& L, const Co
 }
 
 // Exact coarsest solve in FP64, p = A^-1 b: 1024 / n column chunks per row, their partial sums added in order (the
-// arithmetic of tail_direct_fp64_cta in fire_mg.cu, whatever the thread count).
+// arithmetic of tail_direct_fp64_cta in fire_mg.cu, whatever the thread count).  A hierarchy of this one level (5x5x5, 6x12x6) has
+// its right-hand side and its result in global memory.
 __device__ __noinline__ void coarsest_direct(const CoDesc& D, int tid, int nthreads) {
   const int l = D.n - 1, k4 = D.l[l].k == 4;
   const Slab L = co_slab[l];
@@ -658,8 +659,9 @@ __device__ __noinline__ void coarsest_direct(const CoDesc& D, int tid, int nthre
   float* b = co_smem() + D.dsum + 2 * 1024;
   for (int t = tid; t < n; t += nthreads) {
     const int x = t % L.nx, q = t / L.nx, y = q % L.ny, z = q / L.ny, c = (x + y + z) & 1, col = (x >> 1) + L.hx * z;
-    b[t] = plain ? co_smem()[D.gather + x + L.nx * (z + L.nz * y)]
-                 : sm_at(L.B)[k4 ? 4 * (c * L.items + col + L.n * (y >> 2)) + row_slot(y & 3) : c * L.items + col + L.n * y];
+    b[t] = l == 0  ? D.gb[t]
+           : plain ? co_smem()[D.gather + x + L.nx * (z + L.nz * y)]
+                   : sm_at(L.B)[k4 ? 4 * (c * L.items + col + L.n * (y >> 2)) + row_slot(y & 3) : c * L.items + col + L.n * y];
   }
   team_sync(L.bar, L.team);
   for (int t = tid; t < n * chunks; t += nthreads) {
@@ -680,6 +682,7 @@ __device__ __noinline__ void coarsest_direct(const CoDesc& D, int tid, int nthre
     const int x = t % L.nx, q = t / L.nx, y = q % L.ny, z = q / L.ny, c = (x + y + z) & 1, col = (x >> 1) + L.hx * (z + 1);
     sm_at(L.P)[k4 ? 4 * (c * L.arr + col + L.plane * ((y >> 2) + 1)) + row_slot(y & 3) : c * L.arr + col + L.plane * (y + 1)] = (float)s;
     if (l > 0) co_smem()[L.plain + x + L.nx * (z + L.nz * y)] = (float)s;
+    else D.gp[t] = (float)s;
   }
   team_sync(L.bar, L.team);
 }
