@@ -169,12 +169,13 @@ int fire_sim_set_spots(FireSim* sim, const float* spots, int n);
  * needs (no counterpart in the reference).                                                            */
 int fire_sim_set_mg_omega(FireSim* sim, float omega);
 /* Fault-injection hook for the device-side bounded wait (no counterpart in the reference, which logs
- * WebGPU device loss, src/gpu.js:25-26).  A value other than the default runs the multigrid's coarse end in its
- * TMA-staged tail kernels (the same bits): the single-CTA one waits for the TMA bulk copies that
- * stage its first level into shared memory for at most `polls` polls (default 4194304, and about a second)
- * before it records a timeout, waits again at the full bound for the copies in flight and returns without
- * running the cycle; fire_sim_sync then reports FIRE_ERR_CUDA ("a device-side wait timed out") and clears
- * the flag.  0 makes the first wait give up at once, so a test can exercise that path on a healthy GPU.   */
+ * WebGPU device loss, src/gpu.js:25-26): bounds the waits of the multigrid's coarse end, which runs on a
+ * cluster of CTAs that send each other rows, to `polls` polls (default 4194304, and about a second).  A wait
+ * that runs out is recorded; the kernel leaves the cycle unfinished and ends once rows still in flight have had
+ * time to land (50 ms).  fire_sim_sync then reports FIRE_ERR_CUDA ("a device-side wait timed out") and
+ * clears the flag.  0 makes the first wait give up at once, so a test can exercise that path on a healthy GPU.
+ * A coarse end small enough for one CTA waits for no rows; with a value other than the default it runs in
+ * a kernel that stages its first level with TMA bulk copies (the same bits) and bounds the wait for those.  */
 int fire_sim_set_tail_wait_limit(FireSim* sim, int polls);
 
 /* ---- events (src/main.js:401-407, 456-461; src/timeline.js:126-157) ---------------------------- */

@@ -189,17 +189,20 @@ void record_smooth(FireSim* s, int l, int iters, cudaStream_t st) {
     launch_smooth(s->levels[l], 1, st);
   }
 }
-// Whether the coarse levels run in the register-resident coarse kernel; the TMA-staged tail takes over when nothing fits
-// it, and while its wait limit is lowered (fire_sim_set_tail_wait_limit exercises that kernel's bounded wait).
-bool use_coarse(const FireSim* s) { return s->coarseFirst < (int)s->levels.size() && s->tailWaitPolls == TAIL_WAIT_POLLS; }
+// Whether the coarse levels from `first` on run in the register-resident coarse kernel; the TMA-staged tail takes over when nothing
+// fits it, and while the wait limit is lowered and the coarse kernel, on one CTA, has no wait that it could bound.
+bool use_coarse(const FireSim* s, int first) {
+  const int n = (int)s->levels.size();
+  return coarse_fits(s->levels.data(), first, n) && (s->tailWaitPolls == TAIL_WAIT_POLLS || coarse_waits(s->levels.data(), first, n));
+}
 // One V(2,2) cycle (src/sim.js:588-599).  Levels [T, n) run inside one launch.
 void record_vcycle(FireSim* s, cudaStream_t st) {
   const int n = (int)s->levels.size();
-  const bool co = use_coarse(s);
+  const bool co = use_coarse(s, s->coarseFirst);
   const int T = co ? s->coarseFirst : s->tailFirst;
   const int top = std::min(T, n - 1);
   launch_down(s->levels.data(), top, st);
-  if (co) launch_coarse(s->levels.data(), T, n, 2, 2, s->coarseIters, nullptr, 1, s->dCounter + 2, st);
+  if (co) launch_coarse(s->levels.data(), T, n, 2, 2, s->coarseIters, nullptr, 1, s->dCounter + 2, st, s->tailWaitPolls);
   else if (T < n) launch_tail(s->levels.data(), T, n, 2, 2, s->coarseIters, s->dCounter + 2, st, false, nullptr, s->tailWaitPolls);
   else launch_sweeps(s->levels[n - 1], s->coarseIters, st);
   launch_up(s->levels.data(), top, st);
@@ -216,9 +219,10 @@ int record_ev(FireSim* sim, int idx, cudaStream_t st, bool prof) {
 // count (launch_div with the counter), else a clearing kernel is recorded here.
 int record_mg(FireSim* sim, cudaStream_t st, bool counter_cleared) {
   if (sim->mg_max_cycles <= 0) {
-    if (use_coarse(sim) && sim->coarseFirst == 0) {   // the whole hierarchy is on chip: every cycle in one launch
+    if (sim->coarseFirst == 0 && use_coarse(sim, 0)) {   // the whole hierarchy is on chip: every cycle in one launch
       if (sim->vcycles > 0)
-        launch_coarse(sim->levels.data(), 0, (int)sim->levels.size(), 2, 2, sim->coarseIters, nullptr, sim->vcycles, sim->dCounter + 2, st);
+        launch_coarse(sim->levels.data(), 0, (int)sim->levels.size(), 2, 2, sim->coarseIters, nullptr, sim->vcycles, sim->dCounter + 2, st,
+                      sim->tailWaitPolls);
       return FIRE_OK;
     }
     for (int c = 0; c < sim->vcycles; ++c) record_vcycle(sim, st);
@@ -574,7 +578,7 @@ int fire_sim_sync(FireSim* sim) {
   CK(cudaMemcpy(&err, sim->dCounter + 2, sizeof(int), cudaMemcpyDeviceToHost));
   if (err) {
     CK(cudaMemset(sim->dCounter + 2, 0, sizeof(int)));
-    return set_err(sim, FIRE_ERR_CUDA, "a device-side wait timed out (multigrid tail bulk copy)");
+    return set_err(sim, FIRE_ERR_CUDA, "a device-side wait timed out (coarse end of the multigrid)");
   }
   return FIRE_OK;
 }
@@ -655,7 +659,7 @@ int fire_sim_set_mg_omega(FireSim* sim, float omega) {
 int fire_sim_set_tail_wait_limit(FireSim* sim, int polls) {
   if (!sim || polls < 0) return FIRE_ERR_BAD_ARG;
   sim->tailWaitPolls = polls;
-  drop_graph(sim);   // the tail launch carries the limit in its descriptor
+  drop_graph(sim);   // the launch of the coarse end carries the limit in its descriptor
   return FIRE_OK;
 }
 
@@ -967,8 +971,8 @@ int fire_sim_run_mg(FireSim* sim, int op, int level, int arg, void* stream) {
       break;
     case 4:   // the shared-memory V-cycle from `level` down, if it fits
       if (!tail_fits(sim->levels.data(), level, n)) return FIRE_ERR_BAD_ARG;
-      if (sim->tailWaitPolls == TAIL_WAIT_POLLS && coarse_fits(sim->levels.data(), level, n))
-        launch_coarse(sim->levels.data(), level, n, 2, 2, sim->coarseIters, nullptr, 1, sim->dCounter + 2, st);
+      if (use_coarse(sim, level))
+        launch_coarse(sim->levels.data(), level, n, 2, 2, sim->coarseIters, nullptr, 1, sim->dCounter + 2, st, sim->tailWaitPolls);
       else launch_tail(sim->levels.data(), level, n, 2, 2, sim->coarseIters, sim->dCounter + 2, st, false, nullptr, sim->tailWaitPolls);
       break;
     default: return FIRE_ERR_BAD_ARG;
@@ -1501,7 +1505,7 @@ int fire_ensemble_sync(FireEnsemble* e) {
   if (cudaMemcpy(&err, e->dErr, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return FIRE_ERR_CUDA;
   if (err) {
     cudaMemset(e->dErr, 0, sizeof(int));
-    return ens_err(e, FIRE_ERR_CUDA, "a device-side wait timed out (multigrid tail bulk copy)");
+    return ens_err(e, FIRE_ERR_CUDA, "a device-side wait timed out (coarse end of the multigrid)");
   }
   return FIRE_OK;
 }

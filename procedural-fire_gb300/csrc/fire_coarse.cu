@@ -75,6 +75,7 @@ struct CoDesc {
   int coarse;            // sweeps of the coarsest level
   const double* cinv;    // or its dense inverse (transposed), applied in FP64
   int* err;              // set to 1 when a bounded wait runs out
+  int polls;             // its limit
 };
 
 extern __shared__ float4 co_smem4[];
@@ -118,9 +119,17 @@ __device__ __forceinline__ float rcp_approx(float d) {
 // uses the barrier pair of its parity: a neighbour sends exchange i + 1 only after it has received this CTA's exchange i, which
 // this CTA sends after arming exchange i's barriers, and it sends i + 2 only after this CTA has finished waiting for i.  The
 // threads that read the received rows are those that send the next ones, so a row is never overwritten before it is read.
+// Every wait is bounded.  A CTA whose wait runs out is dead from then on: it runs through the remaining phases on what it has
+// and takes part in every barrier of its team and of the cluster, but it arms no barrier (a phase of it may be incomplete), waits for no
+// row, stores nothing and, from the next visit of a level on, sends none and tells its neighbours not to wait out their
+// limits (until then it sends at most 128 exchanges of 4 KB, well inside a barrier's 2^20 pending bytes).  They miss its rows
+// and end the same way.  Rows that arrive at a dead CTA are waited for by nobody, so it reports the timeout and holds its
+// shared memory for CO_LANDING_NS after the cluster's last barrier, when nothing is sent any more.
 __shared__ alignas(8) unsigned long long co_bar[2][2];   // [from below, from above][parity]
-__shared__ int co_dead;                                   // a wait ran out: later ones do not wait again
-constexpr int CO_WAIT_POLLS = 1 << 20;
+__shared__ int co_limit;   // polls of a wait; -1: dead (thread 0 sets it before the team's barrier of the phase)
+__shared__ int co_told;    // a neighbour is dead
+constexpr unsigned long long CO_LANDING_NS = 50000000ull;
+__device__ __forceinline__ int wait_limit() { return *(volatile int*)&co_limit; }
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -135,15 +144,15 @@ __device__ __forceinline__ bool bar_test(unsigned bar, unsigned parity) {
                : "=r"(done) : "r"(bar), "r"(parity) : "memory");
   return done != 0;
 }
-__device__ __forceinline__ void bar_wait(unsigned bar, unsigned parity, int* err) {
-  if (bar_test(bar, parity)) return;
+// Up to `polls` polls, about a second, and no longer than until a neighbour is dead.
+__device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity, int polls) {
+  if (bar_test(bar, parity) && polls > 0) return true;
   const unsigned long long t0 = global_ns();
-  for (int i = 0; i < CO_WAIT_POLLS && !*(volatile int*)&co_dead; ++i) {
-    if (bar_test(bar, parity)) return;
+  for (int i = 1; i < polls && !*(volatile int*)&co_told; ++i) {
+    if (bar_test(bar, parity)) return true;
     if ((i & 63) == 63 && global_ns() - t0 > 1000000000ull) break;
   }
-  *(volatile int*)&co_dead = 1;   // bounded: report, and run the rest of the cycle without waiting
-  atomicExch(err, 1);
+  return false;
 }
 __device__ __forceinline__ void team_sync(int bar, int team) {
   asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(team) : "memory");
@@ -180,7 +189,6 @@ struct Slab {
   int bar, team;
   unsigned lo, hi;         // shared-memory addresses of the halo rows this CTA's edge rows go to (0: none)
   unsigned lo_bar, hi_bar; // and of the receivers' barriers (parity 0)
-  int* err;
 };
 __shared__ Slab co_slab[CO_MAX];   // one thread per level fills it in, once per launch
 __device__ __forceinline__ int row_bound(const CoDesc& D, int l, int r) { return (int)D.bound[min(r, D.nact)] << (D.base - l); }
@@ -205,7 +213,6 @@ __device__ __forceinline__ Slab make_slab(const CoDesc& D, int l, int r) {
   s.bar = l + 1;
   s.team = L.team;
   s.lo = s.hi = s.lo_bar = s.hi_bar = 0;
-  s.err = D.err;
   if (l < D.nd) {
     s.y0 = row_bound(D, l, r);
     s.R = row_bound(D, l, r + 1) - s.y0;
@@ -225,23 +232,28 @@ __device__ __forceinline__ Slab make_slab(const CoDesc& D, int l, int r) {
   s.runs = (s.R + L.k - 1) / L.k;
   return s;
 }
-// Arms exchange `ex` for `colours` colours from each neighbour (one thread, before this CTA sends its own rows).
+// Arms exchange `ex` for `colours` colours from each neighbour (thread 0, before this CTA sends its own rows).
 template <bool kSplit>
-__device__ __forceinline__ void exchange_arm(const Slab& L, int colours, int ex) {
-  if (!kSplit || threadIdx.x != 0) return;
+__device__ __forceinline__ void exchange_arm(const Slab& L, int colours, int ex, int limit) {
+  if (!kSplit || threadIdx.x != 0 || limit < 0) return;
   const unsigned bytes = 4u * (unsigned)(colours * L.n);
   if (L.lo) bar_expect(smem32(&co_bar[0][ex & 1]), bytes);
   if (L.hi) bar_expect(smem32(&co_bar[1][ex & 1]), bytes);
 }
-// The end of a phase: the neighbours' rows of exchange `ex` have arrived (warp 0 waits for them), and this CTA's cells and
-// those rows are visible to the level's threads.
+// The end of a phase: the neighbours' rows of exchange `ex` have arrived (warp 0 waits for them; thread 0's wait decides whether
+// this CTA is dead), and this CTA's cells and those rows are visible to the level's threads.  limit: the thread's copy of co_limit.
+// (A call in place of the inlined loops costs 30 ns a phase.)
 template <bool kSplit>
-__device__ __forceinline__ void level_sync(const Slab& L, int& ex) {
+__device__ __forceinline__ void level_sync(const Slab& L, int& ex, int& limit) {
   if (kSplit) {
     if (threadIdx.x < 32) {
-      const unsigned parity = (unsigned)(ex >> 1) & 1u;
-      if (L.lo) bar_wait(smem32(&co_bar[0][ex & 1]), parity, L.err);
-      if (L.hi) bar_wait(smem32(&co_bar[1][ex & 1]), parity, L.err);
+      if (limit >= 0) {
+        const unsigned parity = (unsigned)(ex >> 1) & 1u;
+        if ((L.lo && !bar_wait(smem32(&co_bar[0][ex & 1]), parity, limit)) || (L.hi && !bar_wait(smem32(&co_bar[1][ex & 1]), parity, limit))) {
+          limit = -1;
+          if (threadIdx.x == 0) *(volatile int*)&co_limit = -1;
+        }
+      }
     }
     ++ex;
   }
@@ -300,6 +312,13 @@ __device__ __forceinline__ void own_cells(Own<K>& o, const Slab& L, int tid) {
   const unsigned col = 4u * (unsigned)o.col;
   o.lo = L.lo && !idle && o.j0 == 0 ? L.lo + col : 0u;
   o.hi = L.hi && !idle && o.j0 + o.nv == L.R ? L.hi + col : 0u;
+}
+// A dead CTA sends no rows any more and tells its neighbours.
+template <int K>
+__device__ __forceinline__ void no_rows(Own<K>& o, const Slab& L) {
+  o.lo = o.hi = 0u;
+  if (threadIdx.x == 0 && L.lo) st_cluster(map_rank(smem32(&co_told), cluster_rank() - 1), __int_as_float(1));
+  if (threadIdx.x == 0 && L.hi) st_cluster(map_rank(smem32(&co_told), cluster_rank() + 1), __int_as_float(1));
 }
 // Reciprocal diagonals: open sides and top add 1 to 6, the floor subtracts 1 (rb_update's ghost rules).
 template <int K>
@@ -422,8 +441,8 @@ __device__ __forceinline__ float nbr_yp(const Own<K>& o, const Nbr<K>& n, int c,
 // One colour of a red-black sweep (mgSmooth, src/sim.js:417-437; the order of rb_update in fire_mg.cu; the sum of the two x
 // neighbours, which starts at +0, is the same in either order).  zero: the level's pressure is zero, so only the right-hand side counts.
 template <int K, bool kSplit, bool kRelax>
-__device__ __forceinline__ void sweep_colour(Own<K>& o, const Slab& L, int c, bool zero, int ex) {
-  exchange_arm<kSplit>(L, 1, ex);
+__device__ __forceinline__ void sweep_colour(Own<K>& o, const Slab& L, int c, bool zero, int ex, int limit) {
+  exchange_arm<kSplit>(L, 1, ex, limit);
   if (zero) {
 #pragma unroll
     for (int k = 0; k < K; ++k) {
@@ -449,18 +468,18 @@ __device__ __forceinline__ void sweep_colour(Own<K>& o, const Slab& L, int c, bo
   own_write<K, kSplit>(o, L, c, ex);
 }
 template <int K, bool kSplit, bool kRelax>
-__device__ __forceinline__ void sweeps(Own<K>& o, const Slab& L, int iters, bool zero, int& ex) {
+__device__ __forceinline__ void sweeps(Own<K>& o, const Slab& L, int iters, bool zero, int& ex, int& limit) {
   for (int it = 0; it < iters; ++it) {
-    sweep_colour<K, kSplit, kRelax>(o, L, 0, zero && it == 0, ex);
-    level_sync<kSplit>(L, ex);
-    sweep_colour<K, kSplit, kRelax>(o, L, 1, false, ex);
-    level_sync<kSplit>(L, ex);
+    sweep_colour<K, kSplit, kRelax>(o, L, 0, zero && it == 0, ex, limit);
+    level_sync<kSplit>(L, ex, limit);
+    sweep_colour<K, kSplit, kRelax>(o, L, 1, false, ex, limit);
+    level_sync<kSplit>(L, ex, limit);
   }
 }
 // The first level between global memory and the threads' registers.
 template <int K, bool kSplit>
-__device__ __forceinline__ void load_global(const CoDesc& D, Own<K>& o, const Slab& L, int ex) {
-  exchange_arm<kSplit>(L, 2, ex);
+__device__ __forceinline__ void load_global(const CoDesc& D, Own<K>& o, const Slab& L, int ex, int limit) {
+  exchange_arm<kSplit>(L, 2, ex, limit);
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     const size_t g = 2 * (size_t)o.gx + (size_t)L.nx * ((L.y0 + o.j0 + k) + (size_t)L.ny * o.z);
@@ -692,43 +711,47 @@ __device__ __noinline__ void coarsest_direct(const CoDesc& D, int tid, int nthre
 template <int K, bool kSplit, bool kRelax>
 __device__ __forceinline__ void down(const CoDesc& D, int l, int tid, int rank, int pre, bool load, bool store, int ex) {
   const Slab L = co_slab[l];
+  int limit = kSplit ? wait_limit() : 0;
   Own<K> o;
   own_cells<K, kSplit>(o, L, tid);
+  if (limit < 0) no_rows(o, L);
   if (load) {
-    load_global<K, kSplit>(D, o, L, ex);
+    load_global<K, kSplit>(D, o, L, ex, limit);
   } else {
     if (l == 0) own_read_p(o, L);
     else own_zero(o);
     own_read_b(D, l, o, L);
   }
   own_diag(o, L);
-  if (load) level_sync<kSplit>(L, ex);
+  if (load) level_sync<kSplit>(L, ex, limit);
   const bool last = l == D.n - 1;
-  sweeps<K, kSplit, kRelax>(o, L, last ? D.coarse : pre, l > 0, ex);
+  sweeps<K, kSplit, kRelax>(o, L, last ? D.coarse : pre, l > 0, ex, limit);
   if (!last) restrict_level<K, kSplit>(D, l, o, L, tid, rank);
   else if (l > 0) publish<K, kSplit>(o, L);
-  if (last && store) store_global(D, o, L);
+  if (last && store && (!kSplit || wait_limit() >= 0)) store_global(D, o, L);
 }
 // Prolongation onto level l and post-smoothing; the first level's pressure goes back to global memory.
 template <int K, bool kSplit, bool kRelax>
 __device__ __forceinline__ void up(const CoDesc& D, int l, int tid, int rank, int post, bool store, int ex) {
   const Slab L = co_slab[l];
+  int limit = kSplit ? wait_limit() : 0;
   Own<K> o;
   own_cells<K, kSplit>(o, L, tid);
+  if (limit < 0) no_rows(o, L);
   own_read_p(o, L);
   const CoLevel& C = D.l[l + 1];
   // rows from cy0 - 1 on for a split level (the staged copy when the coarse level is gathered), from 0 on otherwise
   const int plain = kSplit && l + 1 == D.nd ? D.stage : C.plain;
   prolong_level(o, L, C, co_smem() + plain - (kSplit ? C.nx * C.nz * ((L.y0 >> 1) - 1) : 0));
-  exchange_arm<kSplit>(L, 2, ex);
+  exchange_arm<kSplit>(L, 2, ex, limit);
   own_write<K, kSplit>(o, L, 0, ex);
   own_write<K, kSplit>(o, L, 1, ex);
   own_read_b(D, l, o, L);
   own_diag(o, L);
-  level_sync<kSplit>(L, ex);
-  sweeps<K, kSplit, kRelax>(o, L, post, false, ex);
+  level_sync<kSplit>(L, ex, limit);
+  sweeps<K, kSplit, kRelax>(o, L, post, false, ex, limit);
   if (l > 0) publish<K, kSplit>(o, L);
-  if (store) store_global(D, o, L);
+  if (store && (!kSplit || wait_limit() >= 0)) store_global(D, o, L);
 }
 
 template <bool kRelax>
@@ -737,7 +760,8 @@ __device__ __forceinline__ void coarse_body(const CoDesc& D, int smem_floats, in
   const int rank = D.csize > 1 ? (int)cluster_rank() : 0;
   if (tid < n) co_slab[tid] = make_slab(D, tid, rank);
   if (tid == 0) {
-    co_dead = 0;
+    co_limit = D.polls;
+    co_told = 0;
     for (int i = 0; i < 4; ++i)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem32(&co_bar[i >> 1][i & 1])) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -783,7 +807,13 @@ __device__ __forceinline__ void coarse_body(const CoDesc& D, int smem_floats, in
       else up<1, false, kRelax>(D, l, tid, rank, post, store && l == 0, ex0);
     }
   }
+  const bool dead = tid == 0 && wait_limit() < 0;
   if (D.csize > 1) cluster_sync();   // a CTA's shared memory outlives its neighbours' stores into it
+  if (dead) {
+    atomicExch(D.err, 1);
+    const unsigned long long t0 = global_ns();
+    for (int i = 0; i < TAIL_WAIT_POLLS && global_ns() - t0 < CO_LANDING_NS; ++i) __nanosleep(1000);
+  }
 }
 
 // T: the most threads a CTA is launched with, and so its registers per thread (128 / 72 / 64).
@@ -916,8 +946,9 @@ bool make_plan(const MGLevel* levels, int first, int n, bool direct, CoDesc& D, 
   }
   return false;
 }
-void fill_plan(CoDesc& D, const MGLevel* levels, int first, int coarse, const double* cinv, int* err) {
+void fill_plan(CoDesc& D, const MGLevel* levels, int first, int coarse, const double* cinv, int* err, int polls) {
   D.err = err;
+  D.polls = polls;
   D.gp = levels[first].p;
   D.gb = levels[first].b;
   D.vec = levels[first].nx % 2 == 0 && ((reinterpret_cast<uintptr_t>(D.gp) | reinterpret_cast<uintptr_t>(D.gb)) & 7u) == 0;
@@ -956,12 +987,12 @@ int coarse_first(const MGLevel* levels, int n, bool direct) {
   return first;
 }
 cudaError_t launch_coarse(const MGLevel* levels, int first, int n, int pre, int post, int coarse, const double* cinv, int cycles,
-                          int* err, cudaStream_t st) {
+                          int* err, cudaStream_t st, int wait_polls) {
   CoDesc D;
   size_t smem = 0;
   int threads = 0;
   if (!make_plan(levels, first, n, cinv != nullptr, D, smem, threads)) return cudaErrorInvalidValue;
-  fill_plan(D, levels, first, coarse, cinv, err);
+  fill_plan(D, levels, first, coarse, cinv, err, wait_polls);
   const int floats = (int)(smem / sizeof(float));
   return with_kernel(threads, D.omega != 1.0f, [&](auto kernel) {
     return launch_clusters(kernel, D.csize, 1, threads, smem, st, D, floats, pre, post, cycles);
@@ -973,6 +1004,12 @@ bool coarse_fits(const MGLevel* levels, int first, int n, bool direct) {
   int threads;
   return first < n && make_plan(levels, first, n, direct, D, smem, threads);
 }
+bool coarse_waits(const MGLevel* levels, int first, int n) {
+  CoDesc D;
+  size_t smem;
+  int threads;
+  return first < n && make_plan(levels, first, n, false, D, smem, threads) && D.nd > 0 && D.nact > 1;
+}
 
 // ---- batched form: members are grouped by cluster and CTA size ----
 size_t coarse_desc_size() { return sizeof(CoDesc); }
@@ -980,7 +1017,7 @@ int coarse_desc_fill(const MGLevel* levels, int first, int n, int coarse, int* e
   CoDesc D;
   int threads = 0;
   if (!make_plan(levels, first, n, false, D, *smem, threads)) return -1;
-  fill_plan(D, levels, first, coarse, nullptr, err);
+  fill_plan(D, levels, first, coarse, nullptr, err, TAIL_WAIT_POLLS);
   std::memcpy(out, &D, sizeof D);
   return (D.csize > 1 ? 1 : 0) + (threads <= CO_THREADS[0] ? 0 : 2);
 }

@@ -194,11 +194,13 @@ cudaError_t launch_tail(const MGLevel* levels, int first, int n, int pre, int po
 // The coarse end of the cycle with register-resident cells (fire_coarse.cu): levels [first, n) in one launch of one CTA
 // or one cluster.  coarse_first: the finest `first` it takes (n if none); direct: the coarsest level is solved with
 // a dense FP64 inverse (cinv).  `cycles` > 1 (first == 0 only) repeats the whole V-cycle inside the launch.
-// Bit-identical to the launch-per-phase kernels.  `err` receives 1 if a bounded wait for a neighbouring CTA's rows ran out.
+// Bit-identical to the launch-per-phase kernels.  `err` receives 1 if a bounded wait for a neighbouring CTA's rows ran out
+// (wait_polls: its limit; the levels are then left unfinished).  coarse_waits: whether the launch has such waits at all.
 int coarse_first(const MGLevel* levels, int n, bool direct = false);
 bool coarse_fits(const MGLevel* levels, int first, int n, bool direct = false);
+bool coarse_waits(const MGLevel* levels, int first, int n);
 cudaError_t launch_coarse(const MGLevel* levels, int first, int n, int pre, int post, int coarse, const double* cinv, int cycles,
-                          int* err, cudaStream_t st);
+                          int* err, cudaStream_t st, int wait_polls = TAIL_WAIT_POLLS);
 cudaError_t coarse_configure();
 // Batched over simulations: the host fills coarse_desc_size() bytes each and groups them by the returned kind
 // (COARSE_KINDS of them; -1: does not fit); a launch takes `count` descriptors of one kind and their largest smem.

@@ -39,8 +39,8 @@ struct FireSim {
   std::vector<fire::MGLevel> levels;
   int coarseIters = 8;
   int coarseFirst = 0;   // levels [coarseFirst, n) run in one launch of the register-resident coarse kernel (n: none fits)
-  int tailFirst = 0;     // and where the TMA-staged tail starts, which runs while tailWaitPolls is lowered or when that is n
-  int tailWaitPolls = fire::TAIL_WAIT_POLLS;   // bound of the tail's first bulk-copy wait (fire_sim_set_tail_wait_limit)
+  int tailFirst = 0;     // and where the TMA-staged tail starts, which runs when that is n, or has no wait for a lowered tailWaitPolls
+  int tailWaitPolls = fire::TAIL_WAIT_POLLS;   // bound of the coarse end's waits (fire_sim_set_tail_wait_limit)
   uint2* noise = nullptr;
   uint2* curl = nullptr;
   float* dBlock = nullptr;

@@ -375,7 +375,7 @@ class FireSim:
         self._check(self._lib.fire_sim_load(self._h, buf, len(blob)), "load")
 
     def set_tail_wait_limit(self, polls: int):
-        """Fault-injection hook: bound of the multigrid tail's first bulk-copy wait (0 = give up at once)."""
+        """Fault-injection hook: bound of the waits of the multigrid's coarse end (0 = the first gives up at once)."""
         self._check(self._lib.fire_sim_set_tail_wait_limit(self._h, int(polls)), "set_tail_wait_limit")
 
     def set_mg_omega(self, omega: float):
