@@ -373,7 +373,7 @@ __device__ __forceinline__ void forces_cell(const PA& pa, const Fields& f, const
   const float kMix = pa[P_kMix], heatOut = pa[P_heatOut], expansion = pa[P_expansion];
   auto finite = [](float x) { return fabsf(x) <= 3.4028235e38f; };
   // without finite uniforms a product with an exact 0 need not be 0
-  const bool plain = finite(kMix) && finite(heatOut) && finite(expansion) && rs > 0.0f && dt > 0.0f && finite(dt);
+  const bool plain = finite(kMix) && finite(heatOut) && finite(expansion) && rs > 0.0f && finite(rs) && dt > 0.0f && finite(dt);
   float b = 0.0f, T = T0, q = 0.0f, phi = 0.0f;
   if (plain && ign == 0.0f && T0 > 0.0f) {
     s2.x = fminf(s2.x, 1.0f);
