@@ -63,6 +63,7 @@ struct Sweeper {
   float4* S;                                // published columns: [parity][row + 1][pair + 1], at this thread's first row
   int par, pitch;                           // float4 strides of a parity and of a row
   bool live;                                // the columns lie inside the domain
+  bool both, wide;                          // and so do the second row and (rows of an odd length) the second column
 };
 template <bool kRelax>
 __device__ __forceinline__ float update(const Sweeper& w, float old, float own, float far, float zm, float zp, float ym, float yp, float b, float rd) {
@@ -76,7 +77,7 @@ __device__ __forceinline__ float update(const Sweeper& w, float old, float own, 
   return kRelax ? __fmaf_rn(w.omega, __fmaf_rn(t, rd, -old), old) : __fmul_rn(t, rd);
 }
 // Step k = I (mod 6) of the march.  kEdge: some of the planes k-4 .. k-1 lie outside the domain or touch its bottom or top.
-template <typename T, bool kRelax, int I, bool kEdge>
+template <typename T, bool kRelax, bool kOdd, int I, bool kEdge>
 __device__ __forceinline__ void step(const Sweeper& w, Col (&c)[SW_ROWS][2], int k) {
   constexpr int a0 = (I & 1) ? 0 : 1;   // working column of row 0: (x + y + k - 1) even, y even; row 1's is the other
   float4 far[SW_ROWS];
@@ -103,6 +104,7 @@ __device__ __forceinline__ void step(const Sweeper& w, Col (&c)[SW_ROWS][2], int
       float v = update<kRelax>(w, m.v[slot(I, j)], c[r][1 - a].v[slot(I, j)], f[j - 1], m.v[slot(I, j + 1)], m.v[slot(I, j - 1)], ym, yp,
                                      m.b[slot(I, j)], rd);
       v = Cells2<T>::one(Cells2<T>::back(v));   // what a colour launch would have stored
+      if ((r == 1 && !w.both) || (kOdd && a == 1 && !w.wide)) v = 0.0f;   // whatever its neighbours hold, also an infinity
       if (!kEdge || (unsigned)z < (unsigned)w.nz) m.v[slot(I, j)] = v;
     }
   }
@@ -134,8 +136,8 @@ __device__ __forceinline__ void sweep2_body(const T* __restrict__ p, const T* __
   for (int i = tid; i < 2 * w.par; i += blockDim.x) sw_smem[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   const int x = t.lx + 2 * px, y = t.ly + SW_ROWS * ty;
   w.live = work && x < nx && y < ny;   // of an odd nx or ny the last pair or thread row has one column or row in the domain
-  const bool wide = !kOdd || x + 1 < nx;
-  const bool both = y + 1 < ny;
+  const bool wide = w.wide = !kOdd || x + 1 < nx;
+  const bool both = w.both = y + 1 < ny;
   const bool core = w.live && x >= t.x0 && x < t.x1 && y >= t.y0 && y < t.y1;
   Col c[SW_ROWS][2];
 #pragma unroll
@@ -145,7 +147,6 @@ __device__ __forceinline__ void sweep2_body(const T* __restrict__ p, const T* __
       const float d = 6.0f + (x + q == 0 ? 1.0f : 0.0f) + (x + q == nx - 1 ? 1.0f : 0.0f) + (y + r == ny - 1 ? 1.0f : 0.0f) - (y + r == 0 ? 1.0f : 0.0f);
       asm("rcp.approx.f32 %0, %1;" : "=f"(w.rd[r][q]) : "f"(d));
       asm("rcp.approx.f32 %0, %1;" : "=f"(w.rdz[r][q]) : "f"(d + 1.0f));
-      if ((r == 1 && !both) || (q == 1 && !wide)) w.rd[r][q] = w.rdz[r][q] = 0.0f;   // a row or column outside stays zero
 #pragma unroll
       for (int j = 0; j < 6; ++j) c[r][q].v[j] = c[r][q].b[j] = 0.0f;
     }
@@ -192,7 +193,7 @@ __device__ __forceinline__ void sweep2_body(const T* __restrict__ p, const T* __
         c[r][0].v[slot(I, 0)] = c[r][1].v[slot(I, 0)] = 0.0f;
       }
     }
-    step<T, kRelax, I, kEdge>(w, c, k);
+    step<T, kRelax, kOdd, I, kEdge>(w, c, k);
 #pragma unroll
     for (int r = 0; r < SW_ROWS; ++r) {   // b of plane k: used from the next step on; its slot held plane k - 6's
       const float2 v = Cells2<T>::get(ring[SW_ROWS + r][I]);
