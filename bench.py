@@ -178,18 +178,27 @@ def make_sim(F, device: int, mg_fixed: int = 0):
 
 def launches_per_step(sim, cycles_per_step: float) -> float:
     """Kernels launched per step by the captured graph: 5 stencil kernels (the divergence kernel also clears
-    the solve's cycle count), and per V-cycle 4 per level above the coarse kernel (two sweeps in one launch before and after,
-    restriction, prolongation), the coarse kernel, the residual norm and the decision kernel.  The coarse kernel takes the
-    levels whose half-row x z columns, times their groups of four rows per CTA of a 16-CTA cluster, fit 512 threads (1024 for
-    the finest and the coarsest level)."""
-    T = len(sim.levels)
+    the solve's cycle count), and per V-cycle the residual norm, the decision kernel, the coarse kernel, and per level above
+    it restriction, prolongation and four sweeps: two launches of the two-sweep kernel from 150,000 cells on, eight of one
+    colour below.  The coarse kernel takes the levels whose half-row x z columns, times their groups of four rows per CTA of
+    a 16-CTA cluster, fit 512 threads (1024 for the finest and the coarsest level); a coarsest level that it does not take is
+    swept by launches, two sweeps at once from 280,000 cells on (500,000 for rows of an odd length)."""
+    n = len(sim.levels)
+    dims = [level["dims"] for level in sim.levels]
+    cells = [nx * ny * nz for nx, ny, nz in dims]
+    T = n
     while T > 0:
-        nx, ny, nz = sim.levels[T - 1]["dims"]
-        if (nx + 1) // 2 * nz * ((ny + 63) // 64) > (1024 if T in (1, len(sim.levels)) else 512):
+        nx, ny, nz = dims[T - 1]
+        if (nx + 1) // 2 * nz * ((ny + 63) // 64) > (1024 if T in (1, n) else 512):
             break
         T -= 1
-    top = min(T, len(sim.levels) - 1)
-    per_cycle = 4 * top + (1 if T < len(sim.levels) else 0) + 2
+    per_cycle = 2 + sum(4 if c >= 150000 else 10 for c in cells[:min(T, n - 1)])
+    if T < n:
+        per_cycle += 1
+    else:
+        k = sim.coarse_iters
+        pairs = k // 4 if cells[-1] >= (500000 if dims[-1][0] % 2 else 280000) else 0
+        per_cycle += 2 * pairs + 2 * (k - 4 * pairs)
     return 5 + per_cycle * cycles_per_step
 
 
