@@ -119,15 +119,15 @@ __device__ __forceinline__ float rcp_approx(float d) {
 // uses the barrier pair of its parity: a neighbour sends exchange i + 1 only after it has received this CTA's exchange i, which
 // this CTA sends after arming exchange i's barriers, and it sends i + 2 only after this CTA has finished waiting for i.  The
 // threads that read the received rows are those that send the next ones, so a row is never overwritten before it is read.
-// Every wait is bounded.  A CTA whose wait runs out is dead from then on: it runs through the remaining phases on what it has
-// and takes part in every barrier of its team and of the cluster, but it arms no barrier (a phase of it may be incomplete), waits for no
-// row, stores nothing and, from the next visit of a level on, sends none and tells its neighbours not to wait out their
-// limits (until then it sends at most 128 exchanges of 4 KB, well inside a barrier's 2^20 pending bytes).  They miss its rows
-// and end the same way.  Rows that arrive at a dead CTA are waited for by nobody, so it reports the timeout and holds its
+// Every wait is bounded.  A CTA whose wait runs out reports it and is dead from then on: it runs through the remaining phases on
+// what it has and takes part in every barrier of its team and of the cluster, but it arms no barrier (a phase of it may be
+// incomplete), waits for no row, stores nothing and, from the next visit of a level on, sends none (until then at most 128 exchanges
+// of 4 KB, well inside a barrier's 2^20 pending bytes).  Its neighbours miss its rows and end the same way, sooner than
+// their limits, as a late wait looks for a report.  Rows that arrive at a dead CTA are waited for by nobody, so it holds its
 // shared memory for CO_LANDING_NS after the cluster's last barrier, when nothing is sent any more.
 __shared__ alignas(8) unsigned long long co_bar[2][2];   // [from below, from above][parity]
 __shared__ int co_limit;   // polls of a wait; -1: dead (thread 0 sets it before the team's barrier of the phase)
-__shared__ int co_told;    // a neighbour is dead
+__shared__ int* co_err;
 constexpr unsigned long long CO_LANDING_NS = 50000000ull;
 __device__ __forceinline__ int wait_limit() { return *(volatile int*)&co_limit; }
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -144,13 +144,13 @@ __device__ __forceinline__ bool bar_test(unsigned bar, unsigned parity) {
                : "=r"(done) : "r"(bar), "r"(parity) : "memory");
   return done != 0;
 }
-// Up to `polls` polls, about a second, and no longer than until a neighbour is dead.
+// Up to `polls` polls, about a second, and 64 polls where a timeout has been reported already.
 __device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity, int polls) {
   if (bar_test(bar, parity) && polls > 0) return true;
   const unsigned long long t0 = global_ns();
-  for (int i = 1; i < polls && !*(volatile int*)&co_told; ++i) {
+  for (int i = 1; i < polls; ++i) {
     if (bar_test(bar, parity)) return true;
-    if ((i & 63) == 63 && global_ns() - t0 > 1000000000ull) break;
+    if ((i & 63) == 63 && (global_ns() - t0 > 1000000000ull || *(volatile int*)co_err)) break;
   }
   return false;
 }
@@ -251,7 +251,10 @@ __device__ __forceinline__ void level_sync(const Slab& L, int& ex, int& limit) {
         const unsigned parity = (unsigned)(ex >> 1) & 1u;
         if ((L.lo && !bar_wait(smem32(&co_bar[0][ex & 1]), parity, limit)) || (L.hi && !bar_wait(smem32(&co_bar[1][ex & 1]), parity, limit))) {
           limit = -1;
-          if (threadIdx.x == 0) *(volatile int*)&co_limit = -1;
+          if (threadIdx.x == 0) {
+            *(volatile int*)&co_limit = -1;
+            *(volatile int*)co_err = 1;
+          }
         }
       }
     }
@@ -312,13 +315,6 @@ __device__ __forceinline__ void own_cells(Own<K>& o, const Slab& L, int tid) {
   const unsigned col = 4u * (unsigned)o.col;
   o.lo = L.lo && !idle && o.j0 == 0 ? L.lo + col : 0u;
   o.hi = L.hi && !idle && o.j0 + o.nv == L.R ? L.hi + col : 0u;
-}
-// A dead CTA sends no rows any more and tells its neighbours.
-template <int K>
-__device__ __forceinline__ void no_rows(Own<K>& o, const Slab& L) {
-  o.lo = o.hi = 0u;
-  if (threadIdx.x == 0 && L.lo) st_cluster(map_rank(smem32(&co_told), cluster_rank() - 1), __int_as_float(1));
-  if (threadIdx.x == 0 && L.hi) st_cluster(map_rank(smem32(&co_told), cluster_rank() + 1), __int_as_float(1));
 }
 // Reciprocal diagonals: open sides and top add 1 to 6, the floor subtracts 1 (rb_update's ghost rules).
 template <int K>
@@ -714,7 +710,7 @@ __device__ __forceinline__ void down(const CoDesc& D, int l, int tid, int rank, 
   int limit = kSplit ? wait_limit() : 0;
   Own<K> o;
   own_cells<K, kSplit>(o, L, tid);
-  if (limit < 0) no_rows(o, L);
+  if (limit < 0) o.lo = o.hi = 0u;   // a dead CTA sends no rows any more
   if (load) {
     load_global<K, kSplit>(D, o, L, ex, limit);
   } else {
@@ -737,7 +733,7 @@ __device__ __forceinline__ void up(const CoDesc& D, int l, int tid, int rank, in
   int limit = kSplit ? wait_limit() : 0;
   Own<K> o;
   own_cells<K, kSplit>(o, L, tid);
-  if (limit < 0) no_rows(o, L);
+  if (limit < 0) o.lo = o.hi = 0u;   // a dead CTA sends no rows any more
   own_read_p(o, L);
   const CoLevel& C = D.l[l + 1];
   // rows from cy0 - 1 on for a split level (the staged copy when the coarse level is gathered), from 0 on otherwise
@@ -761,7 +757,7 @@ __device__ __forceinline__ void coarse_body(const CoDesc& D, int smem_floats, in
   if (tid < n) co_slab[tid] = make_slab(D, tid, rank);
   if (tid == 0) {
     co_limit = D.polls;
-    co_told = 0;
+    co_err = D.err;
     for (int i = 0; i < 4; ++i)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem32(&co_bar[i >> 1][i & 1])) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -810,7 +806,6 @@ __device__ __forceinline__ void coarse_body(const CoDesc& D, int smem_floats, in
   const bool dead = tid == 0 && wait_limit() < 0;
   if (D.csize > 1) cluster_sync();   // a CTA's shared memory outlives its neighbours' stores into it
   if (dead) {
-    atomicExch(D.err, 1);
     const unsigned long long t0 = global_ns();
     for (int i = 0; i < TAIL_WAIT_POLLS && global_ns() - t0 < CO_LANDING_NS; ++i) __nanosleep(1000);
   }
