@@ -166,7 +166,8 @@ int fire_sim_set_spots(FireSim* sim, const float* spots, int n);
 /* Over-relaxation factor of every red-black sweep of the step's V-cycle (pre/post smoothing and the
  * coarsest-level sweeps): p += omega (p_GS - p), 0 < omega < 2.  1 (default) is the reference's
  * Gauss-Seidel (src/sim.js:417-437) bit for bit; a larger value can cut the cycles a residual-driven solve
- * needs (no counterpart in the reference).                                                            */
+ * needs (no counterpart in the reference).  On a member of an ensemble it acts on the levels that the ensemble
+ * smooths by batched launches; the coarse ends keep omega 1.                                           */
 int fire_sim_set_mg_omega(FireSim* sim, float omega);
 /* Fault-injection hook for the device-side bounded wait (no counterpart in the reference, which logs
  * WebGPU device loss, src/gpu.js:25-26): bounds the waits of the multigrid's coarse end, which runs on a

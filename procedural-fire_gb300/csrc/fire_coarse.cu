@@ -977,7 +977,9 @@ int coarse_first(const MGLevel* levels, int n, bool direct) {
   size_t smem;
   int threads, first = n;
   // A level that needs more than 512 threads a CTA leaves a thread too few registers: 40x60x40 on top of 20x30x20 costs 18 us a
-  // cycle here and 14 in launches.  Where it is the finest level, one launch for all cycles outweighs that.
+  // cycle here and 14 in launches.  It stays where it is the coarsest level (one launch for all its sweeps) or the finest: one launch
+  // for all cycles outweighs the loss where a simulation alone runs a fixed number of them; to a tolerance, in the solver and in
+  // an ensemble, which launch every cycle, a finest level of that size pays those 4 us.
   while (first > 0 && make_plan(levels, first - 1, n, direct, D, smem, threads) && (threads <= CO_THREADS[0] || first == 1 || first == n)) --first;
   return first;
 }

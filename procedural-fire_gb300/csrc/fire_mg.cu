@@ -1091,7 +1091,8 @@ bool tail_fits(const MGLevel* levels, int first, int n, bool coarse64) {
 //   the same ordering at 64x128x64 and 256x512x256.  A level of more than TAIL_FIRST_CELLS (8192) cells is cheaper
 //   as its own launches than inside the tail, so a simulation's tail starts at the finest level that fits and
 //   is no larger than that.  An ensemble runs its members' tails side by side in one launch, which hides a
-//   larger tail's latency, so it lets the tail start at the finest level that fits.
+//   larger tail's latency, so it lets the tail start at the finest level that fits.  (Measured with launches of one colour
+//   sweep each, before the coarse kernel; a tail serves only the coarse ends which that does not take.)
 int tail_first(const MGLevel* levels, int n, bool coarse64, long max_cells) {
   int first = n;
   for (int l = n - 1; l >= 0 && tail_fits(levels, l, n, coarse64) && (long)levels[l].nx * levels[l].ny * levels[l].nz <= max_cells; --l)

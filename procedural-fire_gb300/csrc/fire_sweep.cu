@@ -257,8 +257,8 @@ __global__ void __launch_bounds__(SW_THREADS, 1) k_sweep2(const T* __restrict__ 
   sweep2_body<T, kZero, kRelax, kOdd>(p, b, out, nx, ny, nz, h, omega, P.px, P.ty, tile_of(P, nx, ny, nz, blockIdx.x));
 }
 
-// Measured (GB300, ensemble of 16 grids from 32x64x32 to 96x192x96, 4 cycles): 16 launches per level and cycle of batched colour
-// sweeps, 1245 us of a step's 2978, became 4 and the step takes 2486; CTAs of 256 or 448 threads give the same within 1 %.
+// Measured (GB300, ensemble of 16 grids from 32x64x32 to 96x192x96, 4 cycles): 8 launches per level and cycle of batched colour
+// sweeps, 1245 us of a step's 2978, became 2 and the step takes 2486; CTAs of 256 or 448 threads give the same within 1 %.
 // With both bodies (omega 1 and not) in one kernel 160 bytes of registers spilled: a step 2244, with one body 2032.
 // A level of every simulation of a batch: down from p (kZero: from zero) into p2, else back from p2 into p.
 // kMixed: some member's omega is not 1 (a second body, which costs registers).
