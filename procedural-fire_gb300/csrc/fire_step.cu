@@ -72,7 +72,7 @@ __device__ __forceinline__ void adv1_body(const float* __restrict__ P, const Fie
 // points one cell apart, so the upper four texels of the first sample are the lower four of the second: they are kept, and
 // loaded again only where the two floors differ.  A sample is formed from the same texels by the same operations as sample() in
 // adv1_body, plane by plane; which product of a lerp the compiler rounds there (measured: of a x lerp of velocities the
-// first, elsewhere the second) is written out, so the results are the same bits.
+// first, elsewhere, and in the mix with the wind, the second) is written out, so the results are the same bits.
 // adv2, whose stencils' ranges double the arithmetic, gains nothing from it (256x512x256: 1469 -> 1508 us).
 struct Corner { int o, dx, dy, dz; };   // offset of a 2 x 2 x 2 stencil's first cell and the steps to the second ones (0 at a clamped edge)
 struct Weights { float x, y, z; };
@@ -149,10 +149,9 @@ __device__ __forceinline__ void adv1_column(const float* __restrict__ P, const F
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     const float ws = sstep(0.03f, 0.4f, b[k].y * dx);
-    const f3 wind = mk3(__ldg(P + P_windX) * ws, 0.0f * ws, __ldg(P + P_windZ) * ws);
-    const f3 sv = xyz(s[k]);
-    if (id.k + k < d.nz)
-      f.velX[ci[k]] = make_float4(mixf(wind.x, sv.x, fade[k]), mixf(wind.y, sv.y, fade[k]), mixf(wind.z, sv.z, fade[k]), 0.0f);
+    const float4 wind = make_float4(__ldg(P + P_windX) * ws, 0.0f * ws, __ldg(P + P_windZ) * ws, 0.0f);
+    const f3 v = xyz(lerp_as<false>(wind, s[k], fade[k]));
+    if (id.k + k < d.nz) f.velX[ci[k]] = make_float4(v.x, v.y, v.z, 0.0f);
   }
   sample_column<false>(s, f.S, at, w);
 #pragma unroll
