@@ -227,7 +227,8 @@ int fire_sim_run_stage(FireSim* sim, int stage, float dt, void* stream);
  * 5 = `arg` red-black sweeps, 6 = level-0 residual norms into device scratch without waiting), for
  * kernel-level parity tests and timing (mgSmooth/mgRestrict/mgProlong, src/sim.js:417-495).        */
 int fire_sim_run_mg(FireSim* sim, int op, int level, int arg, void* stream);
-/* Level arrays (which: 0 = p, 1 = b) of any multigrid level, as float32 host arrays.               */
+/* Level arrays (which: 0 = p, 1 = b) of any multigrid level, as float32 host arrays.  A V-cycle's coarse end
+ * runs on chip: it leaves the arrays of the levels below its first one as they were.                     */
 int fire_sim_level_io(FireSim* sim, int level, int which, void* host, size_t bytes, int to_device);
 int fire_sim_level_dims(FireSim* sim, int level, int dims3[3], float* h);
 /* Per-stage GPU milliseconds of the most recent profiled step: enable, then read FIRE_STAGE_COUNT
